@@ -264,6 +264,12 @@ int vx_radiance_mlp_forward(const float* x, int64_t ldx, int64_t n_points, int i
                             const float* W0, const float* b0, const float* W1, const float* b1, float* colors,
                             void* stream);
 
+/* vx_radiance_mlp_forward that also writes each row's ReLU mask for the adjoint: relu_mask (n_points, 2)
+ * 32-bit words, bit j of word k set when hidden unit 32 k + j is active. The same colours. */
+int vx_radiance_mlp_forward_masked(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
+                                   const float* W0, const float* b0, const float* W1, const float* b1, float* colors,
+                                   uint32_t* relu_mask, void* stream);
+
 /* Appearance branch + MLP in one pass (models/voxneus.py:147-157): hash features of o + d*mid
  * (16 levels x 2), SH of the ray direction and the normal are built in shared memory and fed to
  * the 51-64-3 MLP; writes colors (n,3) and, when rows is given, the MLP input rows (row stride
@@ -277,6 +283,15 @@ int vx_appearance_mlp_forward(const float* table, int n_levels, int log2_size, i
                               const float xyz_max[3], int64_t n_points, const float* normals, const float* W0,
                               const float* b0, const float* W1, const float* b1, float* colors, float* rows,
                               int64_t ld_rows, void* stream);
+
+/* vx_appearance_mlp_forward with rows that also writes the ReLU mask (as vx_radiance_mlp_forward_masked):
+ * the training forward, whose rows, colours and mask the adjoint reads. */
+int vx_appearance_mlp_forward_masked(const float* table, int n_levels, int log2_size, int n_features,
+                                     const int32_t* level_res, const float* level_weights, const float* rays_o,
+                                     const float* rays_d, const float* mid, int n_samples, const float xyz_min[3],
+                                     const float xyz_max[3], int64_t n_points, const float* normals, const float* W0,
+                                     const float* b0, const float* W1, const float* b1, float* colors, float* rows,
+                                     int64_t ld_rows, uint32_t* relu_mask, void* stream);
 
 /* Inference form of vx_appearance_mlp_forward (models/voxneus.py:147-157 under no_grad, the path
  * of scripts/render.py:35-54; no rows kept for an adjoint): the same colours,
@@ -297,8 +312,8 @@ int vx_appearance_mlp_forward_chunked(const float* table, int n_levels, int log2
 int vx_mlp_blocks(int64_t n_points);
 int vx_mlp_partial_floats(void);
 
-/* The three MLP kernels run on the tcgen05 tensor cores (kind::tf32, hi/lo split for FP32-level
- * accuracy) and wait on the tensor core with bounded mbarrier polls. Returns how many blocks gave
+/* The MLP kernels run on the tcgen05 tensor cores (forward: kind::tf32, hi/lo split; adjoint:
+ * kind::f16 on three exact bf16 parts; both of FP32-level accuracy) and wait on the tensor core with bounded mbarrier polls. Returns how many blocks gave
  * up on such a wait since the last call (their outputs are invalid) and resets the count; -1 on
  * a CUDA error. Synchronises the device (diagnostic only). No counterpart in the reference. */
 int vx_tensor_core_timeouts(void);
@@ -312,15 +327,24 @@ int vx_tensor_core_timeouts(void);
  * launches captured in a CUDA graph. Thread-local; no counterpart in the reference. */
 int vx_tc_guard(int* status, int64_t wait_polls);
 
-/* Adjoint of vx_radiance_mlp_forward (recomputes the hidden layer): d_colors (n,3) -> d_hash (n,32)
+/* Adjoint of vx_radiance_mlp_forward: d_colors (n,3) -> d_hash (n,32)
  * (gradient of input columns 0..31), d_normal (n,3) (columns 48..50), and the weight gradients
  * dW0, db0, dW1, db1 (written, not accumulated; summed over blocks in a fixed order).
  * colors: the forward's outputs (n,3) for the sigmoid's derivative, or NULL to recompute them
- * (the same bits either way). partials: >= vx_mlp_blocks(n) * vx_mlp_partial_floats() floats. */
+ * (the same bits either way). The hidden layer's ReLU mask comes from one more forward launch; the
+ * _masked form below takes the one its forward wrote. partials: >= vx_mlp_blocks(n) * vx_mlp_partial_floats() floats. */
 int vx_radiance_mlp_backward(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
                              const float* W0, const float* b0, const float* W1, const float* b1, const float* d_colors,
                              const float* colors, float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1,
                              float* db1, float* partials, int64_t n_partial_floats, void* stream);
+
+/* vx_radiance_mlp_backward with the forward's colours and ReLU mask (vx_radiance_mlp_forward_masked on
+ * the same rows and weights): nothing is recomputed; the same bits. relu_mask NULL: as above. */
+int vx_radiance_mlp_backward_masked(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
+                                    const float* W0, const float* b0, const float* W1, const float* b1,
+                                    const float* d_colors, const float* colors, const uint32_t* relu_mask,
+                                    float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1, float* db1,
+                                    float* partials, int64_t n_partial_floats, void* stream);
 
 /* The adjoint of the fused appearance path on its compact rows: n_points rows of 36 floats
  * [hash 32 | normal 3 | pad] (16-byte aligned, contiguous) whose SH(d) features come from rays_d
@@ -328,8 +352,7 @@ int vx_radiance_mlp_backward(const float* x, int64_t ldx, int64_t n_points, int 
  * depend on the ray only (models/embedder.py:55-87). Outputs and partials as
  * vx_radiance_mlp_backward. When n_samples is a multiple of 128 (every 128-sample tile inside one
  * ray: the training and serving shapes) the MLP is folded: SH(d) enters as a per-ray bias of the
- * hidden layer (b0 + W0[:, 32:48] SH(d)) and the SH columns of dW0 come from per-tile column sums
- * of dL/dz, so the results agree with the full rows within FP32 rounding; otherwise SH(d) is
+ * hidden layer (b0 + W0[:, 32:48] SH(d)) and the SH columns of dW0 come from per-tile sums, so the results agree with the full rows within FP32 rounding; otherwise SH(d) is
  * rebuilt per sample and they are the same bits. vx_appearance_mlp_forward folds on the same
  * condition. */
 int vx_appearance_mlp_backward(const float* rows, const float* rays_d, int n_samples, int64_t n_points,
@@ -337,6 +360,16 @@ int vx_appearance_mlp_backward(const float* rows, const float* rays_d, int n_sam
                                const float* d_colors, const float* colors, float* d_hash, float* d_normal, float* dW0,
                                float* db0, float* dW1, float* db1, float* partials, int64_t n_partial_floats,
                                void* stream);
+
+/* vx_appearance_mlp_backward with the colours and ReLU mask of vx_appearance_mlp_forward_masked on the
+ * same rows (ld_rows 36): nothing is recomputed. The folded form needs the mask, 16-byte aligned d_colors,
+ * colors and relu_mask and whole tiles (n_points a multiple of 128); otherwise, and for relu_mask NULL, the
+ * rows are taken unfolded: the same results within FP32 rounding. */
+int vx_appearance_mlp_backward_masked(const float* rows, const float* rays_d, int n_samples, int64_t n_points,
+                                      const float* W0, const float* b0, const float* W1, const float* b1,
+                                      const float* d_colors, const float* colors, const uint32_t* relu_mask,
+                                      float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1, float* db1,
+                                      float* partials, int64_t n_partial_floats, void* stream);
 
 /* ---------------------------------------------------------- render (per ray) --------------- */
 

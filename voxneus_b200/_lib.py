@@ -54,6 +54,9 @@ _PROTOS = {
     "vx_hash_backward_det_workspace": [I64, I32, I32],
     "vx_hash_encode_backward_det": [P, I32, I32, I32, P, P, P, P, P, P, I32, HF3, HF3, I64, P, I64, P, SZ, P],
     "vx_radiance_mlp_forward": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P],
+    "vx_radiance_mlp_forward_masked": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P, P],
+    "vx_appearance_mlp_forward_masked": [P, I32, I32, I32, HI3, HF3, P, P, P, I32, HF3, HF3, I64, P, P, P, P, P, P, P,
+                                         I64, P, P],
     "vx_appearance_mlp_forward": [P, I32, I32, I32, HI3, HF3, P, P, P, I32, HF3, HF3, I64, P, P, P, P, P, P, P, I64,
                                   P],
     "vx_appearance_mlp_forward_chunked": [P, I32, I32, I32, HI3, HF3, P, P, P, I32, HF3, HF3, I64, P, P, P, P, P,
@@ -65,6 +68,8 @@ _PROTOS = {
     "vx_huber_loss": [P, P, I64, F32, P, P, P, I64, P],
     "vx_cat_z_vals": [P, P, P, P, I64, I32, I32, P, P, P],
     "vx_radiance_mlp_backward": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, P],
+    "vx_radiance_mlp_backward_masked": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, P],
+    "vx_appearance_mlp_backward_masked": [P, P, I32, I64, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, P],
     "vx_appearance_mlp_backward": [P, P, I32, I64, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, P],
     "vx_composite_workspace_blocks": [I64],
     "vx_composite_forward": [P, P, P, P, I64, I64, P, P, P, P, P, I32, F32, F32, P, I32, I32, F32, I64, I32, P, P, P,

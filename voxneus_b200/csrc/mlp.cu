@@ -11,21 +11,15 @@
 //   X    (128 sample rows, K = features): chunk (m, 4f..4f+3) at (f*16 + m/8)*128 + (m%8)*16
 //   W0   [hi; lo] (128 rows: hidden unit n's hi part in row n, its lo part in row 64 + n, K =
 //        features): element (r, k) at ((k/4)*16 + r/8)*128 + (r%8)*16 + (k%4)*4
-//   W0^T [hi; lo] (128 feature rows, K = hidden), DZ (128 sample rows, K = hidden), and X^T [hi; lo]
-//   / DZ^T [hi; lo] (128 rows, K = the tile's samples) likewise.
-// The stacked hi/lo operands let one N = 128 MMA form two of the three products:
+// The stacked hi/lo operand lets one N = 128 MMA form two of the three products:
 //   Z   = X W0^T   A = X_hi, B = [W_hi; W_lo] (N = 128) + A = X_lo, B = W_hi (N = 64), K = 56 in 7
 //                  steps; Z = columns [0, 64) + [64, 128)
-//   dX  = DZ W0    the same with A = DZ_hi / DZ_lo, B = W0^T [hi; lo], K = 64 in 8 steps
-//   dW0 = [DZh;DZl]^T X   A = DZ^T [hi; lo], B = X^T [hi; lo] (N = 128), K = 128 samples in 16 steps
-// The forward writes the colours (and, for the adjoint, the input rows: 52 floats, or the compact
-// 36-float rows of the fused appearance path); the adjoint recomputes Z with the identical MMA
-// sequence, writes dL/d(hash) and dL/d(normal), accumulates dW0 (and db0 through a ones column) in
-// TMEM across its tiles and dW1 in TMEM / db1 in registers, and writes per-block partials that
-// k_mlp_wgrad_reduce sums in a fixed order (deterministic). The folded variant (compact rows whose
-// tiles each lie inside one ray) contracts K = 40 features [hash | normal | one] in 5 steps, with
-// SH(d) as a per-ray bias of the hidden layer and the SH columns of dW0 taken from each tile's
-// column sum of dL/dz.
+// The forward writes the colours and, for the adjoint (mlp_adjoint.cuh), the input rows (52 floats, or
+// the compact 36-float rows of the fused appearance path) and each sample's ReLU mask; the adjoint
+// writes dL/d(hash), dL/d(normal) and per-block weight-gradient partials that k_mlp_wgrad_reduce sums in
+// a fixed order (deterministic). The folded variant (compact rows whose tiles each lie inside one ray)
+// contracts K = 40 features [hash | normal | 0] in 5 steps, with SH(d) as a per-ray bias of the hidden
+// layer.
 #include "hashgrid.cuh"
 #include "tc.cuh"
 
@@ -115,23 +109,17 @@ struct MlpW {
 
 // The folded MLP (compact rows whose 128-row tiles each lie inside one ray, so SH(d) is constant
 // over a tile): the 16 SH columns leave the contraction and become a per-ray bias of the hidden
-// layer, b0 + W0[:, 32:48] SH(d). Its input features are [hash 32 | normal 3 | one | 0 x 4], K = 40.
+// layer, b0 + W0[:, 32:48] SH(d). Its input features are [hash 32 | normal 3 | 0 x 5], K = 40
+// (the adjoint puts a one after the normal).
 // Folded feature k comes from column fold_col(k) of W0 (-1: none).
 __device__ __forceinline__ int fold_col(int k) { return k < 32 ? k : (k < 35 ? 48 + (k - 32) : -1); }
 
-// The per-ray bias of hidden unit n: b0[n] + sum_k W0[n, 32 + k] sh[k], k = 0..15 in order (the
-// forward and the adjoint evaluate it identically, so the adjoint's recomputed hidden layer has
-// the forward's bits).
+// The per-ray bias of hidden unit n: b0[n] + sum_k W0[n, 32 + k] sh[k], k = 0..15 in order.
 __device__ __forceinline__ float fold_bias(const MlpW& w, int n, const float sh[16]) {
   float b = __ldg(w.b0 + n);
 #pragma unroll
   for (int k = 0; k < 16; ++k) b = fmaf(__ldg(w.W0 + n * KIN + 32 + k), sh[k], b);
   return b;
-}
-
-// SH(d) of ray r.
-__device__ __forceinline__ void ray_sh(const float* __restrict__ rays_d, int64_t r, float sh[16]) {
-  sh16(__ldg(rays_d + 3 * r), __ldg(rays_d + 3 * r + 1), __ldg(rays_d + 3 * r + 2), sh);
 }
 
 __device__ __forceinline__ uint32_t x_off(int f, int m) { return (uint32_t)((f * 16 + (m >> 3)) * 128 + (m & 7) * 16); }
@@ -254,10 +242,22 @@ __device__ __forceinline__ void tmem_ld_sum32(uint32_t taddr, float v[32]) {
   for (int j = 0; j < 32; ++j) v[j] += u[j];
 }
 
-// This thread's half of the colour pre-activation: hidden units 32*hh..32*hh+31 of sample lane.
-__device__ __forceinline__ void colour_partial(const float z[32], int hh, const float* B0, const float* W1s,
-                                               float& p0, float& p1, float& p2) {
+// Where a forward's outputs go: colours (row stride ldc) and, when mask is given, each sample's ReLU
+// mask (bit j of word k: hidden unit 32 k + j is active; two words a sample, row stride ldm).
+struct MlpOut {
+  float* colors;
+  int64_t ldc;
+  uint32_t* mask;
+  int64_t ldm;
+};
+
+// This thread's half of the colour pre-activation: hidden units 32*hh..32*hh+31 of sample lane; kMask:
+// their ReLU bits.
+template <bool kMask>
+__device__ __forceinline__ uint32_t colour_partial(const float z[32], int hh, const float* B0, const float* W1s,
+                                                   float& p0, float& p1, float& p2) {
   p0 = p1 = p2 = 0.0f;
+  uint32_t bits = 0;
 #pragma unroll
   for (int j4 = 0; j4 < 8; ++j4) {
     const int n = 32 * hh + 4 * j4;
@@ -270,21 +270,22 @@ __device__ __forceinline__ void colour_partial(const float z[32], int hh, const 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float h = fmaxf(z[4 * j4 + i] + bb[i], 0.0f);
+      if (kMask) bits |= (h > 0.0f ? 1u : 0u) << (4 * j4 + i);
       p0 = fmaf(w0[i], h, p0);
       p1 = fmaf(w1[i], h, p1);
       p2 = fmaf(w2[i], h, p2);
     }
   }
+  return bits;
 }
 
 // Forward. kHashIn: the 51 features of a tile are built in place (two threads per sample, 8 hash
 // levels each; SH of the view direction; the normal); else they are read from rows X. kRowsOut
 // also writes the rows for the adjoint. 256 threads: warp w reads TMEM lanes 32*(w%4).. and
 // hidden columns 32*(w/4)..; the two column halves meet in shared memory.
-template <bool kHashIn, bool kRowsOut, bool kCustomWait>
+template <bool kHashIn, bool kRowsOut, bool kMask, bool kCustomWait>
 __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* __restrict__ X, int64_t ldx, int xvec,
-                                                       int64_t P, MlpW w, float* __restrict__ colors,
-                                                       TcGuard g) {
+                                                       int64_t P, MlpW w, MlpOut out, TcGuard g) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t wait_limit = kCustomWait ? g.limit : kWaitLimit;  // a constant bound unless a caller set one
   uint8_t* XH = smem;
@@ -400,7 +401,8 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
     float z[32];
     tmem_ld_sum32(tbase + ((uint32_t)(32 * q) << 16) + 32 * hh, z);
     float p0, p1, p2;
-    colour_partial(z, hh, B0, W1s, p0, p1, p2);
+    const uint32_t bits = colour_partial<kMask>(z, hh, B0, W1s, p0, p1, p2);
+    if (kMask && m0 + 32 * q + lane < P) out.mask[(m0 + 32 * q + lane) * out.ldm + hh] = bits;
     float* r = RED + (hh * TM + 32 * q + lane) * 4;
     r[0] = p0;
     r[1] = p1;
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
 #pragma unroll
       for (int c = 0; c < NO; ++c) {
         const float o = (B1[c] + RED[tid * 4 + c]) + RED[(TM + tid) * 4 + c];
-        colors[(m0 + tid) * NO + c] = sigmoidf_ref(o);
+        out.colors[(m0 + tid) * out.ldc + c] = sigmoidf_ref(o);
       }
     }
   }
@@ -446,9 +448,9 @@ __device__ __forceinline__ void slot_sync(int slot) {
   asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");
 }
 
-template <bool kCustomWait, bool kCompact, bool kFold>
-__global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restrict__ X, int64_t P, MlpW w,
-                                                         float* __restrict__ colors, TcGuard g, RowSrc src) {
+template <bool kCustomWait, bool kCompact, bool kFold, bool kMask>
+__global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restrict__ X, int64_t P, MlpW w, MlpOut out,
+                                                         TcGuard g, RowSrc src) {
   static_assert(!kFold || kCompact, "the folded MLP reads compact rows");
   constexpr int kLd = kCompact ? KC : KP;  // floats per row in global memory
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -625,7 +627,8 @@ __global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restric
     float z[32];
     tmem_ld_sum32(tcol + lane_base + 32 * hh, z);
     float p0, p1, p2;
-    colour_partial(z, hh, kFold ? BETA : B0, W1s, p0, p1, p2);
+    const uint32_t bits = colour_partial<kMask>(z, hh, kFold ? BETA : B0, W1s, p0, p1, p2);
+    if (kMask && valid) out.mask[(m0 + m) * out.ldm + hh] = bits;
     float* r = RED + (hh * TM + m) * 4;
     r[0] = p0;
     r[1] = p1;
@@ -636,7 +639,7 @@ __global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restric
 #pragma unroll
       for (int c = 0; c < NO; ++c) {
         const float o = (B1[c] + RED[stid * 4 + c]) + RED[(TM + stid) * 4 + c];
-        colors[(m0 + stid) * NO + c] = sigmoidf_ref(o);
+        out.colors[(m0 + stid) * out.ldc + c] = sigmoidf_ref(o);
       }
     }
   }
@@ -652,536 +655,11 @@ __global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restric
   if (tid < 32) tc::tmem_dealloc(*s_taddr, 512);
 }
 
-// Adjoint. d_out (P,3) -> d_hash (P,32), d_normal (P,3), per-block weight-gradient partials
-// [dW0 (64 x 52) | dW1 (3 x 64) | db0 (64) | db1 (3)]. tcgen05 kind::tf32 takes K-major operands
-// only here, so the sample contraction of dW0 reads transposed copies: X^T (written as the rows
-// are staged) and DZ^T, whose scalar stores are bank-conflict free because their 16-byte K chunks
-// of 4 samples sit 1040 / 2064 bytes apart (one 16-byte pad per chunk slab).
-// Per tile: stage rows -> Z MMA -> epilogue (colours, dO, dW1 in registers, DZ) -> dX MMA ->
-// DZ^T -> dW0 MMA (overlapping the dX readout). TMEM columns: Z, then dX, in [0,128) (two halves
-// each); dW0 = [DZ_hi | DZ_lo]^T X_hi in [128,192) and x X_lo in [192,256); dW1 sums in
-// [256,448); the hi part of the Z and dX MMAs' A operand (X_hi, then DZ_hi; sample lanes, K along
-// the columns) in [448,512), written by the threads with tcgen05.st, so it takes no shared-memory
-// stores or operand reads (the lo parts stay in R1).
-constexpr uint32_t kXtSlab = 16 * 128 + 16;   // X^T: 4 samples x 128 rows (features hi | features lo)
-constexpr uint32_t kDztSlab = 16 * 128 + 16;  // DZ^T: 4 samples x 128 rows (hidden hi | hidden lo)
-constexpr uint32_t kXtBytes = 32 * kXtSlab;
-constexpr uint32_t kR1Bytes = 66560;          // X (hi, lo) -> DZ (hi, lo) -> DZ^T, one at a time
-constexpr uint32_t kRowBytes = KP * 4;        // one 52-float input row
-constexpr uint32_t kRowsBytes = TM * kRowBytes;  // the next tile's rows, brought in by a bulk copy
-constexpr uint32_t kAhiCol = 448;                // TMEM column of A_hi (X_hi, then DZ_hi)
+}  // namespace vx
 
-__device__ __forceinline__ uint32_t xt_off(int f, int m) {
-  return (uint32_t)((m >> 2) * kXtSlab + (f >> 3) * 128 + (f & 7) * 16 + (m & 3) * 4);
-}
-__device__ __forceinline__ uint32_t dzt_off(int r, int m) {
-  return (uint32_t)((m >> 2) * kDztSlab + (r >> 3) * 128 + (r & 7) * 16 + (m & 3) * 4);
-}
-// W0^T [hi; lo] (row f < 64: hi of feature f, else lo of feature f - 64; hidden K): element (f, n)
-// at (n/4)*2048 + (f/8)*128 + (f%8)*16 + (n%4)*4
-__device__ __forceinline__ uint32_t wt_off(int f, int n) {
-  return (uint32_t)((n >> 2) * 2048 + (f >> 3) * 128 + (f & 7) * 16 + (n & 3) * 4);
-}
+#include "mlp_adjoint.cuh"
 
-// kBulk: the rows are contiguous 52-float rows (ldx = 52, 16-byte aligned); each tile's rows reach
-// shared memory through one bulk copy issued as soon as the previous tile has been staged, so no
-// registers or load instructions are spent on the prefetch. Otherwise the rows are prefetched
-// into registers during the previous tile.
-template <bool kBulk, bool kCustomWait, bool kCompact, bool kFold>
-__global__ void __launch_bounds__(256, 1) k_mlp_bwd_tc(const float* __restrict__ X, int64_t ldx, int xvec, int64_t P,
-                                                      MlpW w, const float* __restrict__ d_out,
-                                                      const float* __restrict__ y_in,
-                                                      float* __restrict__ d_hash, float* __restrict__ d_normal,
-                                                      float* __restrict__ partials, TcGuard g, RowSrc src) {
-  static_assert(!kFold || (kCompact && kBulk), "the folded MLP reads compact rows by bulk copy");
-  constexpr uint32_t kRowB = (kCompact ? KC : KP) * 4;  // bytes per row in global and shared memory
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const uint32_t wait_limit = kCustomWait ? g.limit : kWaitLimit;
-  uint8_t* W2 = smem;
-  uint8_t* WT2 = W2 + kWBytes;
-  uint8_t* XT2 = WT2 + kWBytes;
-  uint8_t* R1 = XT2 + kXtBytes;
-  uint8_t* ROWS = R1 + kR1Bytes;  // kBulk only
-  float* RED = reinterpret_cast<float*>(ROWS + (kBulk ? TM * kRowB : 0));  // [2][TM][4]
-  float* W1s = RED + 2 * TM * 4;
-  float* B0 = W1s + NO * NH;
-  float* B1 = B0 + NH;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(B1 + 4);
-  uint64_t* bar_rows = bar + 1;
-  uint32_t* s_taddr = reinterpret_cast<uint32_t*>(bar + 2);
-  // kFold: the SH columns of dW0, [16][128]: one column per TMEM lane of DZ^T (hidden unit hi
-  // parts in lanes 0..63, lo parts in 64..127; lanes consecutive, so a warp's accesses are
-  // conflict-free); the hidden bias of the last two tiles (read as float4: 16-byte aligned) and
-  // their SH(d). The dynamic shared memory starts 1024-byte aligned, so aligning the address
-  // aligns the offset.
-  float* SHACC = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(bar) + 24 + 15) & ~uintptr_t(15));
-  float* BETA = SHACC + TM * 16;  // [2][64]: tiles by parity
-  float* SHT = BETA + 2 * NH;     // [2][16]
-  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, q = wid & 3, hh = wid >> 2;
-  const int m = 32 * q + lane;  // this thread's sample in the tile (its TMEM lane)
-  // W0 [hi; lo] (hidden rows) for Z, W0^T [hi; lo] (feature rows) for dX, b0, W1, b1; X^T feature
-  // rows 52..63 (hi and lo) zero
-  for (int e = tid; e < NH * 64; e += blockDim.x) {
-    const int n = e >> 6, k = e & 63;
-    const int col = kFold ? fold_col(k) : (k < KIN ? k : -1);
-    float h, l;
-    tc::split_tf32(col >= 0 ? w.W0[n * KIN + col] : 0.0f, h, l);
-    *reinterpret_cast<float*>(W2 + w_off(n, k)) = h;
-    *reinterpret_cast<float*>(W2 + w_off(NH + n, k)) = l;
-    *reinterpret_cast<float*>(WT2 + wt_off(k, n)) = h;
-    *reinterpret_cast<float*>(WT2 + wt_off(64 + k, n)) = l;
-  }
-  constexpr int kXtZero = kFold ? 36 : 52;  // X^T feature rows never written by the tiles
-  for (int e = tid; e < (64 - kXtZero) * TM; e += blockDim.x) {
-    *reinterpret_cast<float*>(XT2 + xt_off(kXtZero + e / TM, e % TM)) = 0.0f;
-    *reinterpret_cast<float*>(XT2 + xt_off(64 + kXtZero + e / TM, e % TM)) = 0.0f;
-  }
-  if (kFold && hh == 1) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) SHACC[k * TM + m] = 0.0f;
-  }
-
-  for (int i = tid; i < NH; i += blockDim.x) B0[i] = w.b0[i];
-  for (int i = tid; i < NO * NH; i += blockDim.x) W1s[i] = w.W1[i];
-  if (tid < NO) B1[tid] = w.b1[tid];
-  if (tid == 0) {
-    tc::mbar_init(bar, 1);
-    tc::mbar_init(bar_rows, 1);
-  }
-  if (wid == 0) tc::tmem_alloc(s_taddr, 512);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t tbase = *s_taddr;
-  const uint32_t lane_base = (uint32_t)(32 * q) << 16;
-  const uint32_t w2 = tc::smem_u32(W2), wt2 = tc::smem_u32(WT2), xt2 = tc::smem_u32(XT2), r1 = tc::smem_u32(R1);
-  float ones_prev = 0.0f;  // kFold: this lane's ones column of dW0 after the previous tile
-  int it = 0;              // tiles this block has completed
-  // kFold, warps 4..7 (lanes 0..127 = the rows of DZ^T): the SH columns of dW0 from a completed
-  // tile: its column sum of dL/dz (its growth of the ones column, feature 35 of the X_hi product;
-  // lane m is hidden unit m % 64, hi or lo part) times its SH(d)
-  auto fold_sh_columns = [&](const float* sht) {
-    float v[4];
-    tc::tmem_ld4(tbase + lane_base + 128 + 32, v);
-    tc::tmem_wait_ld();
-    const float sum = v[3] - ones_prev;
-    ones_prev = v[3];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) SHACC[k * TM + m] = fmaf(sum, sht[k], SHACC[k * TM + m]);
-  };
-  // kFold, threads 0..63: the hidden bias and (thread 0) the SH(d) of tile `tile` into buffer
-  // `buf`, a tile ahead (the global loads overlap the previous tile's dW0 MMAs)
-  auto fold_prepare = [&](int64_t tile, int buf) {
-    if (tid < NH) {
-      float sh[16];
-      ray_sh(src.rays_d, tile * TM / src.S, sh);
-      BETA[NH * buf + tid] = fold_bias(w, tid, sh);
-      if (tid == 0) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) SHT[16 * buf + k] = sh[k];
-      }
-    }
-  };
-  const int64_t ntiles = (P + TM - 1) / TM;
-  // rows of tile t into ROWS (kBulk): one copy of the tile's valid rows, issued by thread 0
-  auto fetch_rows = [&](int64_t t) {
-    const int64_t m0 = t * TM;
-    const uint32_t bytes = (uint32_t)(P - m0 < TM ? P - m0 : TM) * kRowB;
-    tc::mbar_arrive_expect_tx(bar_rows, bytes);
-    tc::bulk_g2s(ROWS, X + m0 * (kRowB / 4), bytes, bar_rows);
-  };
-  uint32_t rphase = 0;
-  // thread 0's bookkeeping for a give-up: a rows copy in flight and the mbarrier parity it completes
-  bool rows_pending = false;
-  uint32_t rows_parity = 0;
-  if (kBulk && tid == 0 && (int64_t)blockIdx.x < ntiles) {
-    fetch_rows(blockIdx.x);
-    rows_pending = true;
-  }
-  // dW1 accumulators of hidden units 32*hh+j, colour c, summed over this thread's samples: TMEM
-  // columns 256 + 96*hh + 32*c + j of this thread's lane (registers are spent on the prefetch)
-  const uint32_t g1addr = tbase + lane_base + 256 + 96 * hh;
-  {
-    float zero[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) zero[j] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < NO; ++c) tc::tmem_st32(g1addr + 32 * c, zero);
-    tc::tmem_wait_st();
-  }
-  float sb[NO] = {0.0f, 0.0f, 0.0f};
-  bool first_w = true, failed = false;
-  bool mma_pending = false;  // thread 0: its own wait on an MMA gave up
-  uint32_t phase = 0;
-  float4 pre[7];  // !kBulk: this tile's row chunks, loaded during the previous tile
-  float dy[NO], yv[NO] = {0.0f, 0.0f, 0.0f};  // dL/dcolour and (y_in) the forward's colour of this sample
-  if ((int64_t)blockIdx.x < ntiles) {
-    const int64_t m0 = (int64_t)blockIdx.x * TM;
-    if (kFold) fold_prepare(blockIdx.x, 0);
-    if (!kBulk) load_row_chunks(X, ldx, xvec != 0, P, m0, m, hh, pre);
-#pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      dy[c] = m0 + m < P ? d_out[(m0 + m) * NO + c] : 0.0f;
-      if (y_in) yv[c] = m0 + m < P ? y_in[(m0 + m) * NO + c] : 0.0f;
-    }
-  }
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t m0 = t * TM;
-    const bool valid = m0 + m < P;
-    if (kBulk) {
-      const bool got = tc::mbar_wait(bar_rows, rphase, wait_limit);
-      rphase ^= 1u;
-      if (__syncthreads_or(!got)) {
-        failed = true;
-        break;
-      }
-      if (tid == 0) rows_pending = false;
-    }
-    // rows -> X_hi (TMEM, sample lanes), X_lo (sample rows, R1) and X^T (feature rows); column 51
-    // (folded: 35) = 1 on real rows (db0)
-    if constexpr (kFold) {
-      const int c0 = hh ? 5 : 0;
-      const float4* rrow = reinterpret_cast<const float4*>(ROWS + m * kRowB);
-      float xh[20];  // features 4*c0 .. 4*c0 + 19: [hash 32 | normal 3 | one | 0 x 4]
-#pragma unroll
-      for (int jc = 0; jc < 5; ++jc) {
-        const int c = c0 + jc;
-        float4 u = (valid && c < 9) ? rrow[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (c == 8) u.w = valid ? 1.0f : 0.0f;
-        const float v[4] = {u.x, u.y, u.z, u.w};
-        float lo[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          tc::split_tf32(v[i], xh[4 * jc + i], lo[i]);
-          if (c < 9) {
-            *reinterpret_cast<float*>(XT2 + xt_off(4 * c + i, m)) = xh[4 * jc + i];
-            *reinterpret_cast<float*>(XT2 + xt_off(64 + 4 * c + i, m)) = lo[i];
-          }
-        }
-        *reinterpret_cast<float4*>(R1 + kXBytes + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-      }
-      const uint32_t ta = tbase + lane_base + kAhiCol + 4 * c0;  // stores aligned to their widths
-      if (hh == 0) {
-        tc::tmem_st16(ta, xh);
-        tc::tmem_st4(ta + 16, xh + 16);
-      } else {
-        tc::tmem_st4(ta, xh);
-        tc::tmem_st8(ta + 4, xh + 4);
-        tc::tmem_st8(ta + 12, xh + 12);
-      }
-      tc::tmem_wait_st();
-    } else {
-      const int c0 = hh ? 7 : 0;
-      const float4* rrow = reinterpret_cast<const float4*>(ROWS + m * kRowB);
-      const float3 dir = stage_dir<kCompact>(src, m0 + m, valid && hh);
-      float xh[28];  // features 4*c0 .. 4*c0 + 27 (hh = 1: 28..55, with 52..55 the zero chunk 13)
-#pragma unroll
-      for (int jc = 0; jc < 7; ++jc) {
-        const int c = c0 + jc;
-        if (c < 13) {
-          float4 u;
-          if (kBulk)
-            u = valid ? x_chunk<kCompact>(rrow, hh, jc, dir) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          else
-            u = pre[jc];
-          float v[4] = {u.x, u.y, u.z, u.w};
-          if (c == 12 && valid) v[3] = 1.0f;
-          float lo[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            tc::split_tf32(v[i], xh[4 * jc + i], lo[i]);
-            *reinterpret_cast<float*>(XT2 + xt_off(4 * c + i, m)) = xh[4 * jc + i];
-            *reinterpret_cast<float*>(XT2 + xt_off(64 + 4 * c + i, m)) = lo[i];
-          }
-          *reinterpret_cast<float4*>(R1 + kXBytes + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-        } else {  // feature chunk 13 (columns 52..55) is inside the Z contraction: zero
-#pragma unroll
-          for (int i = 0; i < 4; ++i) xh[4 * jc + i] = 0.0f;
-          *reinterpret_cast<float4*>(R1 + kXBytes + x_off(13, m)) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-      }
-      // X_hi at TMEM column kAhiCol + feature, in stores aligned to their widths
-      const uint32_t ta = tbase + lane_base + kAhiCol + 4 * c0;
-      if (hh == 0) {
-        tc::tmem_st16(ta, xh);
-        tc::tmem_st8(ta + 16, xh + 16);
-        tc::tmem_st4(ta + 24, xh + 24);
-      } else {
-        tc::tmem_st4(ta, xh);
-        tc::tmem_st16(ta + 4, xh + 4);
-        tc::tmem_st8(ta + 20, xh + 20);
-      }
-      tc::tmem_wait_st();
-    }
-    tc::fence_smem_to_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc::fence_after_sync();
-      issue_split_ts(tbase, tbase + kAhiCol, r1 + kXBytes, w2, kFold ? 5 : 7);
-      tc::commit(bar);
-      if (kBulk && t + gridDim.x < ntiles) {  // ROWS has been read: bring the next tile's rows
-        fetch_rows(t + gridDim.x);
-        rows_pending = true;
-        rows_parity = rphase;
-      }
-    }
-    // while the Z MMA runs: the previous tile's SH columns of dW0
-    if (kFold && hh == 1 && it > 0) fold_sh_columns(SHT + 16 * ((it - 1) & 1));
-    bool ok = tc::mbar_wait(bar, phase, wait_limit);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      mma_pending = !ok;
-      break;
-    }
-    tc::fence_after_sync();
-    float z[32];
-    tmem_ld_sum32(tbase + lane_base + 32 * hh, z);
-    float d[NO];
-    if (y_in) {  // the forward's colours: the same bits as the recomputation below
-#pragma unroll
-      for (int c = 0; c < NO; ++c) d[c] = dy[c] * ((1.0f - yv[c]) * yv[c]);  // 0 on rows past P
-    } else {     // block-uniform branch: every thread takes the same side of the barrier
-      {
-        float p0, p1, p2;
-        colour_partial(z, hh, kFold ? BETA + NH * (it & 1) : B0, W1s, p0, p1, p2);
-        float* r = RED + (hh * TM + m) * 4;
-        r[0] = p0;
-        r[1] = p1;
-        r[2] = p2;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < NO; ++c) {
-        const float o = (B1[c] + RED[m * 4 + c]) + RED[(TM + m) * 4 + c];
-        const float y = sigmoidf_ref(o);
-        d[c] = dy[c] * ((1.0f - y) * y);  // dL/d(pre-sigmoid); 0 on rows past P
-      }
-    }
-    if (hh == 0) {
-#pragma unroll
-      for (int c = 0; c < NO; ++c) sb[c] += d[c];
-    }
-    // dW1 (TMEM accumulators), dL/dz (kept in z), then DZ: the Z MMA has read X
-#pragma unroll
-    for (int j4 = 0; j4 < 8; ++j4) {
-      const float4 b = *reinterpret_cast<const float4*>((kFold ? BETA + NH * (it & 1) : B0) + 32 * hh + 4 * j4);
-      z[4 * j4] += b.x;
-      z[4 * j4 + 1] += b.y;
-      z[4 * j4 + 2] += b.z;
-      z[4 * j4 + 3] += b.w;
-    }
-#pragma unroll 1
-    for (int c = 0; c < NO; ++c) {
-      float acc[32];
-      tc::tmem_ld32(g1addr + 32 * c, acc);
-      tc::tmem_wait_ld();
-      const float dc = c == 0 ? d[0] : (c == 1 ? d[1] : d[2]);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = fmaf(dc, fmaxf(z[j], 0.0f), acc[j]);
-      tc::tmem_st32(g1addr + 32 * c, acc);
-    }
-    tc::tmem_wait_st();
-#pragma unroll
-    for (int j4 = 0; j4 < 8; ++j4) {
-      const int n = 32 * hh + 4 * j4;
-      const float4 u0 = *reinterpret_cast<const float4*>(W1s + n);
-      const float4 u1 = *reinterpret_cast<const float4*>(W1s + NH + n);
-      const float4 u2 = *reinterpret_cast<const float4*>(W1s + 2 * NH + n);
-      const float w0[4] = {u0.x, u0.y, u0.z, u0.w}, w1[4] = {u1.x, u1.y, u1.z, u1.w};
-      const float w2[4] = {u2.x, u2.y, u2.z, u2.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float dhid = d[0] * w0[i] + d[1] * w1[i] + d[2] * w2[i];
-        z[4 * j4 + i] = z[4 * j4 + i] > 0.0f ? dhid : 0.0f;
-      }
-    }
-    float zl[32];  // dL/dz split once: hi in z, lo in zl (stored as DZ now and as DZ^T below)
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float v = z[j];
-      tc::split_tf32(v, z[j], zl[j]);
-    }
-    // DZ_hi into TMEM (over X_hi: the Z MMA has completed), DZ_lo (sample rows) into R1
-    tc::tmem_st32(tbase + lane_base + kAhiCol + 32 * hh, z);
-#pragma unroll
-    for (int j4 = 0; j4 < 8; ++j4)
-      *reinterpret_cast<float4*>(R1 + kXBytes + x_off(8 * hh + j4, m)) =
-          make_float4(zl[4 * j4], zl[4 * j4 + 1], zl[4 * j4 + 2], zl[4 * j4 + 3]);
-    tc::tmem_wait_st();
-    tc::fence_smem_to_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {  // dX = DZ W0 (B = W0^T [hi; lo], feature rows) into the columns Z used
-      tc::fence_after_sync();
-      issue_split_ts(tbase, tbase + kAhiCol, r1 + kXBytes, wt2, 8);
-      tc::commit(bar);
-    }
-    ok = tc::mbar_wait(bar, phase, wait_limit);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      mma_pending = !ok;
-      break;
-    }
-    tc::fence_after_sync();
-    // DZ^T into R1 (the dX MMA has read DZ): rows 0..63 hi, 64..127 lo
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int n = 32 * hh + j;
-      *reinterpret_cast<float*>(R1 + dzt_off(n, m)) = z[j];
-      *reinterpret_cast<float*>(R1 + dzt_off(NH + n, m)) = zl[j];
-    }
-    tc::fence_smem_to_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    // dW0 (+db0) += [DZ_hi | DZ_lo]^T X, K = the tile's samples; issued by a warp whose dX readout
-    // is short (d_normal), so the d_hash readout warps are not held behind the issue
-    if (tid == 128) {
-      tc::fence_after_sync();
-#pragma unroll 1
-      for (int s = 0; s < 16; ++s) {
-        const uint64_t ad = tc::sdesc(r1 + s * 2 * kDztSlab, kDztSlab, 128);
-        const uint64_t b = tc::sdesc(xt2 + s * 2 * kXtSlab, kXtSlab, 128);
-        tc::mma_tf32(tbase + 128, ad, b, kId128, !first_w);  // [128,192): x X_hi, [192,256): x X_lo
-        first_w = false;
-      }
-      tc::commit(bar);
-    }
-    // next tile's rows fly during the dW0 MMAs and the dX readout
-    if (t + gridDim.x < ntiles) {
-      const int64_t mn = (t + gridDim.x) * TM;
-      if (kFold) fold_prepare(t + gridDim.x, (it + 1) & 1);
-      if (!kBulk) load_row_chunks(X, ldx, xvec != 0, P, mn, m, hh, pre);
-#pragma unroll
-      for (int c = 0; c < NO; ++c) {
-        dy[c] = mn + m < P ? d_out[(mn + m) * NO + c] : 0.0f;
-        if (y_in) yv[c] = mn + m < P ? y_in[(mn + m) * NO + c] : 0.0f;
-      }
-    }
-    // dX readout while the dW0 MMAs run
-    if (hh == 0) {
-      float v[32];
-      tmem_ld_sum32(tbase + lane_base, v);
-      if (valid) {
-        float4* o = reinterpret_cast<float4*>(d_hash + (m0 + m) * 32);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) o[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-      }
-    } else {
-      float v[4], u[4];
-      constexpr int kNrmCol = kFold ? 32 : 48;  // the normal's feature columns
-      tc::tmem_ld4(tbase + lane_base + kNrmCol, v);
-      tc::tmem_ld4(tbase + lane_base + 64 + kNrmCol, u);
-      tc::tmem_wait_ld();
-      if (valid) {
-        v[0] += u[0];
-        v[1] += u[1];
-        v[2] += u[2];
-        d_normal[(m0 + m) * 3] = v[0];
-        d_normal[(m0 + m) * 3 + 1] = v[1];
-        d_normal[(m0 + m) * 3 + 2] = v[2];
-      }
-    }
-    ok = tc::mbar_wait(bar, phase, wait_limit);  // R1 and X^T are rewritten by the next tile
-    phase ^= 1u;
-    tc::fence_before_sync();
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      mma_pending = !ok;
-      break;
-    }
-    tc::fence_after_sync();
-    ++it;
-  }
-  if (kFold && hh == 1 && it > 0 && !failed) fold_sh_columns(SHT + 16 * ((it - 1) & 1));  // the last tile's
-  if (failed && tid == 0) {
-    // the MMAs and a rows copy may still run: let them finish (bounded) before tensor memory is
-    // read and freed and the block leaves
-    if (mma_pending) tc::mbar_wait(bar, phase ^ 1u, kDrainLimit);
-    if (kBulk && rows_pending) tc::mbar_wait(bar_rows, rows_parity, kDrainLimit);
-    report_timeout(g.status);
-  }
-  // weight-gradient partials of this block
-  const bool have = blockIdx.x < ntiles && !failed;  // every block with a tile issued the dW0 MMAs
-  float* pb = partials + (int64_t)blockIdx.x * WG;
-  float* R2 = reinterpret_cast<float*>(R1);           // [64][64]: dW0 rows of DZ_lo x X_hi
-  float* RW1 = R2 + 64 * 64;                          // [4 q][2 hh][3][32] dW1, then [4][3] db1
-  __syncthreads();
-  tc::fence_after_sync();  // thread 0's drain (after a give-up) before this block reads tensor memory
-  if (q >= 2) {
-    float v[32];
-    tc::tmem_ld32(tbase + lane_base + 128 + 32 * hh, v);
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 32; ++j) R2[(m - 64) * 64 + 32 * hh + j] = have ? v[j] : 0.0f;
-  }
-#pragma unroll 1
-  for (int c = 0; c < NO; ++c) {
-    float acc[32];
-    tc::tmem_ld32(g1addr + 32 * c, acc);
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 32; ++j) acc[j] = warp_sum(acc[j]);
-    const float sbc = warp_sum(c == 0 ? sb[0] : (c == 1 ? sb[1] : sb[2]));
-    if (lane == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) RW1[((q * 2 + hh) * 3 + c) * 32 + j] = acc[j];
-      if (hh == 0) RW1[4 * 2 * 3 * 32 + q * 3 + c] = sbc;
-    }
-  }
-  __syncthreads();
-  if (q < 2) {
-    float v1[32], v2[32];
-    tc::tmem_ld32(tbase + lane_base + 128 + 32 * hh, v1);
-    tc::tmem_ld32(tbase + lane_base + 192 + 32 * hh, v2);
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int col = 32 * hh + j;
-      const float val = have ? (v1[j] + v2[j]) + R2[m * 64 + col] : 0.0f;
-      if (kFold) {  // folded feature col -> the column of W0 it came from; 35 is the ones column
-        const int oc = fold_col(col);
-        if (oc >= 0) pb[m * KP + oc] = val;
-        if (col == 35) pb[NH * KP + NO * NH + m] = val;
-      } else {
-        if (col < KP) pb[m * KP + col] = val;
-        if (col == KIN) pb[NH * KP + NO * NH + m] = val;  // ones column: db0
-      }
-    }
-    if (kFold && hh == 0) {  // the SH columns 32..47 (hi + lo lanes) and the padding column
-#pragma unroll
-      for (int k = 0; k < 16; ++k) pb[m * KP + 32 + k] = have ? SHACC[k * TM + m] + SHACC[k * TM + 64 + m] : 0.0f;
-      pb[m * KP + KIN] = 0.0f;
-    }
-  }
-  if (tid < NO * NH) {
-    const int c = tid / NH, n = tid % NH, h2 = n >> 5, j = n & 31;
-    float s = 0.0f;
-#pragma unroll
-    for (int qq = 0; qq < 4; ++qq) s += RW1[((qq * 2 + h2) * 3 + c) * 32 + j];
-    pb[NH * KP + c * NH + n] = have ? s : 0.0f;
-  }
-  if (tid < NO) {
-    float s = 0.0f;
-#pragma unroll
-    for (int qq = 0; qq < 4; ++qq) s += RW1[4 * 2 * 3 * 32 + qq * 3 + tid];
-    pb[NH * KP + NO * NH + NH + tid] = have ? s : 0.0f;
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (wid == 0) tc::tmem_dealloc(tbase, 512);
-}
-
-constexpr size_t kBwdSmemRegs = 2 * kWBytes + kXtBytes + kR1Bytes + sizeof(float) * (2 * TM * 4 + NO * NH + NH + 4) + 24;
-constexpr size_t kBwdSmemBulk = kBwdSmemRegs + kRowsBytes;
-constexpr size_t kBwdSmemCompact = kBwdSmemRegs + TM * KC * 4;
-// SHACC, BETA, SHT after the compact layout, from the next 16-byte boundary (BETA is read as float4)
-constexpr size_t kBwdSmemFold = (kBwdSmemCompact + 15) / 16 * 16 + sizeof(float) * (TM * 16 + 2 * NH + 32);
-static_assert((TM * 16 * sizeof(float)) % 16 == 0, "BETA must stay 16-byte aligned after SHACC");
-static_assert(kBwdSmemFold <= 227 * 1024, "the folded adjoint's shared memory exceeds a CTA's");
-
+namespace vx {
 
 // Sum the per-block partials into dW0 (64,51), dW1 (3,64), db0 (64), db1 (3), in a fixed order
 // (deterministic): a block of 32 x 8 threads takes 32 consecutive elements; thread (x, y) sums
@@ -1296,41 +774,65 @@ void launch_hash_rows(const HashArgs& a, cudaStream_t st) {
   kern<<<grid_for((a.P + kRowsPerBlock - 1) / kRowsPerBlock * 256, 256, rows_per_sm[compact]), 256, 0, st>>>(a);
 }
 
+template <bool kMask>
+auto rows2_kernel(bool fold, bool compact, bool cw) {
+  return fold      ? (cw ? k_mlp_fwd_rows2<true, true, true, kMask> : k_mlp_fwd_rows2<false, true, true, kMask>)
+         : compact ? (cw ? k_mlp_fwd_rows2<true, true, false, kMask> : k_mlp_fwd_rows2<false, true, false, kMask>)
+                   : (cw ? k_mlp_fwd_rows2<true, false, false, kMask> : k_mlp_fwd_rows2<false, false, false, kMask>);
+}
+
 template <bool kHashIn, bool kRowsOut>
-int launch_fwd(const HashArgs& a, const float* X, int64_t ldx, int64_t P, const MlpW& w, float* colors,
+int launch_fwd(const HashArgs& a, const float* X, int64_t ldx, int64_t P, const MlpW& w, const MlpOut& out,
                cudaStream_t st, RowSrc src = RowSrc{nullptr, 0}) {
   const int64_t tiles = (P + TM - 1) / TM;
   const bool compact = src.rays_d != nullptr;
+  const bool cw = custom_wait();
   if (!kHashIn && (compact || ldx == KP) && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {  // contiguous rows: two slots
     // compact rows whose tiles each lie inside one ray (samples per ray a multiple of the tile):
     // the folded MLP
     const bool fold = compact && src.S % TM == 0;
-    const bool cw = custom_wait();
-    auto kern2 = fold ? (cw ? k_mlp_fwd_rows2<true, true, true> : k_mlp_fwd_rows2<false, true, true>)
-                 : compact ? (cw ? k_mlp_fwd_rows2<true, true, false> : k_mlp_fwd_rows2<false, true, false>)
-                           : (cw ? k_mlp_fwd_rows2<true, false, false> : k_mlp_fwd_rows2<false, false, false>);
+    auto kern2 = out.mask ? rows2_kernel<true>(fold, compact, cw) : rows2_kernel<false>(fold, compact, cw);
     cudaError_t e = cudaFuncSetAttribute(kern2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
     if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
     const int64_t pairs = (tiles + 1) / 2;
     const unsigned blocks = (unsigned)(pairs < (int64_t)kSMs ? pairs : (int64_t)kSMs);
-    kern2<<<blocks, 512, kFwd2Smem, st>>>(X, P, w, colors, t_guard, src);
+    kern2<<<blocks, 512, kFwd2Smem, st>>>(X, P, w, out, t_guard, src);
     return VX_OK;
   }
-  auto kern = custom_wait() ? k_mlp_fwd_tc<kHashIn, kRowsOut, true> : k_mlp_fwd_tc<kHashIn, kRowsOut, false>;
+  auto kern = cw ? k_mlp_fwd_tc<kHashIn, kRowsOut, false, true> : k_mlp_fwd_tc<kHashIn, kRowsOut, false, false>;
+  if constexpr (!kHashIn)
+    if (out.mask) kern = cw ? k_mlp_fwd_tc<false, false, true, true> : k_mlp_fwd_tc<false, false, true, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
   if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
   const unsigned blocks = (unsigned)(tiles < (int64_t)kSMs * 2 ? tiles : (int64_t)kSMs * 2);
   const int xvec = X && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
-  kern<<<blocks, 256, kFwdSmem, st>>>(a, X, ldx, xvec, P, w, colors, t_guard);
+  kern<<<blocks, 256, kFwdSmem, st>>>(a, X, ldx, xvec, P, w, out, t_guard);
+  return VX_OK;
+}
+
+template <int kMode>
+int launch_adjoint(const float* x, int64_t ldx, int64_t P, const MlpW& w, const float* d_colors, const float* y,
+                   int64_t ldy, const uint32_t* mask, int64_t ldm, float* d_hash, float* d_normal, float* partials,
+                   int blocks, cudaStream_t st, RowSrc src, const char* what) {
+  constexpr int smem = (int)AdjShape<kMode>::kSmem;
+  auto kern = custom_wait() ? k_mlp_adjoint<kMode, true> : k_mlp_adjoint<kMode, false>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  kern<<<blocks, kAdjThreads, smem, st>>>(x, ldx, P, w, d_colors, y, ldy, mask, ldm, d_hash, d_normal, partials,
+                                          t_guard, src);
   return VX_OK;
 }
 
 // The adjoint and its weight-gradient reduction. Full rows (src.rays_d == nullptr, any stride
-// >= 51: 52-float contiguous rows take the bulk-copy kernel) or compact rows (bulk copy only).
+// >= 51: 52-float contiguous rows arrive by bulk copies) or compact rows (bulk copies only; folded
+// when the samples of a ray fill whole tiles, as in the forward). A caller without the forward's
+// mask (or colours) gets them from a forward launch that leaves them in d_hash's rows (words 0..1
+// and floats 2..4 of each), which the adjoint reads before it writes them.
 int mlp_backward_launch(const float* x, int64_t ldx, int64_t n_points, const float* W0, const float* b0,
-                        const float* W1, const float* b1, const float* d_colors, const float* colors, float* d_hash,
-                        float* d_normal, float* dW0, float* db0, float* dW1, float* db1, float* partials,
-                        int64_t n_partial_floats, cudaStream_t st, RowSrc src, const char* what) {
+                        const float* W1, const float* b1, const float* d_colors, const float* colors,
+                        const uint32_t* mask, float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1,
+                        float* db1, float* partials, int64_t n_partial_floats, cudaStream_t st, RowSrc src,
+                        const char* what) {
   VX_REQUIRE(x && W0 && b0 && W1 && b1 && d_colors && d_hash && d_normal && dW0 && db0 && dW1 && db1 && partials,
              "null pointer");
   VX_REQUIRE((reinterpret_cast<uintptr_t>(d_hash) & 15) == 0, "d_hash must be 16-byte aligned");
@@ -1339,26 +841,38 @@ int mlp_backward_launch(const float* x, int64_t ldx, int64_t n_points, const flo
              (long long)n_partial_floats, (long long)nb * WG);
   MlpW w{W0, b0, W1, b1};
   const bool compact = src.rays_d != nullptr;
+  int launches = 1;
   if (n_points > 0) {
-    const int xvec = (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    const bool bulk = xvec && (compact || ldx == KP);
-    // compact rows whose tiles each lie inside one ray: the folded MLP (as in the forward)
-    const bool fold = compact && src.S % TM == 0;
-    const size_t smem = fold ? kBwdSmemFold : compact ? kBwdSmemCompact : bulk ? kBwdSmemBulk : kBwdSmemRegs;
-    const bool cw = custom_wait();
-    auto kern = fold ? (cw ? k_mlp_bwd_tc<true, true, true, true> : k_mlp_bwd_tc<true, false, true, true>)
-                : compact ? (cw ? k_mlp_bwd_tc<true, true, true, false> : k_mlp_bwd_tc<true, false, true, false>)
-                : bulk ? (cw ? k_mlp_bwd_tc<true, true, false, false> : k_mlp_bwd_tc<true, false, false, false>)
-                       : (cw ? k_mlp_bwd_tc<false, true, false, false> : k_mlp_bwd_tc<false, false, false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    kern<<<nb, 256, smem, st>>>(x, ldx, xvec, n_points, w, d_colors, colors, d_hash, d_normal, partials, t_guard, src);
+    const float* y = colors;
+    int64_t ldy = NO, ldm = 2;
+    if (!mask || !colors) {
+      uint32_t* dm = reinterpret_cast<uint32_t*>(d_hash);
+      HashArgs none{};
+      if (int s = launch_fwd<false, false>(none, x, ldx, n_points, w, MlpOut{d_hash + 2, 32, dm, 32}, st, src)) return s;
+      mask = dm;
+      ldm = 32;
+      if (!colors) {
+        y = d_hash + 2;
+        ldy = 32;
+      }
+      ++launches;
+    }
+    const bool bulk = ldx == KP && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    // folded: whole tiles, each inside one ray, whose d_colors, colours and mask rows are bulk copies too
+    const bool fold = compact && src.S % TM == 0 && n_points % TM == 0 && ldy == NO && ldm == 2 &&
+                      ((reinterpret_cast<uintptr_t>(d_colors) | reinterpret_cast<uintptr_t>(y) |
+                        reinterpret_cast<uintptr_t>(mask)) & 15) == 0;
+    auto go = compact ? (fold ? launch_adjoint<kAdjFold> : launch_adjoint<kAdjCompact>)
+                      : (bulk ? launch_adjoint<kAdjFull> : launch_adjoint<kAdjStrided>);
+    if (int s = go(x, ldx, n_points, w, d_colors, y, ldy, mask, ldm, d_hash, d_normal, partials, nb, st, src, what))
+      return s;
+    ++launches;
   } else {
     cudaMemsetAsync(partials, 0, sizeof(float) * WG, st);
   }
   k_mlp_wgrad_reduce<<<(WG + 31) / 32, dim3(32, kReduceSlices), 0, st>>>(partials, n_points > 0 ? nb : 1, dW0, db0,
                                                                         dW1, db1);
-  count_launches(2);
+  count_launches(launches);
   return check_launch(what);
 }
 
@@ -1366,14 +880,12 @@ int mlp_backward_launch(const float* x, int64_t ldx, int64_t n_points, const flo
 
 using namespace vx;
 
-extern "C" {
-
-int vx_appearance_mlp_forward(const float* table, int n_levels, int log2_size, int n_features,
+static int appearance_forward(const float* table, int n_levels, int log2_size, int n_features,
                               const int32_t* level_res, const float* level_weights, const float* rays_o,
                               const float* rays_d, const float* mid, int n_samples, const float xyz_min[3],
                               const float xyz_max[3], int64_t n_points, const float* normals, const float* W0,
                               const float* b0, const float* W1, const float* b1, float* colors, float* rows,
-                              int64_t ld_rows, void* stream) {
+                              int64_t ld_rows, uint32_t* mask, void* stream) {
   HashArgs a{};
   if (int s = fill_hash(a, table, n_levels, log2_size, n_features, level_res, level_weights)) return s;
   VX_REQUIRE(n_levels == 16, "the fused appearance MLP takes 16 hash levels x 2 features (got %d)", n_levels);
@@ -1390,17 +902,53 @@ int vx_appearance_mlp_forward(const float* table, int n_levels, int log2_size, i
   a.ld = ld_rows;
   a.normals = normals;
   MlpW w{W0, b0, W1, b1};
+  const MlpOut out{colors, NO, mask, 2};
   cudaStream_t st = (cudaStream_t)stream;
   if (rows) {  // training: rows gathered at high occupancy, then the MLP on the rows
     launch_hash_rows(a, st);
     const RowSrc src{ld_rows == KC ? rays_d : nullptr, n_samples};
-    if (int s = launch_fwd<false, false>(a, rows, ld_rows, n_points, w, colors, st, src)) return s;
+    if (int s = launch_fwd<false, false>(a, rows, ld_rows, n_points, w, out, st, src)) return s;
     count_launches(2);
   } else {  // inference: features built in shared memory, nothing else written
-    if (int s = launch_fwd<true, false>(a, nullptr, 0, n_points, w, colors, st)) return s;
+    if (int s = launch_fwd<true, false>(a, nullptr, 0, n_points, w, out, st)) return s;
     count_launches(1);
   }
   return check_launch("appearance_mlp_forward");
+}
+
+static int radiance_forward(const float* x, int64_t ldx, int64_t n_points, const float* W0, const float* b0,
+                            const float* W1, const float* b1, float* colors, uint32_t* mask, void* stream) {
+  MlpW w{W0, b0, W1, b1};
+  HashArgs a{};
+  if (int s = launch_fwd<false, false>(a, x, ldx, n_points, w, MlpOut{colors, NO, mask, 2}, (cudaStream_t)stream))
+    return s;
+  count_launches(1);
+  return check_launch("radiance_mlp_forward");
+}
+
+extern "C" {
+
+int vx_appearance_mlp_forward(const float* table, int n_levels, int log2_size, int n_features,
+                              const int32_t* level_res, const float* level_weights, const float* rays_o,
+                              const float* rays_d, const float* mid, int n_samples, const float xyz_min[3],
+                              const float xyz_max[3], int64_t n_points, const float* normals, const float* W0,
+                              const float* b0, const float* W1, const float* b1, float* colors, float* rows,
+                              int64_t ld_rows, void* stream) {
+  return appearance_forward(table, n_levels, log2_size, n_features, level_res, level_weights, rays_o, rays_d, mid,
+                            n_samples, xyz_min, xyz_max, n_points, normals, W0, b0, W1, b1, colors, rows, ld_rows,
+                            nullptr, stream);
+}
+
+int vx_appearance_mlp_forward_masked(const float* table, int n_levels, int log2_size, int n_features,
+                                     const int32_t* level_res, const float* level_weights, const float* rays_o,
+                                     const float* rays_d, const float* mid, int n_samples, const float xyz_min[3],
+                                     const float xyz_max[3], int64_t n_points, const float* normals, const float* W0,
+                                     const float* b0, const float* W1, const float* b1, float* colors, float* rows,
+                                     int64_t ld_rows, uint32_t* relu_mask, void* stream) {
+  VX_REQUIRE(n_points <= 0 || (rows && relu_mask), "null pointer");
+  return appearance_forward(table, n_levels, log2_size, n_features, level_res, level_weights, rays_o, rays_d, mid,
+                            n_samples, xyz_min, xyz_max, n_points, normals, W0, b0, W1, b1, colors, rows, ld_rows,
+                            relu_mask, stream);
 }
 
 int vx_appearance_mlp_forward_chunked(const float* table, int n_levels, int log2_size, int n_features,
@@ -1439,7 +987,7 @@ int vx_appearance_mlp_forward_chunked(const float* table, int n_levels, int log2
     ac.normals = normals + 3 * c0;
     ac.P = len;
     launch_hash_rows(ac, st);
-    if (int s = launch_fwd<false, false>(ac, scratch_rows, KC, len, w, colors + 3 * c0, st,
+    if (int s = launch_fwd<false, false>(ac, scratch_rows, KC, len, w, MlpOut{colors + 3 * c0, NO, nullptr, 0}, st,
                                          RowSrc{ac.rays_d, n_samples}))
       return s;
     launches += 2;
@@ -1479,21 +1027,38 @@ int vx_radiance_mlp_forward(const float* x, int64_t ldx, int64_t n_points, int i
   VX_REQUIRE(n_points >= 0 && ldx >= KIN, "bad sizes");
   if (n_points == 0) return VX_OK;
   VX_REQUIRE(x && W0 && b0 && W1 && b1 && colors, "null pointer");
-  MlpW w{W0, b0, W1, b1};
-  HashArgs a{};
-  if (int s = launch_fwd<false, false>(a, x, ldx, n_points, w, colors, (cudaStream_t)stream)) return s;
-  count_launches(1);
-  return check_launch("radiance_mlp_forward");
+  return radiance_forward(x, ldx, n_points, W0, b0, W1, b1, colors, nullptr, stream);
+}
+
+int vx_radiance_mlp_forward_masked(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
+                                   const float* W0, const float* b0, const float* W1, const float* b1, float* colors,
+                                   uint32_t* relu_mask, void* stream) {
+  VX_REQUIRE(in_dim == KIN && hidden == NH && out_dim == NO, "the fused MLP is %d -> %d -> %d (got %d -> %d -> %d)",
+             KIN, NH, NO, in_dim, hidden, out_dim);
+  VX_REQUIRE(n_points >= 0 && ldx >= KIN, "bad sizes");
+  if (n_points == 0) return VX_OK;
+  VX_REQUIRE(x && W0 && b0 && W1 && b1 && colors && relu_mask, "null pointer");
+  return radiance_forward(x, ldx, n_points, W0, b0, W1, b1, colors, relu_mask, stream);
 }
 
 int vx_radiance_mlp_backward(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
                              const float* W0, const float* b0, const float* W1, const float* b1, const float* d_colors,
                              const float* colors, float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1,
                              float* db1, float* partials, int64_t n_partial_floats, void* stream) {
+  return vx_radiance_mlp_backward_masked(x, ldx, n_points, in_dim, hidden, out_dim, W0, b0, W1, b1, d_colors, colors,
+                                         nullptr, d_hash, d_normal, dW0, db0, dW1, db1, partials, n_partial_floats,
+                                         stream);
+}
+
+int vx_radiance_mlp_backward_masked(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
+                                    const float* W0, const float* b0, const float* W1, const float* b1,
+                                    const float* d_colors, const float* colors, const uint32_t* relu_mask,
+                                    float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1, float* db1,
+                                    float* partials, int64_t n_partial_floats, void* stream) {
   VX_REQUIRE(in_dim == KIN && hidden == NH && out_dim == NO, "the fused MLP is %d -> %d -> %d", KIN, NH, NO);
   VX_REQUIRE(n_points >= 0 && ldx >= KIN, "bad sizes");
-  return mlp_backward_launch(x, ldx, n_points, W0, b0, W1, b1, d_colors, colors, d_hash, d_normal, dW0, db0, dW1, db1,
-                             partials, n_partial_floats, (cudaStream_t)stream, RowSrc{nullptr, 0},
+  return mlp_backward_launch(x, ldx, n_points, W0, b0, W1, b1, d_colors, colors, relu_mask, d_hash, d_normal, dW0, db0,
+                             dW1, db1, partials, n_partial_floats, (cudaStream_t)stream, RowSrc{nullptr, 0},
                              "radiance_mlp_backward");
 }
 
@@ -1502,13 +1067,22 @@ int vx_appearance_mlp_backward(const float* rows, const float* rays_d, int n_sam
                                const float* d_colors, const float* colors, float* d_hash, float* d_normal, float* dW0,
                                float* db0, float* dW1, float* db1, float* partials, int64_t n_partial_floats,
                                void* stream) {
+  return vx_appearance_mlp_backward_masked(rows, rays_d, n_samples, n_points, W0, b0, W1, b1, d_colors, colors, nullptr,
+                                           d_hash, d_normal, dW0, db0, dW1, db1, partials, n_partial_floats, stream);
+}
+
+int vx_appearance_mlp_backward_masked(const float* rows, const float* rays_d, int n_samples, int64_t n_points,
+                                      const float* W0, const float* b0, const float* W1, const float* b1,
+                                      const float* d_colors, const float* colors, const uint32_t* relu_mask,
+                                      float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1, float* db1,
+                                      float* partials, int64_t n_partial_floats, void* stream) {
   VX_REQUIRE(n_points >= 0 && n_samples >= 1, "bad sizes");
   VX_REQUIRE(rays_d && rows, "null pointer");
   VX_REQUIRE(((uintptr_t)rows & 15) == 0, "compact rows must be 16-byte aligned");
   VX_REQUIRE(n_points < (int64_t(1) << 32), "compact rows take fewer than 2^32 samples");
-  return mlp_backward_launch(rows, KC, n_points, W0, b0, W1, b1, d_colors, colors, d_hash, d_normal, dW0, db0, dW1,
-                             db1, partials, n_partial_floats, (cudaStream_t)stream, RowSrc{rays_d, n_samples},
-                             "appearance_mlp_backward");
+  return mlp_backward_launch(rows, KC, n_points, W0, b0, W1, b1, d_colors, colors, relu_mask, d_hash, d_normal, dW0,
+                             db0, dW1, db1, partials, n_partial_floats, (cudaStream_t)stream,
+                             RowSrc{rays_d, n_samples}, "appearance_mlp_backward");
 }
 
 }  // extern "C"

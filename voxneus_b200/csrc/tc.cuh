@@ -1,13 +1,13 @@
 // tcgen05 (5th-generation tensor core) helpers for sm_100a: shared-memory matrix descriptors for
-// the no-swizzle canonical layouts, the kind::tf32 instruction descriptor, MMA issue/commit,
+// the no-swizzle canonical layouts, the kind::tf32 and kind::f16 instruction descriptors, MMA issue/commit,
 // TMEM allocation and loads, and bounded mbarrier waits. Inline PTX only.
 //
 // Canonical no-swizzle layouts (16-byte units, "core matrix" = 8 rows x 16 bytes, 128 bytes
 // contiguous, rows 16 bytes apart):
 //   K-major  operand (rows = M or N, 4 tf32 of K per 16 bytes): row groups of 8 are SBO bytes
 //            apart, 16-byte K chunks are LBO bytes apart.
-//   MN-major operand (8 K-rows of 4 consecutive M/N elements): 16-byte M/N chunks are SBO bytes
-//            apart, groups of 8 K-rows are LBO bytes apart.
+//   MN-major operand (16-bit types: 8 K-rows of 8 consecutive M/N elements): 16-byte M/N chunks are
+//            SBO bytes apart, groups of 8 K-rows are LBO bytes apart.
 #pragma once
 
 #include <cstdint>
@@ -34,6 +34,43 @@ constexpr uint32_t idesc_tf32(int M, int N, bool a_mn_major, bool b_mn_major) {
          (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
 
+// Instruction descriptor of kind::f16 with bf16 operands (format 1) and an f32 accumulator; the other
+// fields as above.
+constexpr uint32_t idesc_bf16(int M, int N, bool a_mn_major, bool b_mn_major) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
+         (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
+}
+
+// Issue by a converged warp: every lane runs the issue code (so its operands stay in uniform registers)
+// and `lead`, true in one lane, predicates the instruction itself. A branch taken by one thread makes
+// the compiler move each operand to a uniform register again: 78 cycles an MMA however small, against
+// 50 (M = 128, N = 64) and 62 (N = 112), what the operand reads take, issued this way (a probe of 256
+// dependent MMAs; the same for padded, unpadded and 128-byte-swizzled operands).
+__device__ __forceinline__ bool elect_lead() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+  return r != 0;
+}
+
+// D[tmem] (+)= A[smem] * B[smem]^T on bf16 operands (16 of K per instruction).
+__device__ __forceinline__ void mma_bf16_warp(bool lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(lead ? 1u : 0u));
+}
+
+// The same with A in tensor memory: row i in lane i, two consecutive K elements per column (8 columns
+// per instruction).
+__device__ __forceinline__ void mma_bf16_ts_warp(bool lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                 uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(lead ? 1u : 0u));
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          bool accumulate) {
@@ -57,6 +94,14 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
 __device__ __forceinline__ void commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+__device__ __forceinline__ void commit_warp(bool lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
+      "r"(lead ? 1u : 0u)
+      : "memory");
 }
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -137,27 +182,31 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float v[4]) {
   for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Store 32 consecutive f32 columns of this warp's 32 TMEM lanes (lane = thread); complete with
-// tmem_wait_st() before the values are read back.
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float v[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
+  uint32_t r[16];
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-      "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-      "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
-      "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
-      "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])), "r"(__float_as_uint(v[16])),
-      "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-      "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])),
-      "r"(__float_as_uint(v[23])), "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])),
-      "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])), "r"(__float_as_uint(v[28])),
-      "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
-      : "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float v[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Stores of consecutive f32 columns of this warp's 32 TMEM lanes (lane = thread); complete with
+// tmem_wait_st() before the values are read back.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float v[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "

@@ -536,20 +536,33 @@ MLP_LD_COMPACT = 36
 INFER_CHUNK_ROWS = 1 << 22
 
 
-def mlp_forward(rows: torch.Tensor, W0, b0, W1, b1) -> torch.Tensor:
-    """Fused radiance MLP on input rows (P, >=51) with any row stride: colours (P, 3)."""
+def mlp_forward(rows: torch.Tensor, W0, b0, W1, b1, mask: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Fused radiance MLP on input rows (P, >=51) with any row stride: colours (P, 3). mask: (P, 2)
+    int32 receiving the ReLU bits of the hidden layer (for mlp_backward)."""
     p = rows.shape[0]
     if rows.stride(1) != 1:
         raise RuntimeError("MLP rows must have unit column stride")
     out = torch.empty(p, 3, device=rows.device)
-    call("vx_radiance_mlp_forward", ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0],
-         ptr(W0.detach()), ptr(b0.detach()), ptr(W1.detach()), ptr(b1.detach()), ptr(out), stream_ptr(rows.device))
+    args = (ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0], ptr(W0.detach()), ptr(b0.detach()),
+            ptr(W1.detach()), ptr(b1.detach()), ptr(out))
+    if mask is None:
+        call("vx_radiance_mlp_forward", *args, stream_ptr(rows.device))
+    else:
+        call("vx_radiance_mlp_forward_masked", *args, ptr(_relu_mask(mask, p, rows.device)), stream_ptr(rows.device))
     return out
 
 
-def mlp_backward(rows, W0, b0, W1, b1, d_colors, colors=None, rays_d=None, n_samples=0):
+def _relu_mask(mask, p: int, dev):
+    check_tensor(mask, "relu_mask", dtype=torch.int32, device=dev)
+    if mask.numel() != 2 * p:
+        raise RuntimeError(f"relu_mask has {mask.numel()} elements, need {2 * p}")
+    return mask
+
+
+def mlp_backward(rows, W0, b0, W1, b1, d_colors, colors=None, rays_d=None, n_samples=0, mask=None):
     """colors: the forward's (P, 3) outputs (the adjoint then skips recomputing the output layer),
-    or None. rays_d given: rows are the compact rows of AppearanceMLPFn (P, 36) whose SH(d) the
+    or None. mask: the ReLU bits that forward wrote (the adjoint then recomputes nothing), or None.
+    rays_d given: rows are the compact rows of AppearanceMLPFn (P, 36) whose SH(d) the
     kernel recomputes from rays_d of row i's ray (i // n_samples)."""
     dev = rows.device
     p = rows.shape[0]
@@ -557,6 +570,8 @@ def mlp_backward(rows, W0, b0, W1, b1, d_colors, colors=None, rays_d=None, n_sam
         check_tensor(colors, "colors", device=dev)
         if colors.numel() != 3 * p:
             raise RuntimeError(f"colors has {colors.numel()} elements, need {3 * p}")
+    if mask is not None:
+        _relu_mask(mask, p, dev)
     nb = int(L.query("vx_mlp_blocks", p))
     nf = int(L.query("vx_mlp_partial_floats"))
     sc = Scratch.get(dev)
@@ -566,15 +581,15 @@ def mlp_backward(rows, W0, b0, W1, b1, d_colors, colors=None, rays_d=None, n_sam
     d_normal = torch.empty(p, 3, device=dev)
     dW0, db0, dW1, db1 = (torch.empty_like(t) for t in (W0, b0, W1, b1))
     weights = (ptr(W0.detach()), ptr(b0.detach()), ptr(W1.detach()), ptr(b1.detach()))
-    outs = (ptr(check_tensor(d_colors.contiguous(), "d_colors")), ptr(colors), ptr(d_hash), ptr(d_normal), ptr(dW0),
-            ptr(db0), ptr(dW1), ptr(db1), ptr(sc.mlp_partials), sc.mlp_partials.numel(), stream_ptr(dev))
+    outs = (ptr(check_tensor(d_colors.contiguous(), "d_colors")), ptr(colors), ptr(mask), ptr(d_hash), ptr(d_normal),
+            ptr(dW0), ptr(db0), ptr(dW1), ptr(db1), ptr(sc.mlp_partials), sc.mlp_partials.numel(), stream_ptr(dev))
     if rays_d is None:
-        call("vx_radiance_mlp_backward", ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0],
+        call("vx_radiance_mlp_backward_masked", ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0],
              *weights, *outs)
     else:
         if rows.shape[1] != MLP_LD_COMPACT or not rows.is_contiguous():
             raise RuntimeError(f"compact MLP rows must be contiguous ({MLP_LD_COMPACT} floats a row)")
-        call("vx_appearance_mlp_backward", ptr(rows), ptr(check_tensor(rays_d, "rays_d")), n_samples, p, *weights,
+        call("vx_appearance_mlp_backward_masked", ptr(rows), ptr(check_tensor(rays_d, "rays_d")), n_samples, p, *weights,
              *outs)
     return d_hash, d_normal, dW0, db0, dW1, db1
 
@@ -584,13 +599,15 @@ class RadianceMLPFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, rows, W0, b0, W1, b1):
-        ctx.save_for_backward(rows, W0, b0, W1, b1)
-        return mlp_forward(rows.detach(), W0, b0, W1, b1)
+        mask = torch.empty(rows.shape[0], 2, dtype=torch.int32, device=rows.device)
+        out = mlp_forward(rows.detach(), W0, b0, W1, b1, mask)
+        ctx.save_for_backward(rows, W0, b0, W1, b1, out, mask)
+        return out
 
     @staticmethod
     def backward(ctx, g):
-        rows, W0, b0, W1, b1 = ctx.saved_tensors
-        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows.detach(), W0, b0, W1, b1, g)
+        rows, W0, b0, W1, b1, out, mask = ctx.saved_tensors
+        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows.detach(), W0, b0, W1, b1, g, out.detach(), mask=mask)
         d_rows = None
         if ctx.needs_input_grad[0]:
             d_rows = torch.zeros(rows.shape, device=rows.device)
@@ -625,8 +642,10 @@ class AppearanceMLPFn(torch.autograd.Function):
         args = (ptr(embeddings.detach()), cfg.n_levels, cfg.log2_size, cfg.n_features, cfg._res_c,
                 cfg.level_weights(active_levels), ptr(rays_o), ptr(rays_d), ptr(mid), ns, f3(xyz_min), f3(xyz_max), p,
                 ptr(nrm), ptr(W0.detach()), ptr(b0.detach()), ptr(W1.detach()), ptr(b1.detach()), ptr(colors))
+        mask = None
         if rows is not None:
-            call("vx_appearance_mlp_forward", *args, ptr(rows), ld, stream_ptr(mid.device))
+            mask = torch.empty(p, 2, dtype=torch.int32, device=mid.device)
+            call("vx_appearance_mlp_forward_masked", *args, ptr(rows), ld, ptr(mask), stream_ptr(mid.device))
         else:  # inference: rows pass through an L2-sized scratch, whole rays at a time
             n_rows = max(ns, min(p, (INFER_CHUNK_ROWS // ns) * ns))
             scratch = torch.empty(n_rows, MLP_LD_COMPACT, device=mid.device)
@@ -634,6 +653,7 @@ class AppearanceMLPFn(torch.autograd.Function):
         ctx.save_for_backward(rays_o, rays_d, mid, W0, b0, W1, b1)
         ctx.rows = rows
         ctx.colors = colors if rows is not None else None  # the adjoint's sigmoid derivative reads them
+        ctx.mask = mask  # the hidden layer's ReLU bits
         ctx.handoff = handoff
         ctx.meta = (xyz_min, xyz_max, cfg, active_levels, embeddings.shape, normals.shape)
         return colors.reshape(nr, ns, 3)
@@ -643,12 +663,12 @@ class AppearanceMLPFn(torch.autograd.Function):
         rays_o, rays_d, mid, W0, b0, W1, b1 = ctx.saved_tensors
         xyz_min, xyz_max, cfg, active_levels, eshape, nshape = ctx.meta
         nr, ns = mid.shape
-        rows, colors = ctx.rows, ctx.colors
-        ctx.rows = ctx.colors = None
+        rows, colors, mask = ctx.rows, ctx.colors, ctx.mask
+        ctx.rows = ctx.colors = ctx.mask = None
         if rows is None:
             raise RuntimeError("AppearanceMLPFn: forward ran with keep_rows=False; no adjoint input kept")
         d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows, W0, b0, W1, b1, g.reshape(-1, 3), colors, rays_d,
-                                                            ns)
+                                                            ns, mask)
         d_emb = None
         if ctx.needs_input_grad[0]:
             d_emb = torch.zeros(eshape, device=g.device)
