@@ -29,7 +29,7 @@ constexpr int KIN = 51;  // input features
 constexpr int KP = 52;   // row width of the input rows (column 51 is padding)
 // Compact rows of the fused appearance path: [hash 32 | normal 3 | pad], 144 bytes. The 16 SH(d)
 // features (columns 32..47 of a full row) depend on the ray only. When a ray's samples fill whole
-// 128-row tiles the folded MLP (fold_col, fold_bias below) adds them as a per-ray hidden bias;
+// 128-row tiles the folded MLP (fold_col below) adds them as a per-ray hidden bias;
 // otherwise the MLP kernels rebuild them from the ray's direction while they stage a tile, the same
 // function on the same operands as the row writer, so that both layouts give the same bits.
 constexpr int KC = 36;
@@ -109,18 +109,10 @@ struct MlpW {
 
 // The folded MLP (compact rows whose 128-row tiles each lie inside one ray, so SH(d) is constant
 // over a tile): the 16 SH columns leave the contraction and become a per-ray bias of the hidden
-// layer, b0 + W0[:, 32:48] SH(d). Its input features are [hash 32 | normal 3 | 0 x 5], K = 40
+// layer, b0 + W0[:, 32:48] SH(d) (columns summed in order). Its input features are [hash 32 | normal 3 | 0 x 5], K = 40
 // (the adjoint puts a one after the normal).
 // Folded feature k comes from column fold_col(k) of W0 (-1: none).
 __device__ __forceinline__ int fold_col(int k) { return k < 32 ? k : (k < 35 ? 48 + (k - 32) : -1); }
-
-// The per-ray bias of hidden unit n: b0[n] + sum_k W0[n, 32 + k] sh[k], k = 0..15 in order.
-__device__ __forceinline__ float fold_bias(const MlpW& w, int n, const float sh[16]) {
-  float b = __ldg(w.b0 + n);
-#pragma unroll
-  for (int k = 0; k < 16; ++k) b = fmaf(__ldg(w.W0 + n * KIN + 32 + k), sh[k], b);
-  return b;
-}
 
 __device__ __forceinline__ uint32_t x_off(int f, int m) { return (uint32_t)((f * 16 + (m >> 3)) * 128 + (m & 7) * 16); }
 // row r of [W_hi; W_lo] (r < 64: hi of hidden unit r, else lo of hidden unit r - 64), feature k
@@ -211,18 +203,6 @@ __device__ __forceinline__ void issue_split(uint32_t t, uint32_t ah0, uint32_t a
     const uint64_t ah = tc::sdesc(ah0 + ks * 4096, 2048, 128), al = tc::sdesc(al0 + ks * 4096, 2048, 128);
     const uint64_t b = tc::sdesc(b0 + ks * 4096, 2048, 128);
     tc::mma_tf32(t, ah, b, kId128, ks > 0);
-    tc::mma_tf32(t, al, b, kId64, true);
-  }
-}
-
-// issue_split with the A hi part in tensor memory: A_hi's K elements in columns ah_tmem + 8*ks of the
-// sample lanes (the same products in the same order as issue_split).
-__device__ __forceinline__ void issue_split_ts(uint32_t t, uint32_t ah_tmem, uint32_t al0, uint32_t b0, int ksteps) {
-#pragma unroll 1
-  for (int ks = 0; ks < ksteps; ++ks) {
-    const uint64_t al = tc::sdesc(al0 + ks * 4096, 2048, 128);
-    const uint64_t b = tc::sdesc(b0 + ks * 4096, 2048, 128);
-    tc::mma_tf32_ts(t, ah_tmem + 8 * ks, b, kId128, ks > 0);
     tc::mma_tf32(t, al, b, kId64, true);
   }
 }
@@ -424,56 +404,84 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
 
 constexpr size_t kFwdSmem = 2 * kXBytes + kWBytes + sizeof(float) * (NH + NO * NH + 4 + 2 * TM * 4) + 16;
 
-// Forward on contiguous 52-float rows (ldx = 52, 16-byte aligned): one CTA of 512 threads per SM
-// holding two independent tile slots of 256 threads (slot s = threads 256 s ..), which share the
-// stacked weights and alternate on the tensor core. Each slot has its own X operand (the lo part in
-// shared memory, the hi part in TMEM columns 256 + 64 s, sample lanes, written with tcgen05.st),
-// its own 128 accumulator columns, and a row buffer that the next tile's rows reach by one bulk
-// copy, issued as soon as the slot has staged its current tile; a slot synchronises on its own
-// named barrier, so one slot's MMA wait overlaps the other's staging and epilogue. Row prefetch
-// through registers (the general kernel above) left every warp stalled on its 16-byte loads of 32
-// rows at a time.
-constexpr uint32_t kFwdSlotBytes = kXBytes + TM * KP * 4 + 2 * TM * 4 * 4;  // XL, rows, RED
-// shared head: W0 [hi; lo], b0, W1, b1, barriers, TMEM address, fail flags; slots from a 1 KB boundary
-constexpr size_t kFwd2Head =
-    1024 * ((kWBytes + sizeof(float) * (NH + NO * NH + 4) + 64 + 2 * NH * sizeof(float) + 1023) / 1024);
-// the folded MLP's per-ray hidden bias of each slot's tile: the last 2 x 64 floats of the head
-constexpr size_t kFwd2Beta = kFwd2Head - 2 * NH * sizeof(float);
-static_assert(kFwd2Beta >= kWBytes + sizeof(float) * (NH + NO * NH + 4) + 64, "forward head overlaps its bias");
-constexpr size_t kFwd2Smem = kFwd2Head + 2 * (size_t)kFwdSlotBytes;
-// one CTA per SM (it allocates all 512 TMEM columns): two would need <= 116 KB each
-static_assert(kFwd2Smem > 116 * 1024, "two forward CTAs would fit on an SM and contend for TMEM");
+// Forward on contiguous rows (52 floats, or compact): one CTA per SM holding two independent tile slots
+// of 256 worker threads, which share the stacked weights and the tensor core, and one issuing warp a slot
+// (16 + slot), which issues the slot's MMAs and row copies (issuing blocks while the tensor core's queue
+// is full; warp-issued, tc.cuh). A slot has two X operands (the lo part in shared memory, the hi part in
+// TMEM columns, sample lanes, written with tcgen05.st), one accumulator of 128 columns and one or two
+// row buffers that a bulk copy fills. A worker stages tile t+1 while the MMAs of tile t run, reads
+// Z(t) out, hands both facts to the issuing warp (one arrival a warp on `ready`) and forms the colours
+// while the MMAs of tile t+1 run, so no MMA is waited for unless the staging and the epilogue are
+// shorter. What bounds it: the latency of the workers' chain (rows -> parts, accumulators -> colours) at
+// 16 warps an SM, ~2,300 cycles a tile. 1,048,576 samples: 91 us (with masks 98; one X a slot, MMAs
+// issued by one of its threads between two barriers, ~115 cycles apart: 2,000 of a tile's 5,600 cycles in
+// its slot) -> 76 us; 61,440,000 samples 5.01 -> 3.89 ms.
+template <bool kCompact, bool kFold>
+struct FwdShape {
+  static constexpr int kLd = kCompact ? KC : KP;                 // floats per row
+  static constexpr int kKSteps = kFold ? 5 : 7;                  // of 8 features
+  static constexpr int kBufs = kFold ? 2 : 1;                    // row buffers a slot
+  static constexpr uint32_t kX = kKSteps * 2 * 2048;             // X_lo of a tile
+  static constexpr uint32_t kRows = TM * kLd * 4;
+  static constexpr uint32_t kOffHead = 16 * 2048;                // after W0 [hi; lo] (64 features)
+  static constexpr uint32_t kOffSh = kOffHead + 4 * (NH + NO * NH + 4);  // folded: W0's SH columns [16][64]
+  static constexpr uint32_t kOffBeta = kOffSh + (kFold ? 16 * NH * 4 : 0);    // folded: [slot][2][64]
+  static constexpr uint32_t kOffRed = kOffBeta + (kFold ? 2 * 2 * NH * 4 : 0);  // [slot][2][2][TM][4]
+  static constexpr uint32_t kOffBar = kOffRed + 2 * 2 * 2 * TM * 16;
+  static constexpr uint32_t kOffSlot = (kOffBar + 96 + 1023) / 1024 * 1024;
+  static constexpr uint32_t kSlot = 2 * kX + kBufs * kRows;
+  static constexpr uint32_t kSmem = kOffSlot + 2 * kSlot;
+};
+static_assert(FwdShape<true, true>::kSmem <= 227 * 1024 && FwdShape<false, false>::kSmem <= 227 * 1024,
+              "the forward's shared memory exceeds a CTA's");
+static_assert(FwdShape<true, true>::kSmem > 116 * 1024, "two forward CTAs would fit on an SM and contend for TMEM");
+static_assert(FwdShape<true, true>::kOffRed % 16 == 0 && FwdShape<true, true>::kOffBeta % 16 == 0 &&
+                  FwdShape<false, false>::kOffRed % 16 == 0 && FwdShape<true, true>::kRows % 128 == 0 &&
+                  FwdShape<false, false>::kRows % 128 == 0 && FwdShape<true, true>::kOffBar % 8 == 0 &&
+                  FwdShape<false, false>::kOffBar % 8 == 0,
+              "shared-memory alignment");
+constexpr int kFwdThreads = 512 + 64;
 
-__device__ __forceinline__ void slot_sync(int slot) {
-  asm volatile("bar.sync %0, 256;" ::"r"(1 + slot) : "memory");
+// A barrier of a slot's workers that also agrees on whether any of them gave up a wait.
+__device__ __forceinline__ bool slot_sync_or(int slot, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(v ? 1u : 0u), "r"(1 + slot)
+      : "memory");
+  return r != 0;
 }
 
 template <bool kCustomWait, bool kCompact, bool kFold, bool kMask>
-__global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restrict__ X, int64_t P, MlpW w, MlpOut out,
-                                                         TcGuard g, RowSrc src) {
+__global__ void __launch_bounds__(kFwdThreads, 1)
+    k_mlp_fwd_rows2(const float* __restrict__ X, int64_t P, MlpW w, MlpOut out, TcGuard g, RowSrc src) {
   static_assert(!kFold || kCompact, "the folded MLP reads compact rows");
-  constexpr int kLd = kCompact ? KC : KP;  // floats per row in global memory
+  using S = FwdShape<kCompact, kFold>;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t wait_limit = kCustomWait ? g.limit : kWaitLimit;
   uint8_t* W2 = smem;
-  float* B0 = reinterpret_cast<float*>(W2 + kWBytes);
+  float* B0 = reinterpret_cast<float*>(smem + S::kOffHead);
   float* W1s = B0 + NH;
   float* B1 = W1s + NO * NH;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(B1 + 4);  // [slot][mma, rows]
-  uint32_t* s_taddr = reinterpret_cast<uint32_t*>(bars + 4);
-  int* s_fail = reinterpret_cast<int*>(s_taddr + 1);  // [2]
-  const int tid = threadIdx.x, slot = tid >> 8, stid = tid & 255;
-  const int wid = stid >> 5, lane = tid & 31, q = wid & 3, hh = wid >> 2;
+  float* WSH = reinterpret_cast<float*>(smem + S::kOffSh);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // in a uniform register: warp-uniform branches
+  const bool issuer = warp >= 16;
+  const int slot = issuer ? warp - 16 : warp >> 3;
+  const int wid = warp & 7, q = wid & 3, hh = wid >> 2, stid = 32 * wid + lane;
   const int m = 32 * q + lane;  // this thread's sample in its slot's tile
-  uint8_t* SL = smem + kFwd2Head + (size_t)slot * kFwdSlotBytes;
-  float* BETA = reinterpret_cast<float*>(smem + kFwd2Beta) + NH * slot;  // kFold: this slot's tile's bias
-  uint8_t* XL = SL;
-  uint8_t* ROWS = XL + kXBytes;
-  float* RED = reinterpret_cast<float*>(ROWS + TM * KP * 4);  // [2][TM][4]
-  uint64_t* bar = bars + 2 * slot;
-  uint64_t* bar_rows = bar + 1;
-  // weights and each slot's X_lo feature chunks 13..15 (zero), by all 512 threads
-  for (int e = tid; e < NH * 64; e += blockDim.x) {
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kOffBar) + 4 * slot;
+  uint64_t* bar = bars;            // the slot's MMAs of a tile
+  uint64_t* ready = bars + 1;      // X of a tile staged and the previous Z read (8 arrivals)
+  uint64_t* bar_rows = bars + 2;   // [2]
+  volatile int* s_fail = reinterpret_cast<volatile int*>(smem + S::kOffBar + 64);  // [2]
+  uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem + S::kOffBar + 72);
+  uint8_t* SL = smem + S::kOffSlot + slot * S::kSlot;
+  uint8_t* ROWS = SL + 2 * S::kX;
+  float* RED = reinterpret_cast<float*>(smem + S::kOffRed) + slot * (2 * 2 * TM * 4);
+  float* BETA = reinterpret_cast<float*>(smem + S::kOffBeta) + slot * 2 * NH;
+  for (int e = tid; e < NH * 64; e += kFwdThreads) {
     const int n = e >> 6, k = e & 63;
     const int col = kFold ? fold_col(k) : (k < KIN ? k : -1);
     float h, l;
@@ -481,178 +489,197 @@ __global__ void __launch_bounds__(512, 1) k_mlp_fwd_rows2(const float* __restric
     *reinterpret_cast<float*>(W2 + w_off(n, k)) = h;
     *reinterpret_cast<float*>(W2 + w_off(NH + n, k)) = l;
   }
-  for (int e = stid; e < 3 * TM; e += 256)
-    *reinterpret_cast<float4*>(XL + x_off(13 + e / TM, e % TM)) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int i = tid; i < NH; i += blockDim.x) B0[i] = w.b0[i];
-  for (int i = tid; i < NO * NH; i += blockDim.x) W1s[i] = w.W1[i];
+  if (kFold)
+    for (int e = tid; e < 16 * NH; e += kFwdThreads) WSH[(e & 15) * NH + (e >> 4)] = w.W0[(e >> 4) * KIN + 32 + (e & 15)];
+  for (int i = tid; i < NH; i += kFwdThreads) B0[i] = w.b0[i];
+  for (int i = tid; i < NO * NH; i += kFwdThreads) W1s[i] = w.W1[i];
   if (tid < NO) B1[tid] = w.b1[tid];
-  if (stid == 0) {
+  if (issuer && lane == 0) {
     tc::mbar_init(bar, 1);
+    tc::mbar_init(ready, 8);
     tc::mbar_init(bar_rows, 1);
+    tc::mbar_init(bar_rows + 1, 1);
     s_fail[slot] = 0;
   }
-  if (tid < 32) tc::tmem_alloc(s_taddr, 512);
+  if (warp == 0) tc::tmem_alloc(s_taddr, 512);
+  tc::fence_smem_to_async();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tcol = *s_taddr + 128 * slot;       // Z accumulator (two halves)
-  const uint32_t acol = *s_taddr + 256 + 64 * slot;  // X_hi: feature f in column acol + f
+  const uint32_t tb = __shfl_sync(0xffffffffu, *s_taddr, 0);
+  const uint32_t tcol = tb + 128 * slot;        // Z accumulator (two halves)
+  const uint32_t acol = tb + 256 + 128 * slot;  // X_hi: feature f of buffer b in column acol + 64 b + f
   const uint32_t lane_base = (uint32_t)(32 * q) << 16;
-  const uint32_t xl = tc::smem_u32(XL), w2 = tc::smem_u32(W2);
   const int64_t ntiles = (P + TM - 1) / TM;
   const int64_t t0 = 2 * (int64_t)blockIdx.x + slot, tstride = 2 * (int64_t)gridDim.x;
-  auto fetch_rows = [&](int64_t t) {
-    const int64_t m0 = t * TM;
-    const uint32_t bytes = (uint32_t)(P - m0 < TM ? P - m0 : TM) * (uint32_t)(kLd * 4);
-    tc::mbar_arrive_expect_tx(bar_rows, bytes);
-    tc::bulk_g2s(ROWS, X + m0 * kLd, bytes, bar_rows);
-  };
-  // slot thread 0's bookkeeping for a give-up: a rows copy in flight and the mbarrier parity it
-  // completes, and whether its own wait on the slot's MMA gave up
-  bool rows_pending = false, mma_pending = false;
-  uint32_t rows_parity = 0;
-  if (stid == 0 && t0 < ntiles) {
-    fetch_rows(t0);
-    rows_pending = true;
-  }
-  uint32_t phase = 0, rphase = 0;
-  float dnx = 0.0f, dny = 0.0f, dnz = 0.0f;  // kFold, threads 0..63: this tile's ray direction
-  if (kFold && stid < NH && t0 < ntiles) {
-    const int64_t r = t0 * TM / src.S;
-    dnx = __ldg(src.rays_d + 3 * r);
-    dny = __ldg(src.rays_d + 3 * r + 1);
-    dnz = __ldg(src.rays_d + 3 * r + 2);
-  }
-  for (int64_t t = t0; t < ntiles; t += tstride) {
-    const int64_t m0 = t * TM;
-    const bool valid = m0 + m < P;
-    const bool got = tc::mbar_wait(bar_rows, rphase, wait_limit);
-    rphase ^= 1u;
-    if (!got) s_fail[slot] = 1;
-    slot_sync(slot);
-    if (s_fail[slot]) break;
-    if (stid == 0) rows_pending = false;
-    if constexpr (kFold) {  // rows -> X_hi / X_lo: [hash 32 | normal 3 | 0 | 0 x 4]
-      const float4* rrow = reinterpret_cast<const float4*>(ROWS + m * (kLd * 4));
-      const int c0 = hh ? 5 : 0;
-      float xh[20];  // features 4*c0 .. 4*c0 + 19
-#pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        const int c = c0 + j;
-        float4 u = (valid && c < 9) ? rrow[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (c == 8) u.w = 0.0f;
-        const float v[4] = {u.x, u.y, u.z, u.w};
-        float lo[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) tc::split_tf32(v[i], xh[4 * j + i], lo[i]);
-        *reinterpret_cast<float4*>(XL + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+  if (issuer) {
+    const bool lead = tc::elect_lead();
+    const uint64_t dal = tc::sdesc(tc::smem_u32(SL), 2048, 128), db = tc::sdesc(tc::smem_u32(W2), 2048, 128);
+    int n_mma = 0, n_rows[2] = {0, 0};
+    auto fetch_rows = [&](int64_t t, int buf) {
+      if (lead) {
+        const int64_t m0 = t * TM;
+        const uint32_t bytes = (uint32_t)(P - m0 < TM ? P - m0 : TM) * (uint32_t)(S::kLd * 4);
+        tc::mbar_arrive_expect_tx(bar_rows + buf, bytes);
+        tc::bulk_g2s(ROWS + buf * S::kRows, X + m0 * S::kLd, bytes, bar_rows + buf);
       }
-      const uint32_t ta = acol + lane_base + 4 * c0;  // stores aligned to their widths
-      if (hh == 0) {
-        tc::tmem_st16(ta, xh);
-        tc::tmem_st4(ta + 16, xh + 16);
-      } else {
-        tc::tmem_st4(ta, xh);
-        tc::tmem_st8(ta + 4, xh + 4);
-        tc::tmem_st8(ta + 12, xh + 12);
-      }
-      tc::tmem_wait_st();
-    } else {  // rows -> X_hi (TMEM) and X_lo (sample rows); column 51 zero (the padding column may hold anything)
-      const float4* rrow = reinterpret_cast<const float4*>(ROWS + m * (kLd * 4));
-      const int c0 = hh ? 7 : 0;
-      const float3 dir = stage_dir<kCompact>(src, m0 + m, valid && hh);
-      float xh[28];  // features 4*c0 .. 4*c0 + 27 (hh = 1: 28..55, with 52..55 the zero chunk 13)
+      ++n_rows[buf];
+    };
 #pragma unroll
-      for (int j = 0; j < 7; ++j) {
-        const int c = c0 + j;
-        if (c < 13) {
-          float4 u = valid ? x_chunk<kCompact>(rrow, hh, j, dir) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (c == 12) u.w = 0.0f;
-          const float v[4] = {u.x, u.y, u.z, u.w};
-          float lo[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) tc::split_tf32(v[i], xh[4 * j + i], lo[i]);
-          *reinterpret_cast<float4*>(XL + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) xh[4 * j + i] = 0.0f;
-        }
+    for (int b = 0; b < S::kBufs; ++b)
+      if (t0 + b * tstride < ntiles) fetch_rows(t0 + b * tstride, b);
+    int it = 0;
+    bool bad = false;
+    for (int64_t t = t0; t < ntiles; t += tstride, ++it) {
+      bool ok = tc::mbar_wait_unless(ready, it & 1, wait_limit, s_fail + slot);
+      if (__shfl_sync(0xffffffffu, (int)!ok, 0)) {
+        bad = true;
+        break;
       }
-      // stores aligned to their widths (the column base is a multiple of 64)
-      const uint32_t ta = acol + lane_base + 4 * c0;
-      if (hh == 0) {
-        tc::tmem_st16(ta, xh);
-        tc::tmem_st8(ta + 16, xh + 16);
-        tc::tmem_st4(ta + 24, xh + 24);
-      } else {
-        tc::tmem_st4(ta, xh);
-        tc::tmem_st16(ta + 4, xh + 4);
-        tc::tmem_st8(ta + 20, xh + 20);
-      }
-      tc::tmem_wait_st();
-    }
-    tc::fence_smem_to_async();
-    tc::fence_before_sync();
-    slot_sync(slot);
-    if (stid == 0) {
       tc::fence_after_sync();
-      issue_split_ts(tcol, acol, xl, w2, kFold ? 5 : 7);
-      tc::commit(bar);
-      if (t + tstride < ntiles) {  // ROWS has been read: bring this slot's next tile
-        fetch_rows(t + tstride);
-        rows_pending = true;
-        rows_parity = rphase;
+      const uint32_t ah = acol + 64 * (it & 1);
+      const uint64_t al = dal + (it & 1) * (S::kX / 16);
+      // Z = X W0^T: per step of 8 features X_hi [W_hi; W_lo] (N = 128) and X_lo W_hi (N = 64)
+#pragma unroll
+      for (int ks = 0; ks < S::kKSteps; ++ks) {
+        tc::mma_tf32_ts_warp(lead, tcol, ah + 8 * ks, db + ks * 256, kId128, ks > 0);
+        tc::mma_tf32_warp(lead, tcol, al + ks * 256, db + ks * 256, kId64, true);
       }
+      tc::commit_warp(lead, bar);
+      ++n_mma;
+      const int64_t tn = t + S::kBufs * tstride;  // the tile's rows have been read
+      if (tn < ntiles) fetch_rows(tn, S::kBufs == 2 ? it & 1 : 0);
     }
-    if (kFold && stid < NH) {  // the tile's hidden bias, while its MMA runs (read after the wait)
-      float sh[16];
-      sh16(dnx, dny, dnz, sh);
-      if (t + tstride < ntiles) {  // the direction of the slot's next tile's ray, a tile ahead
-        const int64_t r = (t + tstride) * TM / src.S;
+    if (bad && lane == 0) s_fail[slot] = 1;
+    // the workers leave on their own or see the flag; then nothing of this slot may still be in flight
+    tc::fence_before_sync();
+    __syncthreads();
+    if (s_fail[slot] && lane == 0) {
+      if (n_mma > 0) tc::mbar_wait(bar, (n_mma - 1) & 1, kDrainLimit);
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+        if (n_rows[b] > 0) tc::mbar_wait(bar_rows + b, (n_rows[b] - 1) & 1, kDrainLimit);
+      report_timeout(g.status);
+    }
+  } else {
+    float dnx = 0.0f, dny = 0.0f, dnz = 0.0f;  // kFold, threads 0..63: a tile's ray direction, a tile ahead
+    auto load_dir = [&](int64_t t) {
+      if (kFold && stid < NH) {
+        const int64_t r = t * TM / src.S;
         dnx = __ldg(src.rays_d + 3 * r);
         dny = __ldg(src.rays_d + 3 * r + 1);
         dnz = __ldg(src.rays_d + 3 * r + 2);
       }
-      BETA[stid] = fold_bias(w, stid, sh);
-    }
-    const bool ok = tc::mbar_wait(bar, phase, wait_limit);
-    phase ^= 1u;
-    if (!ok) {
-      s_fail[slot] = 1;
-      mma_pending = true;  // read by slot thread 0 only
-    }
-    slot_sync(slot);
-    if (s_fail[slot]) break;
-    tc::fence_after_sync();
-    float z[32];
-    tmem_ld_sum32(tcol + lane_base + 32 * hh, z);
-    float p0, p1, p2;
-    const uint32_t bits = colour_partial<kMask>(z, hh, kFold ? BETA : B0, W1s, p0, p1, p2);
-    if (kMask && valid) out.mask[(m0 + m) * out.ldm + hh] = bits;
-    float* r = RED + (hh * TM + m) * 4;
-    r[0] = p0;
-    r[1] = p1;
-    r[2] = p2;
-    tc::fence_before_sync();
-    slot_sync(slot);
-    if (stid < TM && m0 + stid < P) {
+    };
+    bool ok = true;  // no wait of this thread has given up
+    auto stage = [&](int64_t t, int i) {  // tile t, number i of this slot: rows -> X_hi / X_lo
+      const int buf = i & 1;
+      const bool valid = t * TM + m < P;
+      ok = tc::mbar_wait(bar_rows + (S::kBufs == 2 ? buf : 0), S::kBufs == 2 ? (i >> 1) & 1 : buf, wait_limit) && ok;
+      __syncwarp();
+      const float4* rrow = reinterpret_cast<const float4*>(ROWS + (S::kBufs == 2 ? buf : 0) * S::kRows + m * (S::kLd * 4));
+      uint8_t* XL = SL + buf * S::kX;
+      constexpr int kN = kFold ? 5 : 7;  // chunks of 4 features a thread
+      const int c0 = hh ? kN : 0;
+      float3 dir = make_float3(0.0f, 0.0f, 0.0f);
+      if (!kFold) dir = stage_dir<kCompact>(src, t * TM + m, valid && hh);
+      float xh[4 * kN];
 #pragma unroll
-      for (int c = 0; c < NO; ++c) {
-        const float o = (B1[c] + RED[stid * 4 + c]) + RED[(TM + stid) * 4 + c];
-        out.colors[(m0 + stid) * out.ldc + c] = sigmoidf_ref(o);
+      for (int j = 0; j < kN; ++j) {
+        const int c = c0 + j;
+        float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (kFold) {  // [hash 32 | normal 3 | 0 | 0 x 4]
+          if (valid && c < 9) u = rrow[c];
+          if (c == 8) u.w = 0.0f;
+        } else {  // column 51 zero (the padding column may hold anything), chunk 13 zero
+          if (valid && c < 13) u = x_chunk<kCompact>(rrow, hh, j, dir);
+          if (c == 12) u.w = 0.0f;
+        }
+        const float v[4] = {u.x, u.y, u.z, u.w};
+        float lo[4];
+#pragma unroll
+        for (int i4 = 0; i4 < 4; ++i4) tc::split_tf32(v[i4], xh[4 * j + i4], lo[i4]);
+        *reinterpret_cast<float4*>(XL + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      // stores aligned to their widths (the column base is a multiple of 64)
+      const uint32_t ta = acol + 64 * buf + lane_base + 4 * c0;
+      if (kFold && hh == 0) {
+        tc::tmem_st16(ta, xh);
+        tc::tmem_st4(ta + 16, xh + 16);
+      } else if (kFold) {
+        tc::tmem_st4(ta, xh);
+        tc::tmem_st8(ta + 4, xh + 4);
+        tc::tmem_st8(ta + 12, xh + 12);
+      } else if (hh == 0) {
+        tc::tmem_st16(ta, xh);
+        tc::tmem_st8(ta + 16, xh + 16);
+        tc::tmem_st4(ta + 24, xh + (kFold ? 0 : 24));
+      } else {
+        tc::tmem_st4(ta, xh);
+        tc::tmem_st16(ta + 4, xh + 4);
+        tc::tmem_st8(ta + 20, xh + (kFold ? 0 : 20));
+      }
+      if (kFold && stid < NH) {  // the tile's hidden bias
+        float sh[16];
+        sh16(dnx, dny, dnz, sh);
+        float b = B0[stid];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) b = fmaf(WSH[k * NH + stid], sh[k], b);
+        BETA[NH * buf + stid] = b;
+        if (t + tstride < ntiles) load_dir(t + tstride);
+      }
+      tc::tmem_wait_st();
+    };
+    auto tell = [&]() {  // to the issuing warp: what this warp wrote and read is done
+      tc::fence_smem_to_async();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(ready);
+    };
+    if (t0 < ntiles) {
+      load_dir(t0);
+      stage(t0, 0);
+      tell();
+      slot_sync_or(slot, false);  // the first tile's bias
+    }
+    int it = 0;
+    for (int64_t t = t0; t < ntiles; t += tstride, ++it) {
+      const int par = it & 1;
+      const int64_t m0 = t * TM;
+      const bool valid = m0 + m < P, more = t + tstride < ntiles;
+      if (more) stage(t + tstride, it + 1);
+      ok = tc::mbar_wait(bar, par, wait_limit) && ok;
+      __syncwarp();
+      tc::fence_after_sync();
+      float z[32];
+      tmem_ld_sum32(tcol + lane_base + 32 * hh, z);
+      if (more) tell();
+      float p0, p1, p2;
+      const uint32_t bits = colour_partial<kMask>(z, hh, kFold ? BETA + NH * par : B0, W1s, p0, p1, p2);
+      if (kMask && valid) out.mask[(m0 + m) * out.ldm + hh] = bits;
+      float* red = RED + par * (2 * TM * 4);
+      *reinterpret_cast<float4*>(red + (hh * TM + m) * 4) = make_float4(p0, p1, p2, 0.0f);
+      if (slot_sync_or(slot, !ok)) {
+        if (stid == 0) s_fail[slot] = 1;
+        break;
+      }
+      if (valid) {  // hh = 0: colours 0 and 1, hh = 1: colour 2
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int cc = 2 * hh + c;
+          if (cc < NO) {
+            const float o = (B1[cc] + red[m * 4 + cc]) + red[(TM + m) * 4 + cc];
+            out.colors[(m0 + m) * out.ldc + cc] = sigmoidf_ref(o);
+          }
+        }
       }
     }
-  }
-  if (stid == 0 && s_fail[slot]) {
-    // this slot's MMA and a rows copy into its buffer may still run: let them finish (bounded)
-    // before TMEM and shared memory are released
-    if (mma_pending) tc::mbar_wait(bar, phase ^ 1u, kDrainLimit);
-    if (rows_pending) tc::mbar_wait(bar_rows, rows_parity, kDrainLimit);
-    report_timeout(g.status);
+    tc::fence_before_sync();
+    __syncthreads();
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (tid < 32) tc::tmem_dealloc(*s_taddr, 512);
+  if (warp == 0) tc::tmem_dealloc(tb, 512);
 }
 
 }  // namespace vx
@@ -792,11 +819,14 @@ int launch_fwd(const HashArgs& a, const float* X, int64_t ldx, int64_t P, const 
     // the folded MLP
     const bool fold = compact && src.S % TM == 0;
     auto kern2 = out.mask ? rows2_kernel<true>(fold, compact, cw) : rows2_kernel<false>(fold, compact, cw);
-    cudaError_t e = cudaFuncSetAttribute(kern2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
+    const int smem = fold      ? (int)FwdShape<true, true>::kSmem
+                     : compact ? (int)FwdShape<true, false>::kSmem
+                               : (int)FwdShape<false, false>::kSmem;
+    cudaError_t e = cudaFuncSetAttribute(kern2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
     const int64_t pairs = (tiles + 1) / 2;
     const unsigned blocks = (unsigned)(pairs < (int64_t)kSMs ? pairs : (int64_t)kSMs);
-    kern2<<<blocks, 512, kFwd2Smem, st>>>(X, P, w, out, t_guard, src);
+    kern2<<<blocks, kFwdThreads, smem, st>>>(X, P, w, out, t_guard, src);
     return VX_OK;
   }
   auto kern = cw ? k_mlp_fwd_tc<kHashIn, kRowsOut, false, true> : k_mlp_fwd_tc<kHashIn, kRowsOut, false, false>;

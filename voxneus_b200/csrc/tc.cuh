@@ -71,6 +71,22 @@ __device__ __forceinline__ void mma_bf16_ts_warp(bool lead, uint32_t d_tmem, uin
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(lead ? 1u : 0u));
 }
 
+// kind::tf32 issued by a converged warp (8 of K per instruction), A in shared or tensor memory.
+__device__ __forceinline__ void mma_tf32_warp(bool lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(lead ? 1u : 0u));
+}
+__device__ __forceinline__ void mma_tf32_ts_warp(bool lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                 uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(lead ? 1u : 0u));
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          bool accumulate) {
@@ -78,16 +94,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint6
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u));
-}
-
-// D[tmem] (+)= A[tmem] * B[smem]^T, issued by one thread: A's row i in TMEM lane i, its K
-// elements in consecutive columns from a_tmem (8 columns per K step of kind::tf32).
-__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                            bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1u : 0u));
 }
 
 // Arrive on the mbarrier once every tcgen05 operation this thread issued so far has completed.
@@ -135,6 +141,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // Arrive on the mbarrier and add `bytes` to the transaction count its current phase waits for.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// mbar_wait that also gives up once *flag is set.
+__device__ __forceinline__ bool mbar_wait_unless(uint64_t* bar, uint32_t parity, uint32_t limit,
+                                                 const volatile int* flag) {
+  for (uint32_t i = 0; i < limit; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*flag) return false;
+  }
+  return false;
+}
+
+// One arrival (release: this thread's earlier writes are visible to a thread that sees the phase complete).
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Bulk (TMA, non-tensor) copy global -> this CTA's shared memory, completing `bytes` on the
