@@ -7,6 +7,7 @@ no CUDA device is present, every kernel-backed call raises RuntimeError.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from typing import Optional, Sequence
@@ -118,6 +119,7 @@ _RESTYPES = {
 
 _lib = None
 _lock = threading.Lock()
+_entry = {}  # entry points by name, filled once a CUDA device has been seen (call)
 
 
 def library_path() -> str:
@@ -180,8 +182,9 @@ def set_timer(timer: Optional[KernelTimer]) -> None:
 
 def call(name: str, *args):
     """Call an entry point; raise RuntimeError with the library's message on failure."""
-    lib = load()
-    fn = getattr(lib, name)
+    fn = _entry.get(name)
+    if fn is None:  # the library and device checks, once per entry point
+        fn = _entry[name] = getattr(load(), name)
     t = _timer
     if t is not None and t.wants(name):
         ext = torch.cuda.is_current_stream_capturing()
@@ -194,7 +197,7 @@ def call(name: str, *args):
     else:
         st = fn(*args)
     if st != 0:
-        msg = lib.vx_last_error().decode(errors="replace")
+        msg = load().vx_last_error().decode(errors="replace")
         raise RuntimeError(f"{name}: {msg}")
     return st
 
@@ -212,14 +215,23 @@ def launch_count() -> int:
 # ------------------------------------------------------------------ argument helpers ------
 
 
-def i3(v) -> ctypes.Array:
-    v = [int(x) for x in v]
+# The host triples of the calls (resolutions, bounds) repeat: built once per value, never written to.
+@functools.lru_cache(maxsize=512)
+def _i3(v: tuple) -> ctypes.Array:
     return (ctypes.c_int32 * 3)(*v)
 
 
-def f3(v) -> ctypes.Array:
-    v = [float(x) for x in v]
+@functools.lru_cache(maxsize=512)
+def _f3(v: tuple) -> ctypes.Array:
     return (ctypes.c_float * 3)(*v)
+
+
+def i3(v) -> ctypes.Array:
+    return _i3(tuple(map(int, v)))
+
+
+def f3(v) -> ctypes.Array:
+    return _f3(tuple(map(float, v)))
 
 
 def iarr(v) -> ctypes.Array:
@@ -241,11 +253,18 @@ class AdamSegment(ctypes.Structure):
 
 
 def ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def stream_ptr(device=None):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream of `device` (the current device when None) as an address."""
+    idx = device.index if isinstance(device, torch.device) else device
+    if not isinstance(idx, int):
+        if idx is not None:
+            idx = torch.device(idx).index
+        if idx is None:
+            idx = torch.cuda.current_device()
+    return torch._C._cuda_getCurrentRawStream(idx)
 
 
 def check_tensor(t: torch.Tensor, name: str, dtype=torch.float32, device=None, contiguous=True):

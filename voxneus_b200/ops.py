@@ -33,14 +33,15 @@ class Scratch:
 
     @classmethod
     def get(cls, device: torch.device) -> "Scratch":
-        dev = torch.device(device)
+        dev = device if isinstance(device, torch.device) else torch.device(device)
         idx = dev.index if dev.index is not None else torch.cuda.current_device()
-        key = (idx, torch.cuda.current_stream(idx).cuda_stream)
-        with cls._lock:
-            s = cls._pool.get(key)
-            if s is None:
-                s = cls(torch.device("cuda", idx))
-                cls._pool[key] = s
+        key = (idx, stream_ptr(dev))
+        s = cls._pool.get(key)
+        if s is None:
+            with cls._lock:
+                s = cls._pool.get(key)
+                if s is None:
+                    s = cls._pool[key] = cls(torch.device("cuda", idx))
         return s
 
     def partials_for(self, n: int) -> torch.Tensor:
@@ -243,7 +244,7 @@ _TABLES: Dict[Tuple, torch.Tensor] = {}
 
 def linspace_table(a: float, b: float, n: int, device) -> torch.Tensor:
     """torch.linspace values on the device (cached): the tables the sampler kernel reads."""
-    key = (float(a), float(b), int(n), str(device))
+    key = (float(a), float(b), int(n), device if isinstance(device, torch.device) else torch.device(device))
     t = _TABLES.get(key)
     if t is None:
         t = torch.linspace(a, b, steps=n, device=device, dtype=torch.float32)
@@ -494,6 +495,7 @@ class HashConfig:
         self.resolutions = [math.floor(base * (b ** lvl)) for lvl in range(n_levels)]
         self._res_c = L.iarr(self.resolutions)
         self._dev_tables: Dict[tuple, tuple] = {}
+        self._weights = None
 
     def device_tables(self, dev, level_weights):
         """(resolutions int32, level weights float32) on `dev`, cached per weights. Uploaded from
@@ -510,6 +512,14 @@ class HashConfig:
         return t[0], t[1]
 
     def level_weights(self, active_levels: Optional[float]):
+        if active_levels is not None and not isinstance(active_levels, (int, float)):
+            return self._level_weights(active_levels)
+        last = self._weights  # the previous call's (level count, weights): one tuple, read once; never written to
+        if last is None or last[0] != active_levels:
+            last = self._weights = (active_levels, self._level_weights(active_levels))
+        return last[1]
+
+    def _level_weights(self, active_levels: Optional[float]):
         w = []
         for lvl in range(self.n_levels):
             if active_levels is None:
@@ -543,8 +553,8 @@ def mlp_forward(rows: torch.Tensor, W0, b0, W1, b1, mask: Optional[torch.Tensor]
     if rows.stride(1) != 1:
         raise RuntimeError("MLP rows must have unit column stride")
     out = torch.empty(p, 3, device=rows.device)
-    args = (ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0], ptr(W0.detach()), ptr(b0.detach()),
-            ptr(W1.detach()), ptr(b1.detach()), ptr(out))
+    args = (ptr(rows), rows.stride(0), p, rows.shape[1], W0.shape[0], W1.shape[0], ptr(W0), ptr(b0),
+            ptr(W1), ptr(b1), ptr(out))
     if mask is None:
         call("vx_radiance_mlp_forward", *args, stream_ptr(rows.device))
     else:
@@ -580,7 +590,7 @@ def mlp_backward(rows, W0, b0, W1, b1, d_colors, colors=None, rays_d=None, n_sam
     d_hash = torch.empty(p, 32, device=dev)
     d_normal = torch.empty(p, 3, device=dev)
     dW0, db0, dW1, db1 = (torch.empty_like(t) for t in (W0, b0, W1, b1))
-    weights = (ptr(W0.detach()), ptr(b0.detach()), ptr(W1.detach()), ptr(b1.detach()))
+    weights = (ptr(W0), ptr(b0), ptr(W1), ptr(b1))
     outs = (ptr(check_tensor(d_colors.contiguous(), "d_colors")), ptr(colors), ptr(mask), ptr(d_hash), ptr(d_normal),
             ptr(dW0), ptr(db0), ptr(dW1), ptr(db1), ptr(sc.mlp_partials), sc.mlp_partials.numel(), stream_ptr(dev))
     if rays_d is None:
@@ -639,9 +649,9 @@ class AppearanceMLPFn(torch.autograd.Function):
         rows = torch.empty(p, ld, device=mid.device) if need_rows else None
         nrm = normals.detach().contiguous()
         colors = torch.empty(p, 3, device=mid.device)
-        args = (ptr(embeddings.detach()), cfg.n_levels, cfg.log2_size, cfg.n_features, cfg._res_c,
+        args = (ptr(embeddings), cfg.n_levels, cfg.log2_size, cfg.n_features, cfg._res_c,
                 cfg.level_weights(active_levels), ptr(rays_o), ptr(rays_d), ptr(mid), ns, f3(xyz_min), f3(xyz_max), p,
-                ptr(nrm), ptr(W0.detach()), ptr(b0.detach()), ptr(W1.detach()), ptr(b1.detach()), ptr(colors))
+                ptr(nrm), ptr(W0), ptr(b0), ptr(W1), ptr(b1), ptr(colors))
         mask = None
         if rows is not None:
             mask = torch.empty(p, 2, dtype=torch.int32, device=mid.device)
@@ -688,7 +698,7 @@ class HashEncodeFn(torch.autograd.Function):
         x = check_tensor(norm_xyz.detach().reshape(-1, 3).contiguous(), "norm_xyz")
         p = x.shape[0]
         out = torch.empty(p, 2 * cfg.n_levels, device=x.device)
-        call("vx_appearance_forward", ptr(embeddings.detach()), cfg.n_levels, cfg.log2_size, cfg.n_features,
+        call("vx_appearance_forward", ptr(embeddings), cfg.n_levels, cfg.log2_size, cfg.n_features,
              cfg._res_c, cfg.level_weights(active_levels), ptr(x), None, None, None, 1, None, None, p, ptr(out),
              2 * cfg.n_levels, -1, None, 0, -1, None, -1, stream_ptr(x.device))
         ctx.save_for_backward(x)
