@@ -285,6 +285,44 @@ __device__ __forceinline__ void eq7_gradient(const float* __restrict__ f, const 
   eq7_gradient_block(f, g, e, w, c, out);
 }
 
+// Whether the cell's whole Eq.7 stencil (its corners and their face neighbours) lies inside the grid.
+__device__ __forceinline__ bool eq7_interior(const Grid& g, const Eq7& e) {
+  return (unsigned)(e.x0 - 1) < (unsigned)(g.rx - 3) && (unsigned)(e.y0 - 1) < (unsigned)(g.ry - 3) &&
+         (unsigned)(e.z0 - 1) < (unsigned)(g.rz - 3);
+}
+
+// The gradient of an interior cell, still to be divided by 2 eps per axis; p points at its lower corner
+// in an array of row strides sx, sy (the grid, or a copy of a part of it), c holds its corner block. Every
+// difference spans two voxels, so the weights blend the differences and the division comes once per axis
+// (one rounding each instead of eight), with no index clamps and twelve column addresses.
+__device__ __forceinline__ void eq7_blend_interior(const float* __restrict__ p, int sx, int sy, const float w[8],
+                                                   const float c[8], float out[3]) {
+  float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {  // column (x, y): corners k (z0) and k + 1 (z0 + 1)
+    const float* q = p + ((k & 4) ? sx : 0) + ((k & 2) ? sy : 0);
+    const float* qx = q + ((k & 4) ? sx : -sx);
+    const float* qy = q + ((k & 2) ? sy : -sy);
+    const float zm = q[-1], zp = q[2], x0 = qx[0], x1 = qx[1], y0 = qy[0], y1 = qy[1];
+    gx = fmaf(w[k], (k & 4) ? x0 - c[k ^ 4] : c[k ^ 4] - x0, gx);
+    gx = fmaf(w[k + 1], (k & 4) ? x1 - c[(k + 1) ^ 4] : c[(k + 1) ^ 4] - x1, gx);
+    gy = fmaf(w[k], (k & 2) ? y0 - c[k ^ 2] : c[k ^ 2] - y0, gy);
+    gy = fmaf(w[k + 1], (k & 2) ? y1 - c[(k + 1) ^ 2] : c[(k + 1) ^ 2] - y1, gy);
+    gz = fmaf(w[k], c[k + 1] - zm, gz);
+    gz = fmaf(w[k + 1], zp - c[k], gz);
+  }
+  out[0] = gx;
+  out[1] = gy;
+  out[2] = gz;
+}
+
+__device__ __forceinline__ void eq7_gradient_interior(const float* __restrict__ p, int sx, int sy, const Grid& g,
+                                                      const float w[8], const float c[8], float out[3]) {
+  eq7_blend_interior(p, sx, sy, w, c, out);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) out[a] = out[a] / (2.0f * g.eps[a]);
+}
+
 // query_sdf reusing an Eq.7 corner block: when grid_sample's cell is the same cell with all eight
 // corners inside the grid (interior points), its corner values are c (same accumulation order);
 // otherwise the corners are loaded.
