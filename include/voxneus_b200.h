@@ -124,12 +124,12 @@ int vx_field_query(const float* grid, const int32_t res[3], const float xyz_min[
                    float* weights, void* stream);
 
 /* vx_field_query's sdf, grad and normal outputs (models/sdf_grid.py:90-160) for a large batch of
- * scattered points, computed in spatial order: the points are sorted by the Morton code of their
- * grid cell, queried in that order and each result is written at the point's own index, so the
+ * scattered points, computed in spatial order: the points are brought into bricks of 16^3 grid
+ * cells, queried brick by brick and each result is written at the point's own index, so the
  * outputs are bit-identical to vx_field_query's. For grids larger than the L2 cache, where
- * scattered points read every stencil from a different DRAM row. n < 2^31; workspace: at least
- * vx_field_query_sorted_workspace(n, res) bytes, 256-byte aligned (0 when the size query fails,
- * which needs a CUDA device). */
+ * scattered points read every stencil from a different DRAM row. n < 2^31, taken 2^24 points at a
+ * time; workspace: at least vx_field_query_sorted_workspace(n, res) bytes, 256-byte aligned (52
+ * bytes a point of a pass and 20 a brick; 0 for sizes that the query refuses). */
 int64_t vx_field_query_sorted_workspace(int64_t n, const int32_t res[3]);
 int vx_field_query_sorted(const float* grid, const int32_t res[3], const float xyz_min[3], const float xyz_max[3],
                           const float* xyz, int64_t n, float* sdf, float* grad, float* normal, void* workspace,
