@@ -47,3 +47,23 @@ def test_brick_query_matches_plain(res, n, spread, offset):
             assert (y is None) == (not w)
             if w:
                 assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+
+
+@pytest.mark.parametrize("scale,bad", [(1.0, None), (1e-25, None), (0.0, None), (1e30, None), (1.0, float("inf")),
+                                       (1.0, float("nan"))])
+def test_brick_gradients_divide_as_the_plain_query(scale, bad):
+    """The differences' division by 2 eps from its reciprocal, and where that is left for the division:
+    vanishing, huge and non-finite values."""
+    from voxneus_b200 import ops
+
+    torch.manual_seed(3)
+    grid = torch.randn(1, 1, 61, 47, 52, device=DEV) * scale
+    if bad is not None:
+        grid.view(-1)[::977] = bad
+    lo, hi = (-1.0, -0.7, -1.3), (1.1, 0.9, 0.8)
+    pts = torch.rand(60_000, 3, device=DEV) * 2.0 - 1.0
+    a = ops.field_query(grid, lo, hi, pts, sdf=True, grad=True, normal=True)[:3]
+    b = ops.field_query_sorted(grid, lo, hi, pts, True, True, True)[:3]
+    for x, y in zip(a, b):
+        assert torch.equal(torch.isnan(x), torch.isnan(y))
+        assert torch.equal(x.nan_to_num(7.0, 1e38, -1e38), y.nan_to_num(7.0, 1e38, -1e38))

@@ -47,6 +47,9 @@ struct Grid {
   float inv_den[3];  // 1 / den when den is a power of two (exact), else 0
   float eps[3];  // voxel size (xyz_max - xyz_min) / (res - 1)
   float hi_clamp[3];  // float32(res - 1.0001): Eq.7 coordinate clamp (coordinates.py:73-75)
+  // an interior difference's denominator 2 eps and its reciprocal as a float plus a remainder; fd_r[0] = 0
+  // when some axis' values are outside the range of div_fd
+  float fd_d[3], fd_r[3], fd_rl[3];
 };
 
 // 1 / d when d is a power of two (then x / d == x * (1 / d) exactly for every float x), else 0.
@@ -62,6 +65,17 @@ __device__ __forceinline__ float div_den(float x, float den, float inv) {
   return inv != 0.0f ? __fmul_rn(x, inv) : __fdiv_rn(x, den);
 }
 
+// The fd_* members from eps.
+__host__ inline void set_fd(Grid& g) {
+  for (int a = 0; a < 3; ++a) {
+    g.fd_d[a] = 2.0f * g.eps[a];
+    g.fd_r[a] = (float)(1.0 / (double)g.fd_d[a]);
+    g.fd_rl[a] = (float)(1.0 / (double)g.fd_d[a] - (double)g.fd_r[a]);
+  }
+  for (int a = 0; a < 3; ++a)
+    if (!(g.fd_d[a] > 1e-6f && g.fd_d[a] < 1e6f)) g.fd_r[0] = 0.0f;
+}
+
 __host__ inline Grid make_grid(const int32_t res[3], const float lo[3], const float hi[3]) {
   Grid g;
   g.rx = res[0];
@@ -75,6 +89,7 @@ __host__ inline Grid make_grid(const int32_t res[3], const float lo[3], const fl
     g.eps[a] = span / ((float)res[a] - 1.0f);
     g.hi_clamp[a] = (float)((double)res[a] - 1.0001);
   }
+  set_fd(g);
   return g;
 }
 
@@ -227,6 +242,51 @@ __device__ __forceinline__ void eq7_load_block(const float* __restrict__ f, cons
     c[k] = __ldg(f + lin3(g, (k & 4) ? e.x1 : e.x0, (k & 2) ? e.y1 : e.y0, (k & 1) ? e.z1 : e.z0));
 }
 
+// Whether the cell's whole Eq.7 stencil (its corners and their face neighbours) lies inside the grid.
+__device__ __forceinline__ bool eq7_interior(const Grid& g, const Eq7& e) {
+  return (unsigned)(e.x0 - 1) < (unsigned)(g.rx - 3) && (unsigned)(e.y0 - 1) < (unsigned)(g.ry - 3) &&
+         (unsigned)(e.z0 - 1) < (unsigned)(g.rz - 3);
+}
+
+// x / d correctly rounded, from d's reciprocal as a float r and a remainder rl: x r + x rl is within one
+// unit in the last place of the quotient, and one correction with the exact residual then rounds it
+// correctly (Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM J.
+// Res. Dev. 34, 1990, theorem on division with a correctly rounded reciprocal). Holds while the residual
+// is representable (|x| >= 2^-100, or 0) and nothing overflows.
+__device__ __forceinline__ float div_fd(float x, float d, float r, float rl) {
+  const float q = fmaf(x, rl, x * r);
+  return fmaf(fmaf(-q, d, x), r, q);
+}
+
+// Eq.7 gradient of an interior cell, the values of eq7_gradient_block: p points at the cell's lower corner
+// in an array of row strides sx, sy, c holds its corner block. No index clamps, twelve column addresses, and
+// the 24 divisions by 2 eps from its reciprocal. Returns false where div_fd's range may not hold (values that
+// are infinite or not numbers, vanishing gradients): the caller then divides. For voxels in shared memory,
+// where issue bounds a query (602 -> 536 us for 2^24 points); reading the grid itself the loads bound it and
+// the second code path only costs registers (geometry of 2^20 samples: 93 us without, 94 us with).
+__device__ __forceinline__ bool eq7_gradient_columns(const float* __restrict__ p, int sx, int sy, const Grid& g,
+                                                     const float w[8], const float c[8], float out[3]) {
+  float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {  // column (x, y): corners k (z0) and k + 1 (z0 + 1)
+    const float* q = p + ((k & 4) ? sx : 0) + ((k & 2) ? sy : 0);
+    const float* qx = q + ((k & 4) ? sx : -sx);
+    const float* qy = q + ((k & 2) ? sy : -sy);
+    const float zm = q[-1], zp = q[2], x0 = qx[0], x1 = qx[1], y0 = qy[0], y1 = qy[1];
+    gx = fmaf(w[k], div_fd((k & 4) ? x0 - c[k ^ 4] : c[k ^ 4] - x0, g.fd_d[0], g.fd_r[0], g.fd_rl[0]), gx);
+    gy = fmaf(w[k], div_fd((k & 2) ? y0 - c[k ^ 2] : c[k ^ 2] - y0, g.fd_d[1], g.fd_r[1], g.fd_rl[1]), gy);
+    gz = fmaf(w[k], div_fd(c[k + 1] - zm, g.fd_d[2], g.fd_r[2], g.fd_rl[2]), gz);
+    gx = fmaf(w[k + 1], div_fd((k & 4) ? x1 - c[(k + 1) ^ 4] : c[(k + 1) ^ 4] - x1, g.fd_d[0], g.fd_r[0], g.fd_rl[0]), gx);
+    gy = fmaf(w[k + 1], div_fd((k & 2) ? y1 - c[(k + 1) ^ 2] : c[(k + 1) ^ 2] - y1, g.fd_d[1], g.fd_r[1], g.fd_rl[1]), gy);
+    gz = fmaf(w[k + 1], div_fd(zp - c[k], g.fd_d[2], g.fd_r[2], g.fd_rl[2]), gz);
+  }
+  out[0] = gx;
+  out[1] = gy;
+  out[2] = gz;
+  const float m = fabsf(gx) + fabsf(gy) + fabsf(gz);
+  return m >= 0x1p-60f && m < 0x1p100f;  // false for NaN
+}
+
 // Eq.7 gradient from the corner block c: per corner the central differences of Eq.6 (indices
 // clamped, one-sided at the border) blended with the corner weights. A corner's neighbour towards
 // the other side of the cell is a block value (the lower corner's +1 neighbour is the upper corner by
@@ -285,12 +345,6 @@ __device__ __forceinline__ void eq7_gradient(const float* __restrict__ f, const 
   eq7_gradient_block(f, g, e, w, c, out);
 }
 
-// Whether the cell's whole Eq.7 stencil (its corners and their face neighbours) lies inside the grid.
-__device__ __forceinline__ bool eq7_interior(const Grid& g, const Eq7& e) {
-  return (unsigned)(e.x0 - 1) < (unsigned)(g.rx - 3) && (unsigned)(e.y0 - 1) < (unsigned)(g.ry - 3) &&
-         (unsigned)(e.z0 - 1) < (unsigned)(g.rz - 3);
-}
-
 // The gradient of an interior cell, still to be divided by 2 eps per axis; p points at its lower corner
 // in an array of row strides sx, sy (the grid, or a copy of a part of it), c holds its corner block. Every
 // difference spans two voxels, so the weights blend the differences and the division comes once per axis
@@ -341,7 +395,8 @@ __device__ __forceinline__ float norm3(float x, float y, float z) { return sqrtf
 
 // normal = g / (|g| + 1e-8)  (gradients.py:136-137)
 __device__ __forceinline__ void normalize_eps(const float gr[3], float n[3], float& len) {
-  len = norm3(gr[0], gr[1], gr[2]);
+  // one order of fused products in every kernel, so that all of them give the same bits
+  len = sqrtf(fmaf(gr[2], gr[2], fmaf(gr[1], gr[1], gr[0] * gr[0])));
   const float d = len + 1e-8f;
   n[0] = gr[0] / d;
   n[1] = gr[1] / d;

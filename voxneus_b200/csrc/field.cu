@@ -331,6 +331,7 @@ static Grid grid_from_eps(const int32_t res[3], const float eps[3]) {
   const float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {1.f, 1.f, 1.f};
   Grid g = make_grid(res, lo, hi);
   for (int a = 0; a < 3; ++a) g.eps[a] = eps[a];
+  set_fd(g);
   return g;
 }
 

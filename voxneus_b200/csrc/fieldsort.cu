@@ -17,9 +17,9 @@
 //              inside the bucket's window
 //   collect    each point's result from its k: neighbours of a partition block read the same 256 runs
 // What bounds it: DRAM traffic (records, grid, results: ~180 bytes a point with normals and the grid once)
-// and, with normals, issue (24 IEEE divisions a point). 2^24 uniform points of a 512^3 grid, one query of
+// and, with normals, issue. 2^24 uniform points of a 512^3 grid, one query of
 // the SDF and one of gradient and normal: 4.40 ms (Morton keys, a four-pass radix sort, queries through
-// L1) -> 2.01 ms; with the points scattered to bricks in one step 3.03 ms.
+// L1) -> 1.94 ms; with the points scattered to bricks in one step 3.03 ms.
 #include "common.cuh"
 
 namespace vx {
@@ -36,7 +36,7 @@ constexpr int kCountThreads = 1024;
 constexpr int kBuckets = 256;               // at most
 // Bricks with at least this many points are staged, the others' points read the grid themselves: at 128 points
 // a brick (2^22 of a 512^3 grid) 341 us staged against 269 with normals and 194 against 116 without, at 512
-// points 602 against ~1080 and 270 against ~460. From a mean of kDenseMean on all are staged, which saves
+// points 536 against ~1080 and 270 against ~460. From a mean of kDenseMean on all are staged, which saves
 // the other pass over the records.
 constexpr int kDenseNormals = 160, kDenseSdf = 256, kDenseMean = 400;
 constexpr int kSmemBins = 48 * 1024;        // bins of a block's histogram in shared memory
@@ -324,7 +324,7 @@ __device__ __forceinline__ void store_normals(const float* f, const Grid& g, con
 }
 
 // One chunk of a brick per block: 34 KB of voxels and at most 64 registers keep four blocks or more on an SM,
-// one staging while others compute. 2^24 points: 602 us with normals (1.74 ms in Morton order through L1),
+// one staging while others compute. 2^24 points: 536 us with normals (1.74 ms in Morton order through L1),
 // 270 us without (1.08 ms). kNormals: the results of the record with place k go to res[2 k] = (normal,
 // sdf) and res[2 k + 1] = (gradient, 0), one 32-byte sector; otherwise its SDF to sdf[k].
 template <bool kNormals>
@@ -366,7 +366,6 @@ __global__ void __launch_bounds__(kQueryThreads, kNormals ? 4 : 6)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const float den[3] = {2.0f * g.eps[0], 2.0f * g.eps[1], 2.0f * g.eps[2]};  // fd_den of an interior difference
   for (int j = item.y + tid; j < end; j += kQueryThreads) {
     const float4 q = __ldg(rec + j);
     const int64_t at = __float_as_int(q.w);
@@ -395,22 +394,15 @@ __global__ void __launch_bounds__(kQueryThreads, kNormals ? 4 : 6)
     const bool in = e.x0 >= 1 && e.y0 >= 1 && e.z0 >= 1 && e.x0 + 2 < g.rx && e.y0 + 2 < g.ry && e.z0 + 2 < g.rz &&
                     e.x0 - 1 >= x_lo && e.y0 - 1 >= y_lo && e.z0 - 1 >= z_lo && e.x0 + 2 < x_lo + x_n &&
                     e.y0 + 2 < y_lo + y_n && e.z0 + 2 < z_lo + z_n;
+    bool done = false;
     if (in) {
       constexpr int sx = kReg * kPitch, sy = kPitch;
       const float* p = vox + (e.x0 - x_lo) * sx + (e.y0 - y_lo) * sy + (e.z0 - z_lo);
 #pragma unroll
       for (int k = 0; k < 8; ++k) c[k] = p[((k & 4) ? sx : 0) + ((k & 2) ? sy : 0) + (k & 1)];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {  // eq7_gradient_block of an interior cell: the same values and operations
-        const float* v = p + ((k & 4) ? sx : 0) + ((k & 2) ? sy : 0) + (k & 1);
-        const float dx = (k & 4) ? v[sx] - c[k ^ 4] : c[k ^ 4] - v[-sx];
-        const float dy = (k & 2) ? v[sy] - c[k ^ 2] : c[k ^ 2] - v[-sy];
-        const float dz = (k & 1) ? v[1] - c[k ^ 1] : c[k ^ 1] - v[-1];
-        gr[0] = fmaf(w[k], dx / den[0], gr[0]);
-        gr[1] = fmaf(w[k], dy / den[1], gr[1]);
-        gr[2] = fmaf(w[k], dz / den[2], gr[2]);
-      }
-    } else {
+      done = g.fd_r[0] != 0.0f && eq7_gradient_columns(p, sx, sy, g, w, c, gr);
+    }
+    if (!done) {
       eq7_load_block(f, g, e, c);
       eq7_gradient_block(f, g, e, w, c, gr);
     }

@@ -475,6 +475,7 @@ static Grid grid_eps(const int32_t res[3], const float eps[3]) {
   const float lo[3] = {0, 0, 0}, hi[3] = {1, 1, 1};
   Grid g = make_grid(res, lo, hi);
   for (int a = 0; a < 3; ++a) g.eps[a] = eps[a];
+  set_fd(g);
   return g;
 }
 
