@@ -163,6 +163,14 @@ __device__ __forceinline__ void gs_setup(const Grid& g, float px, float py, floa
 
 __device__ __forceinline__ float gs_sample(const float* __restrict__ f, const Grid& g, const Tri& t) {
   float acc = 0.0f;
+  if (t.inb == 0xffu) {  // all corners inside: fixed offsets from the lower one, no predicates
+    const float* p = f + lin3(g, t.x0, t.y0, t.z0);
+    const int sx = g.ry * g.rz, sy = g.rz;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      acc = fmaf(__ldg(p + ((k & 4) ? sx : 0) + ((k & 2) ? sy : 0) + (k & 1)), t.w[k], acc);
+    return acc;
+  }
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     if (t.inb & (1u << k)) {

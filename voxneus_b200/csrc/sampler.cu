@@ -1,10 +1,10 @@
 // The NeuS multistep sampler (rendering/sampler.py:11-204) as one warp per ray.
 //
-// A warp owns a ray: its z values and SDF values live in shared memory (up to 256 per ray),
-// every per-interval quantity is computed with lanes striding over the intervals, the
-// transmittance product, the pdf normalisation and the CDF are warp-shuffle scans over
-// 32-wide tiles, the inverse CDF is a binary search per new sample, and cat_z_vals'
-// sort becomes a rank sort of the <= 32 new samples plus a merge of two sorted lists.
+// A warp owns a ray: its z and SDF values live in shared memory (up to 256 per ray). For a step each lane
+// takes up to 8 consecutive intervals; the transmittance product, the pdf normalisation and the CDF are one
+// warp scan each, the inverse CDF is a binary search per new sample, and cat_z_vals' sort is the new
+// samples' order plus a merge of two sorted lists by masks. The module functions on a caller's own lists
+// (any length) walk them in tiles of 32.
 #include "common.cuh"
 
 namespace vx {
@@ -22,14 +22,11 @@ __device__ __forceinline__ void near_far(float ox, float oy, float oz, float dx,
 }
 
 struct WarpArrays {
-  float* z;    // current sorted z (n)
+  float* z;    // sorted z (n)
   float* f;    // SDF at z
-  float* z2;   // merge target
-  float* f2;
+  float* occ;  // occupancy factor per interval
   float* cdf;  // per-interval scratch, then the CDF (n entries)
   float* w;    // interval weights
-  float* nz;   // new samples (<= 32), sorted
-  float* nf;
 };
 
 __device__ __forceinline__ bool inside_unit(float ox, float oy, float oz, float dx, float dy, float dz, float t) {
@@ -90,7 +87,7 @@ __device__ void warp_sample_pdf(const WarpArrays& A, int n, int ns, const float*
 // up_sample (sampler.py:243-292): interval weights into A.w, then the inverse CDF. Whole-warp
 // chunks of 32 intervals: the inside-sphere test of z_{i+1} and the previous interval's cos come
 // from the neighbouring lane (the same expressions on the same operands), and the occupancy
-// factor 0.9 occ + 0.1 of each interval is looked up here, into A.z2, so that the serial scan
+// factor 0.9 occ + 0.1 of each interval is looked up here, into A.occ, so that the serial scan
 // below holds no global load.
 __device__ void warp_upsample_weights(const WarpArrays& A, int n, float inv_s, float ox, float oy, float oz, float dx,
                                       float dy, float dz, const Occ& oc, int lane) {
@@ -126,7 +123,7 @@ __device__ void warp_upsample_weights(const WarpArrays& A, int n, float inv_s, f
       if (oc.mask) {
         const float zm = (z0 + z1) * 0.5f;
         const float occ = occupied(oc, ray_at(ox, dx, zm), ray_at(oy, dy, zm), ray_at(oz, dz, zm)) ? 1.0f : 0.0f;
-        A.z2[i] = __fadd_rn(__fmul_rn(occ, 0.90f), 0.10f);
+        A.occ[i] = __fadd_rn(__fmul_rn(occ, 0.90f), 0.10f);
       }
     }
   }
@@ -142,7 +139,7 @@ __device__ void warp_upsample_weights(const WarpArrays& A, int n, float inv_s, f
     exc *= carry;
     if (i < nb) {
       float w = A.w[i] * (float)exc;
-      if (oc.mask) w = w * A.z2[i];
+      if (oc.mask) w = w * A.occ[i];
       A.w[i] = w;
     }
     carry *= __shfl_sync(0xffffffffu, inc, 31);
@@ -150,39 +147,140 @@ __device__ void warp_upsample_weights(const WarpArrays& A, int n, float inv_s, f
   __syncwarp();
 }
 
-// Rank-sort the ns (<= 32) new samples held by lanes < ns into A.nz/A.nf (ascending).
-__device__ __forceinline__ void warp_rank_sort_new(const WarpArrays& A, int ns, float v, float fv, int lane) {
-  int rank = 0;
-#pragma unroll 8
-  for (int k = 0; k < ns; ++k) {
-    const float o = __shfl_sync(0xffffffffu, v, k);
-    if (lane < ns) rank += (o < v) || (o == v && k < lane);
+// The multistep sampler's arrays of one ray.
+struct RayArrays {
+  float2* zf;   // current sorted z with the SDF there (n)
+  float2* zf2;  // merge target
+  float2* nz;   // new samples (<= 32), sorted
+  float* cdf;   // n entries
+};
+
+// One step's CDF: up_sample's interval weights (as warp_upsample_weights) and sample_pdf's normalised
+// running sum (as warp_sample_pdf). A lane takes K consecutive intervals (K * 32 >= n), so each scan is one
+// warp scan of the lanes' products or sums instead of one per 32 intervals. Products and sums are in double
+// and rounded once. The loops stay loops: unrolled for K = 2, 3, 4 and 8 with the intervals in registers the
+// kernel outgrew the instruction cache (65,536 rays 469 us against 392).
+__device__ __forceinline__ void ray_cdf(const RayArrays& A, int n, float inv_s, float ox, float oy, float oz, float dx,
+                                        float dy, float dz, const Occ& oc, int lane) {
+  const int nb = n - 1, K = (n + 31) >> 5, i0 = K * lane, i1 = min(i0 + K, nb);
+  auto inside = [&](float t) {  // |p| < 1 as |p|^2 < 1: the largest float below 1 has a square root that rounds below 1
+    const float x = ray_at(ox, dx, t), y = ray_at(oy, dy, t), z = ray_at(oz, dz, t);
+    return __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)) < 1.0f;
+  };
+  double run = 1.0;
+  if (i0 < nb) {
+    float2 a = A.zf[i0];
+    bool in0 = inside(a.x);
+    float prev = 0.0f;
+    if (i0 > 0) {
+      const float2 p = A.zf[i0 - 1];
+      prev = (a.y - p.y) / __fadd_rn(__fsub_rn(a.x, p.x), 1e-5f);
+    }
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i) {
+      const float2 b = A.zf[i + 1];
+      const bool in1 = inside(b.x);
+      const float dist = __fsub_rn(b.x, a.x), cosv = (b.y - a.y) / __fadd_rn(dist, 1e-5f);
+      float c = fminf(prev, cosv);
+      c = fminf(fmaxf(c, -1e3f), 0.0f) * (in0 || in1 ? 1.0f : 0.0f);
+      const float fm = (a.y + b.y) * 0.5f;
+      const float half = __fmul_rn(__fmul_rn(c, dist), 0.5f);
+      const float e0 = __fsub_rn(fm, half), e1 = __fadd_rn(fm, half);
+      const float c0 = sigmoidf_ref(e0 * inv_s), c1 = sigmoidf_ref(e1 * inv_s);
+      const float alpha = __fadd_rn(__fsub_rn(c0, c1), 1e-5f) / __fadd_rn(c0, 1e-5f);
+      A.cdf[i + 1] = alpha;
+      run *= (double)__fadd_rn(__fsub_rn(1.0f, alpha), 1e-7f);
+      prev = cosv;
+      in0 = in1;
+      a = b;
+    }
   }
-  if (lane < ns) {
-    A.nz[rank] = v;
-    A.nf[rank] = fv;
+  // T_i = prod_{j<i} (1 - alpha_j + 1e-7); w_i = alpha_i T_i
+  run = __shfl_up_sync(0xffffffffu, warp_incl_prod_d(run, lane), 1);
+  if (lane == 0) run = 1.0;
+  double part = 0.0;
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const float alpha = A.cdf[i + 1];
+    float w = __fmul_rn(alpha, (float)run);
+    run *= (double)__fadd_rn(__fsub_rn(1.0f, alpha), 1e-7f);
+    if (oc.mask) {
+      const float zm = (A.zf[i].x + A.zf[i + 1].x) * 0.5f;
+      const float occ = occupied(oc, ray_at(ox, dx, zm), ray_at(oy, dy, zm), ray_at(oz, dz, zm)) ? 1.0f : 0.0f;
+      w = __fmul_rn(w, __fadd_rn(__fmul_rn(occ, 0.90f), 0.10f));
+    }
+    w = __fadd_rn(w, 1e-5f);
+    A.cdf[i + 1] = w;
+    part += (double)w;
+  }
+  const float total = (float)warp_sum_d(part);
+  // cdf[0] = 0, cdf[i+1] = sum_{j<=i} w_j / total; the divisions from total's reciprocal
+  const float r = 1.0f / total, rl = fmaf(-total, r, 1.0f) * r;
+  double sum = 0.0;
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const float pdf = div_fd(A.cdf[i + 1], total, r, rl);
+    A.cdf[i + 1] = pdf;
+    sum += (double)pdf;
+  }
+  run = __shfl_up_sync(0xffffffffu, warp_incl_sum_d(sum, lane), 1);
+  if (lane == 0) {
+    run = 0.0;
+    A.cdf[0] = 0.0f;
+  }
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    run += (double)A.cdf[i + 1];
+    A.cdf[i + 1] = (float)run;
   }
   __syncwarp();
 }
 
-// Merge sorted A.z (n) with sorted A.nz (ns) into A.z2/A.f2 (ties: old first).
-__device__ __forceinline__ void warp_merge(const WarpArrays& A, int n, int ns, int lane) {
-  for (int i = lane; i < n; i += 32) {
-    const float zi = A.z[i];
-    int c = 0;
-    for (int k = 0; k < ns; ++k) c += (A.nz[k] < zi);
-    A.z2[i + c] = zi;
-    A.f2[i + c] = A.f[i];
+// The inverse CDF at u (sampler.py:40-66) and the place of the new sample among the n old ones (after equal
+// ones).
+__device__ __forceinline__ float ray_invert(const RayArrays& A, int n, float u, int& at) {
+  int lo = 0, hi = n;  // searchsorted(cdf, u, right=True)
+#pragma unroll 1
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (A.cdf[mid] <= u) lo = mid + 1; else hi = mid;
   }
-  if (lane < ns) {
-    const float v = A.nz[lane];
-    int lo = 0, hi = n;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (A.z[mid] <= v) lo = mid + 1; else hi = mid;
+  const int below = max(lo - 1, 0), above = min(lo, n - 1);
+  const float c0 = A.cdf[below], b0 = A.zf[below].x;
+  float den = A.cdf[above] - c0;
+  if (den < 1e-5f) den = 1.0f;
+  const float t = (u - c0) / den;
+  const float v = __fadd_rn(b0, __fmul_rn(t, __fsub_rn(A.zf[above].x, b0)));
+  while (lo < n && A.zf[lo].x <= v) ++lo;  // v lies in its bin up to a rounding or equal depths
+  while (lo > 0 && A.zf[lo - 1].x > v) --lo;
+  at = lo;
+  return v;
+}
+
+// cat_z_vals of the ns (<= 32) new samples (v with SDF fv, place `at` among the old) held by lanes < ns:
+// sorted old and new ones into A.zf2, old first at equal depths. Each 32 outputs learn from one mask which of
+// them are new.
+__device__ __forceinline__ void ray_merge(const RayArrays& A, int n, int ns, float v, float fv, int at, int lane) {
+  const float next = __shfl_down_sync(0xffffffffu, v, 1);
+  int rank = lane;
+  if (!__all_sync(0xffffffffu, lane >= ns - 1 || v <= next)) {  // evenly spaced u come in order
+    rank = 0;
+#pragma unroll 4
+    for (int k = 0; k < ns; ++k) {
+      const float o = __shfl_sync(0xffffffffu, v, k);
+      rank += (o < v) || (o == v && k < lane);
     }
-    A.z2[lane + lo] = v;
-    A.f2[lane + lo] = A.nf[lane];
+  }
+  if (lane < ns) A.nz[rank] = make_float2(v, fv);
+  const int p = lane < ns ? at + rank : 1 << 20;
+  __syncwarp();
+  int before = 0;
+#pragma unroll 1
+  for (int base = 0; base < n + ns; base += 32) {
+    const unsigned m = __reduce_or_sync(0xffffffffu, (unsigned)(p - base) < 32u ? 1u << (p - base) : 0u);
+    const int k = before + __popc(m & ((1u << lane) - 1u)), i = base + lane;
+    if (i < n + ns) A.zf2[i] = (m >> lane & 1u) ? A.nz[k] : A.zf[i - k];
+    before += __popc(m);
   }
   __syncwarp();
 }
@@ -205,14 +303,19 @@ struct SamplerArgs {
   float* mid;
 };
 
-__global__ void __launch_bounds__(128, 9) k_sample_multistep(SamplerArgs a, const float* __restrict__ fgrid, Grid g, Occ oc) {
-  extern __shared__ float smem[];
+// What bounds it: issue (a render), or the chain of one ray's steps when the rays are few. 64 + 64 samples, with
+// scans per 32 intervals and a merge by counting -> lanes of consecutive intervals and a merge by masks:
+// 480,000 rays 4.42 -> 2.96 ms, 2,048 rays 37 -> 28 us, 8,192 rays 104 -> 70 us.
+constexpr int sampler_floats(int n_total) { return 4 * n_total + 64 + (n_total + 1) / 2 * 2; }  // a warp
+
+__global__ void __launch_bounds__(128, 8) k_sample_multistep(SamplerArgs a, const float* __restrict__ fgrid, Grid g, Occ oc) {
+  extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int NT = a.n_total;
-  float* base = smem + warp * (6 * NT + 64);
-  WarpArrays A{base, base + NT, base + 2 * NT, base + 3 * NT, base + 4 * NT, base + 5 * NT, base + 6 * NT,
-               base + 6 * NT + 32};
+  float* base = smem + warp * sampler_floats(NT);
+  RayArrays A{reinterpret_cast<float2*>(base), reinterpret_cast<float2*>(base) + NT,
+              reinterpret_cast<float2*>(base) + 2 * NT, base + 4 * NT + 64};
   const int64_t wpb = blockDim.x >> 5;
   for (int64_t r = blockIdx.x * wpb + warp; r < a.n_rays; r += (int64_t)gridDim.x * wpb) {
     const float ox = a.rays_o[3 * r], oy = a.rays_o[3 * r + 1], oz = a.rays_o[3 * r + 2];
@@ -228,58 +331,51 @@ __global__ void __launch_bounds__(128, 9) k_sample_multistep(SamplerArgs a, cons
     // S0: stratified samples (sampler.py:85-125)
     for (int i = lane; i < n; i += 32) {
       const float t = a.t_lin[i];
-      A.z2[i] = __fadd_rn(__fmul_rn(nearv, __fsub_rn(1.0f, t)), __fmul_rn(farv, t));
+      A.cdf[i] = __fadd_rn(__fmul_rn(nearv, __fsub_rn(1.0f, t)), __fmul_rn(farv, t));
     }
     __syncwarp();
+    const bool up = a.n_importance > 0 && a.steps > 0;
+#pragma unroll 1
     for (int i = lane; i < n; i += 32) {
-      float zi = A.z2[i];
+      float zi = A.cdf[i];
       if (a.perturb) {
-        const float zl = A.z2[max(i - 1, 0)], zh = A.z2[min(i + 1, n - 1)];
+        const float zl = A.cdf[max(i - 1, 0)], zh = A.cdf[min(i + 1, n - 1)];
         const float upper = (i < n - 1) ? __fmul_rn(__fadd_rn(zh, zi), 0.5f) : zi;
         const float lower = (i > 0) ? __fmul_rn(__fadd_rn(zi, zl), 0.5f) : zi;
         zi = __fadd_rn(lower, __fmul_rn(__fsub_rn(upper, lower), a.t_rand[r * a.n_samples + i]));
       }
-      A.z[i] = zi;
+      A.zf[i] = make_float2(zi, up ? query_sdf(fgrid, g, ray_at(ox, dx, zi), ray_at(oy, dy, zi), ray_at(oz, dz, zi)) : 0.0f);
     }
     __syncwarp();
-    if (a.n_importance > 0 && a.steps > 0) {
-#pragma unroll 2
-      for (int i = lane; i < n; i += 32) {
-        const float t = A.z[i];
-        A.f[i] = query_sdf(fgrid, g, ray_at(ox, dx, t), ray_at(oy, dy, t), ray_at(oz, dz, t));
-      }
-      __syncwarp();
+    if (up) {
       for (int s = 0; s < a.steps; ++s) {
         const float inv_s = 64.0f * (float)(1 << s);
-        const float* u_ray = a.u ? a.u + ((int64_t)s * a.n_rays + r) * a.per_step : nullptr;
         // this lane's uniform, loaded before the weights so its latency is hidden
-        const float u_lane = lane < a.per_step ? (u_ray ? u_ray[lane] : a.u_det[lane]) : 0.0f;
-        warp_upsample_weights(A, n, inv_s, ox, oy, oz, dx, dy, dz, oc, lane);
-        float v;
-        int idx;
-        warp_sample_pdf(A, n, a.per_step, u_ray, a.u_det, u_lane, lane, nullptr, nullptr, v, idx);
-        const bool last = (s + 1 == a.steps);
-        float fv = 0.0f;
-        if (!last && lane < a.per_step) fv = query_sdf(fgrid, g, ray_at(ox, dx, v), ray_at(oy, dy, v), ray_at(oz, dz, v));
-        if (lane >= a.per_step) v = __int_as_float(0x7f800000);
-        warp_rank_sort_new(A, a.per_step, v, fv, lane);
-        warp_merge(A, n, a.per_step, lane);
+        float u = 0.0f;
+        if (lane < a.per_step) u = a.u ? a.u[((int64_t)s * a.n_rays + r) * a.per_step + lane] : a.u_det[lane];
+        ray_cdf(A, n, inv_s, ox, oy, oz, dx, dy, dz, oc, lane);
+        float v = __int_as_float(0x7f800000), fv = 0.0f;
+        int at = n;
+        if (lane < a.per_step) {
+          v = ray_invert(A, n, u, at);
+          if (s + 1 < a.steps) fv = query_sdf(fgrid, g, ray_at(ox, dx, v), ray_at(oy, dy, v), ray_at(oz, dz, v));
+        }
+        __syncwarp();
+        ray_merge(A, n, a.per_step, v, fv, at, lane);
         n += a.per_step;
-        float* t0 = A.z;
-        A.z = A.z2;
-        A.z2 = t0;
-        t0 = A.f;
-        A.f = A.f2;
-        A.f2 = t0;
+        float2* t0 = A.zf;
+        A.zf = A.zf2;
+        A.zf2 = t0;
       }
     }
     // S7 (sampler.py:197-202): dists with the last repeated, mid = z + dists/2
+#pragma unroll 1
     for (int i = lane; i < n; i += 32) {
-      const float zi = A.z[i];
+      const float zi = A.zf[i].x;
       float di;
       if (n == 1) di = __fdiv_rn(__fsub_rn(farv, nearv), 1.0f);
-      else if (i < n - 1) di = __fsub_rn(A.z[i + 1], zi);
-      else di = __fsub_rn(zi, A.z[i - 1]);
+      else if (i < n - 1) di = __fsub_rn(A.zf[i + 1].x, zi);
+      else di = __fsub_rn(zi, A.zf[i - 1].x);
       const int64_t o = r * n + i;
       if (a.z_out) a.z_out[o] = zi;
       a.dists[o] = di;
@@ -299,8 +395,7 @@ __global__ void __launch_bounds__(128) k_up_sample(const float* __restrict__ ray
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   float* base = smem + warp * (5 * n + 2);
-  // z, f, z2 (the intervals' occupancy factors), cdf, w
-  WarpArrays A{base, base + n, base + 4 * n + 2, nullptr, base + 2 * n, base + 3 * n, nullptr, nullptr};
+  WarpArrays A{base, base + n, base + 4 * n + 2, base + 2 * n, base + 3 * n};
   const int64_t wpb = blockDim.x >> 5;
   for (int64_t r = blockIdx.x * wpb + warp; r < n_rays; r += (int64_t)gridDim.x * wpb) {
     const float ox = rays_o[3 * r], oy = rays_o[3 * r + 1], oz = rays_o[3 * r + 2];
@@ -329,7 +424,7 @@ __global__ void __launch_bounds__(128) k_sample_pdf(const float* __restrict__ bi
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   float* base = smem + warp * (3 * n + 2);
-  WarpArrays A{base, nullptr, nullptr, nullptr, base + n, base + 2 * n, nullptr, nullptr};
+  WarpArrays A{base, nullptr, nullptr, base + n, base + 2 * n};
   const int64_t wpb = blockDim.x >> 5;
   for (int64_t r = blockIdx.x * wpb + warp; r < n_rays; r += (int64_t)gridDim.x * wpb) {
     for (int i = lane; i < n; i += 32) {
@@ -457,7 +552,7 @@ int vx_sample_multistep(const float* grid, const int32_t res[3], const float xyz
   Grid g = make_grid(res, xyz_min, xyz_max);
   Occ oc = make_occ(occupancy, occ_res, occ_min, occ_max);
   const int threads = 128;
-  const size_t smem = (size_t)(threads / 32) * (6 * total + 64) * sizeof(float);
+  const size_t smem = (size_t)(threads / 32) * sampler_floats(total) * sizeof(float);
   // a warp per ray up to 64 blocks a SM (9 are resident): one wave of persistent warps left some
   // warps two rays and others one; the block scheduler balances single-ray warps better
   k_sample_multistep<<<grid_for(n_rays * 32, threads, 64), threads, smem, (cudaStream_t)stream>>>(a, grid, g, oc);
