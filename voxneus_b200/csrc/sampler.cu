@@ -305,7 +305,7 @@ struct SamplerArgs {
 
 // What bounds it: issue (a render), or the chain of one ray's steps when the rays are few. 64 + 64 samples, with
 // scans per 32 intervals and a merge by counting -> lanes of consecutive intervals and a merge by masks:
-// 480,000 rays 4.42 -> 2.96 ms, 2,048 rays 37 -> 28 us, 8,192 rays 104 -> 70 us.
+// 480,000 rays 4.42 -> 2.96 ms, 2,048 rays 37 -> 28 us, 8,192 training rays 104 -> 76 us.
 constexpr int sampler_floats(int n_total) { return 4 * n_total + 64 + (n_total + 1) / 2 * 2; }  // a warp
 
 __global__ void __launch_bounds__(128, 8) k_sample_multistep(SamplerArgs a, const float* __restrict__ fgrid, Grid g, Occ oc) {
