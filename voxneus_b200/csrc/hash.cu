@@ -3,67 +3,108 @@
 // copy of the Eq.7 normal, written as one row per sample of the radiance MLP input
 // ([hash 32 | SH 16 | normal 3], models/radiance_mlp.py:94-98).
 //
-// One thread per sample, all levels in a loop: each thread writes its own row, the 8 corner
-// features of a level are float2 gathers from the (L, 2^19, 2) table (64 MiB at the default
-// size, L2-resident), and the adjoint scatters with float2 atomics (sm_90+ vector atomics).
+// Four threads per sample, a quarter of the levels each: the 8 corner features of a level are
+// gathers from the (L, 2^19, 2) table (64 MiB at the default size, L2-resident), and the adjoint
+// scatters with float2 and float4 atomics (sm_90+ vector atomics).
 // Hash indices are computed in uint32 arithmetic: the low log2(T) bits of
 // x*1 ^ y*2654435761 ^ z*805459861 equal the reference's int64 value modulo 2^log2(T).
 #include "hashgrid.cuh"
 
 namespace vx {
 
+// A block takes 64 rows, four threads each: thread group g encodes levels [g * lpt, (g + 1) * lpt), builds
+// the SH values 4g .. 4g+3 and group 1 copies the normal; the rows meet in shared memory and leave with
+// consecutive lanes on consecutive columns. Bound by the table's sector requests (L1 to L2). 200,003 points,
+// 11 of 16 levels open, with the SH of as many directions: 111 us with a thread a row (4-byte stores a row
+// apart, levels one after the other), 70 us so.
+constexpr int kAppRows = 64;
+
+__host__ __device__ inline int app_columns(const HashArgs& a) {
+  return (a.table ? 2 * a.L : 0) + (a.sh_col >= 0 ? 16 : 0) + (a.nrm_col >= 0 ? 3 : 0) + (a.pad_col >= 0 ? 1 : 0);
+}
+
 __global__ void __launch_bounds__(256) k_appearance_fwd(HashArgs a) {
+  extern __shared__ float srow[];  // [kAppRows][pitch]
   const uint32_t mask = (1u << a.log2T) - 1u;
   const size_t T = (size_t)1 << a.log2T;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.P; i += (int64_t)gridDim.x * blockDim.x) {
-    float* row = a.out + i * a.ld;
-    if (a.table) {
-      float x[3];
-      sample_pos(a, i, x);
-#pragma unroll 1
-      for (int l = 0; l < a.L; ++l) {
-        const float lw = a.lw[l];
-        if (lw == 0.0f) {
-          row[2 * l] = 0.0f;
-          row[2 * l + 1] = 0.0f;
-          continue;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = w >> 1;
+  const int ls = 32 * (w & 1) + lane;  // this thread's row in the block
+  const int ncol = app_columns(a), pitch = ncol | 1, lpt = (a.L + 3) >> 2;
+  const int sh0 = a.table ? 2 * a.L : 0, nrm0 = sh0 + (a.sh_col >= 0 ? 16 : 0), pad0 = nrm0 + (a.nrm_col >= 0 ? 3 : 0);
+  float* mine = srow + ls * pitch;
+  for (int64_t base = (int64_t)blockIdx.x * kAppRows; base < a.P; base += (int64_t)gridDim.x * kAppRows) {
+    const int64_t i = base + ls;
+    if (i < a.P) {
+      if (a.table) {
+        float x[3];
+        sample_pos(a, i, x);
+        const int l1 = min((g + 1) * lpt, a.L);
+#pragma unroll 4
+        for (int l = g * lpt; l < l1; ++l) {
+          const float lw = a.lw[l];
+          float f0 = 0.0f, f1 = 0.0f;
+          if (lw != 0.0f) {
+            LevelCell c;
+            level_cell(x, a.res[l], mask, c);
+            gather_level(reinterpret_cast<const float2*>(a.table) + (size_t)l * T, c, f0, f1);
+            if (lw < 1.0f) {
+              f0 *= lw;
+              f1 *= lw;
+            }
+          }
+          mine[2 * l] = f0;
+          mine[2 * l + 1] = f1;
         }
-        LevelCell c;
-        level_cell(x, a.res[l], mask, c);
-        const float2* tab = reinterpret_cast<const float2*>(a.table) + (size_t)l * T;
-        float f0 = 0.0f, f1 = 0.0f;
-        gather_level(tab, c, f0, f1);
-        if (lw < 1.0f) {
-          f0 *= lw;
-          f1 *= lw;
+      }
+      if (a.sh_col >= 0) {
+        float dx, dy, dz;
+        if (a.dirs) {
+          dx = a.dirs[i * a.dir_ss];
+          dy = a.dirs[i * a.dir_ss + 1];
+          dz = a.dirs[i * a.dir_ss + 2];
+        } else {
+          const int64_t r = i / a.S;
+          dx = __ldg(a.rays_d + 3 * r);
+          dy = __ldg(a.rays_d + 3 * r + 1);
+          dz = __ldg(a.rays_d + 3 * r + 2);
         }
-        row[2 * l] = f0;
-        row[2 * l + 1] = f1;
-      }
-    }
-    if (a.sh_col >= 0) {
-      float dx, dy, dz;
-      if (a.dirs) {
-        dx = a.dirs[i * a.dir_ss];
-        dy = a.dirs[i * a.dir_ss + 1];
-        dz = a.dirs[i * a.dir_ss + 2];
-      } else {
-        const int64_t r = i / a.S;
-        dx = __ldg(a.rays_d + 3 * r);
-        dy = __ldg(a.rays_d + 3 * r + 1);
-        dz = __ldg(a.rays_d + 3 * r + 2);
-      }
-      float o[16];
-      sh16(dx, dy, dz, o);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) row[a.sh_col + k] = o[k];
+        for (int k = 0; k < 4; ++k) {
+          if (g != k) continue;
+          const float4 v = sh_chunk(dx, dy, dz, k);
+          mine[sh0 + 4 * k] = v.x;
+          mine[sh0 + 4 * k + 1] = v.y;
+          mine[sh0 + 4 * k + 2] = v.z;
+          mine[sh0 + 4 * k + 3] = v.w;
+        }
+      }
+      if (a.nrm_col >= 0 && g == 1) {
+        mine[nrm0] = a.normals[3 * i];
+        mine[nrm0 + 1] = a.normals[3 * i + 1];
+        mine[nrm0 + 2] = a.normals[3 * i + 2];
+      }
+      if (a.pad_col >= 0 && g == 2) mine[pad0] = 0.0f;
     }
-    if (a.nrm_col >= 0) {
-      row[a.nrm_col] = a.normals[3 * i];
-      row[a.nrm_col + 1] = a.normals[3 * i + 1];
-      row[a.nrm_col + 2] = a.normals[3 * i + 2];
+    __syncthreads();
+    const int nrows = (int)(a.P - base < kAppRows ? a.P - base : kAppRows);
+    for (int c = lane; c < ncol; c += 32) {
+      int to = c;  // the value's column; of parts laid over one another the last stays
+      bool gone = false;
+      const bool pad = a.pad_col >= 0, nrm = a.nrm_col >= 0, sh = a.sh_col >= 0;
+      if (pad && c >= pad0) {
+        to = a.pad_col;
+      } else if (nrm && c >= nrm0) {
+        to = a.nrm_col + c - nrm0;
+        gone = pad && to == a.pad_col;
+      } else {
+        if (sh && c >= sh0) to = a.sh_col + c - sh0;
+        gone = (pad && to == a.pad_col) || (nrm && to >= a.nrm_col && to < a.nrm_col + 3) ||
+               (c < sh0 && sh && to >= a.sh_col && to < a.sh_col + 16);
+      }
+      if (!gone)
+        for (int r = w; r < nrows; r += 8) a.out[(base + r) * a.ld + to] = srow[r * pitch + c];
     }
-    if (a.pad_col >= 0) row[a.pad_col] = 0.0f;
+    __syncthreads();
   }
 }
 
@@ -146,7 +187,8 @@ int vx_appearance_forward(const float* table, int n_levels, int log2_size, int n
   a.nrm_col = normal_col;
   a.normals = normals;
   a.pad_col = pad_col;
-  k_appearance_fwd<<<grid_for(n_points, 256), 256, 0, (cudaStream_t)stream>>>(a);
+  const size_t smem = (size_t)kAppRows * (app_columns(a) | 1) * sizeof(float);  // at most 21 KB
+  k_appearance_fwd<<<grid_for((n_points + kAppRows - 1) / kAppRows * 256, 256, 32), 256, smem, (cudaStream_t)stream>>>(a);
   count_launches(1);
   return check_launch("appearance_forward");
 }
