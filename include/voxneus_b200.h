@@ -257,6 +257,11 @@ int vx_hash_encode_backward_det(float* table_grad, int n_levels, int log2_size, 
                                 const float xyz_min[3], const float xyz_max[3], int64_t n_points, const float* d_out,
                                 int64_t ld_d, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The radiance MLP's input rows (models/radiance_mlp.py:94-98) from contiguous parts: hash (n, 32), view
+ * (n, 16), normal (n, 3) -> rows (n, 52), the last column 0. rows: 16-byte aligned. */
+int vx_radiance_rows(const float* hash, const float* view, const float* normal, int64_t n_points, float* rows,
+                     void* stream);
+
 /* Radiance MLP (models/radiance_mlp.py:42-53,81-98): rows x (n_points, in_dim) with row stride
  * ldx -> Linear(51,64) -> ReLU -> Linear(64,3) -> Sigmoid -> colors (n_points, 3). W0 (64,51),
  * b0 (64), W1 (3,64), b1 (3) as nn.Linear stores them. Only the 51 -> 64 -> 3 shape is fused. */

@@ -54,3 +54,36 @@ def test_rows_of_parts(levels, p):
     want[:, 3:6] = nrm
     want[:, 4] = 0.0
     assert torch.equal(c, want)
+
+
+@pytest.mark.parametrize("p,offset,grads", [(1, 0, (True, True)), (127, 0, (True, False)), (129, 1, (False, True)),
+                                            (1000, 3, (True, True))])
+def test_radiance_parts_equal_rows(p, offset, grads):
+    """The module's separate inputs (contiguous, off 16 bytes, expanded) against the MLP on the same rows: the
+    same kernels, so the same bits; a part that takes no gradient gets none."""
+    from voxneus_b200 import ops
+    from voxneus_b200.models import RadianceMLP
+
+    gen = torch.Generator(device=DEV).manual_seed(p)
+    mlp = RadianceMLP().to(DEV)
+    ws = [mlp.net[0].weight, mlp.net[0].bias, mlp.net[2].weight, mlp.net[2].bias]
+    h = torch.randn(p * 32 + 4, device=DEV, generator=gen)[offset:offset + p * 32].view(p, 1, 32)
+    v = torch.randn(1, 1, 16, device=DEV, generator=gen).expand(p, 1, 16)
+    n = torch.randn(p, 1, 3, device=DEV, generator=gen)
+    h, n = h.detach().requires_grad_(grads[0]), n.requires_grad_(grads[1])
+    rows = torch.zeros(p, 52, device=DEV)
+    rows[:, :51] = torch.cat([h, v, n], -1).detach().view(p, 51)
+    x = rows[:, :51].requires_grad_(True)
+    cot = torch.randn(p, 3, device=DEV, generator=gen)
+    ref = ops.RadianceMLPFn.apply(x, *ws)
+    want = torch.autograd.grad((ref * cot).sum(), [x, *ws])
+    out = mlp(h, v, n)
+    assert out.shape == (p, 1, 3) and torch.equal(out.view(p, 3), ref)
+    (out.view(p, 3) * cot).sum().backward()
+    assert (h.grad is not None) == grads[0] and (n.grad is not None) == grads[1]
+    if grads[0]:
+        assert torch.equal(h.grad.view(p, 32), want[0][:, :32])
+    if grads[1]:
+        assert torch.equal(n.grad.view(p, 3), want[0][:, 48:51])
+    for w, g in zip(ws, want[1:]):
+        assert torch.equal(w.grad, g)

@@ -54,6 +54,7 @@ _PROTOS = {
     "vx_render_geometry_backward_det": [P, HI3, HF3, HF3, P, P, P, I64, I32, P, P, P, I64, P, P, SZ, P],
     "vx_hash_backward_det_workspace": [I64, I32, I32],
     "vx_hash_encode_backward_det": [P, I32, I32, I32, P, P, P, P, P, P, I32, HF3, HF3, I64, P, I64, P, SZ, P],
+    "vx_radiance_rows": [P, P, P, I64, P, P],
     "vx_radiance_mlp_forward": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P],
     "vx_radiance_mlp_forward_masked": [P, I64, I64, I32, I32, I32, P, P, P, P, P, P, P],
     "vx_appearance_mlp_forward_masked": [P, I32, I32, I32, HI3, HF3, P, P, P, I32, HF3, HF3, I64, P, P, P, P, P, P, P,

@@ -217,9 +217,14 @@ class RadianceMLP(nn.Module):
         embedding (SH of the ray directions) takes none, as in the reference's training."""
         if view_embeddings.requires_grad:
             raise NotImplementedError("the fused MLP adjoint gives no gradient for the view embedding")
-        x = torch.cat([hash_features, view_embeddings, normals], dim=-1)
-        lead = x.shape[:-1]
         l0, l1 = self.net[0], self.net[2]
+        parts = (hash_features, view_embeddings, normals)
+        lead = hash_features.shape[:-1]
+        if ([t.shape[-1] for t in parts] == [32, 16, 3] and all(t.shape[:-1] == lead for t in parts)
+                and all(t.dtype == torch.float32 and t.device == l0.weight.device for t in parts)):
+            return ops.RadiancePartsFn.apply(*parts, l0.weight, l0.bias, l1.weight, l1.bias).reshape(*lead, 3)
+        x = torch.cat(parts, dim=-1)
+        lead = x.shape[:-1]
         out = ops.RadianceMLPFn.apply(x.reshape(-1, x.shape[-1]), l0.weight, l0.bias, l1.weight, l1.bias)
         return out.reshape(*lead, 3)
 

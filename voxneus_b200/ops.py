@@ -635,6 +635,31 @@ class RadianceMLPFn(torch.autograd.Function):
         return d_rows, dW0, db0, dW1, db1
 
 
+class RadiancePartsFn(torch.autograd.Function):
+    """The radiance MLP on its separate inputs (..., 32), (..., 16), (..., 3), float32: rows assembled once in
+    the layout the MLP kernels copy whole, and the parts' gradients returned as the adjoint writes them."""
+
+    @staticmethod
+    def forward(ctx, hash_features, view, normals, W0, b0, W1, b1):
+        h, v, n = (t.detach().reshape(-1, t.shape[-1]).contiguous() for t in (hash_features, view, normals))
+        p = h.shape[0]
+        rows = torch.empty(p, MLP_LD, device=h.device)
+        call("vx_radiance_rows", ptr(h), ptr(v), ptr(n), p, ptr(rows), stream_ptr(h.device))
+        mask = torch.empty(p, 2, dtype=torch.int32, device=h.device)
+        out = mlp_forward(rows[:, :51], W0, b0, W1, b1, mask)
+        ctx.save_for_backward(rows, W0, b0, W1, b1, out, mask)
+        ctx.shapes = hash_features.shape, normals.shape
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        rows, W0, b0, W1, b1, out, mask = ctx.saved_tensors
+        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows[:, :51], W0, b0, W1, b1, g, out.detach(), mask=mask)
+        need = ctx.needs_input_grad
+        return (d_hash.reshape(ctx.shapes[0]) if need[0] else None, None,
+                d_normal.reshape(ctx.shapes[1]) if need[2] else None, dW0, db0, dW1, db1)
+
+
 class AppearanceMLPFn(torch.autograd.Function):
     """Hash encoding + SH + normal rows -> fused MLP -> colours for (rays, midpoints).
 
