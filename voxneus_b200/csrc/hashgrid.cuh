@@ -111,22 +111,6 @@ __device__ __forceinline__ void gather_level(const float2* __restrict__ tab, con
   }
 }
 
-// Adjoint of gather_level: one 16-byte atomic per x-pair when the cell's x index is even.
-__device__ __forceinline__ void scatter_level(float2* __restrict__ tab, const LevelCell& c, float g0, float g1) {
-  if (c.xpair) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float a0 = c.w[k] * g0, a1 = c.w[k] * g1, b0 = c.w[k + 4] * g0, b1 = c.w[k + 4] * g1;
-      const bool odd = c.h[k] & 1u;
-      atomicAdd(reinterpret_cast<float4*>(tab) + (c.h[k] >> 1),
-                odd ? make_float4(b0, b1, a0, a1) : make_float4(a0, a1, b0, b1));
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) atomicAdd(tab + c.h[k], make_float2(c.w[k] * g0, c.w[k] * g1));
-  }
-}
-
 // Degree-4 real spherical harmonics of a unit direction (models/embedder.py:55-87), four at a time:
 // values 4k .. 4k+3. k is a constant at every call (an unrolled loop), so only that group is built.
 // Every product and difference is rounded on its own, left to right as the reference's elementwise
