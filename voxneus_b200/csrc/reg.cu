@@ -13,6 +13,8 @@
 //    and narrow-band predicates, and |V_R| comes from the device-side counts.
 // Both forms also reduce the monitoring losses (mean over interior vertices) through
 // per-block partials and a last-block epilogue.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace vx {
@@ -182,59 +184,34 @@ __device__ __forceinline__ void tile_origin(const StencilArgs& a, int t, int& x0
   x0 = tx * TX;
 }
 
-// Does the halo-1 box of tile t hold any V_R vertex? Word-level test of the filtered bitmap by
-// one warp, one lane per (x, y) row of the box (z range [z0-1, z0+TZ] covers at most 3 words).
-__device__ __forceinline__ bool tile_has_bits_warp(const StencilArgs& a, const uint32_t* bm, int t, int lane) {
-  int x0, y0, z0;
-  tile_origin(a, t, x0, y0, z0);
-  bool hit = false;
-  for (int r = lane; r < MX * MY; r += 32) {
-    const int x = x0 - 1 + r / MY, y = y0 - 1 + r % MY;
-    if (x < 0 || x >= a.g.rx || y < 0 || y >= a.g.ry) continue;
-    const int zlo = max(z0 - 1, 0), zhi = min(z0 + TZ, a.g.rz - 1);
-    const int b0 = lin3(a.g, x, y, zlo), b1 = lin3(a.g, x, y, zhi);
-    for (int w = b0 >> 5; w <= (b1 >> 5); ++w) {
-      uint32_t m = 0xffffffffu;
-      if (w == (b0 >> 5)) m &= 0xffffffffu << (b0 & 31);
-      if (w == (b1 >> 5)) m &= 0xffffffffu >> (31 - (b1 & 31));
-      hit |= (__ldg(bm + w) & m) != 0u;
-    }
-  }
-  return __any_sync(0xffffffffu, hit);
-}
-
 struct StencilConsts {
   float inv_nv, dx, dy, dz, ex2, ey2, ez2, sc, w_eik;
 };
 
-// What active vertex (x, y, z) adds to itself (t0: curvature centre) and to its face neighbours
-// (tp[a] to v + e_a, tm[a] to v - e_a: eikonal +-scale n_a / (2 eps_a) plus curvature scale L_a /
-// eps_a^2), with scale = 2/|V_R| (1 - 1/(|n| + 1e-8)) w_eik and sc = 2/|V_R| w_curv
-// (eikonal_grad.cu, curvature_grad.cu); also its two loss terms.
+// What active vertex (x, y, z) adds to its face neighbours: e[a] + c[a] to v + e_a and c[a] - e[a] to v - e_a
+// (eikonal e = scale n_a / (2 eps_a), curvature c = scale L_a / eps_a^2), and -2 (c[0] + c[1] + c[2]) to
+// itself, with scale = 2/|V_R| (1 - 1/(|n| + 1e-8)) w_eik and sc = 2/|V_R| w_curv (eikonal_grad.cu,
+// curvature_grad.cu); also its two loss terms.
 __device__ __forceinline__ void vertex_terms(const StencilArgs& a, const StencilConsts& k, int x, int y, int z,
-                                             float& t0, float tp[3], float tm[3], double* loss) {
-  const float* f = a.f;
-  const int c = lin3(a.g, x, y, z);
+                                             float e[3], float c[3], double* loss) {
+  const float* f = a.f + lin3(a.g, x, y, z);
   const int sx = a.g.ry * a.g.rz, sy = a.g.rz;
-  const float fc = __ldg(f + c);
-  const float fxp = __ldg(f + c + sx), fxm = __ldg(f + c - sx);
-  const float fyp = __ldg(f + c + sy), fym = __ldg(f + c - sy);
-  const float fzp = __ldg(f + c + 1), fzm = __ldg(f + c - 1);
+  const float fc = __ldg(f);
+  const float fxp = __ldg(f + sx), fxm = __ldg(f - sx);
+  const float fyp = __ldg(f + sy), fym = __ldg(f - sy);
+  const float fzp = __ldg(f + 1), fzm = __ldg(f - 1);
   const float Lx = (fxp + fxm - 2.0f * fc) / k.ex2;
   const float Ly = (fyp + fym - 2.0f * fc) / k.ey2;
   const float Lz = (fzp + fzm - 2.0f * fc) / k.ez2;
   const float nx = (fxp - fxm) / k.dx, ny = (fyp - fym) / k.dy, nz = (fzp - fzm) / k.dz;
   const float len = sqrtf(nx * nx + ny * ny + nz * nz);
   const float se = k.inv_nv * (1.0f - 1.0f / (len + 1e-8f)) * k.w_eik;
-  const float ex = (se * nx) / k.dx, ey = (se * ny) / k.dy, ez = (se * nz) / k.dz;
-  const float cx = k.sc * (Lx / k.ex2), cy = k.sc * (Ly / k.ey2), cz = k.sc * (Lz / k.ez2);
-  t0 = k.sc * (-2.0f * Lx / k.ex2 - 2.0f * Ly / k.ey2 - 2.0f * Lz / k.ez2);
-  tp[0] = ex + cx;
-  tm[0] = -ex + cx;
-  tp[1] = ey + cy;
-  tm[1] = -ey + cy;
-  tp[2] = ez + cz;
-  tm[2] = -ez + cz;
+  e[0] = (se * nx) / k.dx;
+  e[1] = (se * ny) / k.dy;
+  e[2] = (se * nz) / k.dz;
+  c[0] = k.sc * (Lx / k.ex2);
+  c[1] = k.sc * (Ly / k.ey2);
+  c[2] = k.sc * (Lz / k.ez2);
   if (loss) {
     const double l = sqrt((double)nx * nx + (double)ny * ny + (double)nz * nz + 1e-16);
     loss[0] += (l - 1.0) * (l - 1.0);
@@ -263,55 +240,196 @@ __device__ __forceinline__ uint64_t column_window(const StencilArgs& a, const ui
   return v & keep;
 }
 
-__device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {
-  const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)v, src);
-  const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(v >> 32), src);
-  return (uint64_t)hi << 32 | lo;
-}
-
-// Does tile t own a vertex of the filtered V_R set? One thread per tile (its own voxels, no halo).
+// Does tile t own a vertex of the filtered V_R set? A lane per column, two tiles a warp (its own voxels, no
+// halo).
 __global__ void __launch_bounds__(256) k_tile_flags(StencilArgs a, int ntiles, uint8_t* __restrict__ flags) {
+  static_assert(TX * TY == 16, "half a warp a tile");
   const bool relax_on = a.relax_r > 0.0f && a.counts[1] > 0;
   const uint32_t* bm = a.fb + (relax_on ? a.nwords : 0);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
-    int x0, y0, z0;
-    tile_origin(a, t, x0, y0, z0);
+  const int lane = threadIdx.x & 31, q = lane & 15;
+  for (int t0 = 2 * (blockIdx.x * 8 + (threadIdx.x >> 5)); t0 < ntiles; t0 += 16 * gridDim.x) {
+    const int t = t0 + (lane >> 4);
     bool hit = false;
-    const int z1 = min(z0 + TZ, a.g.rz) - 1;
-    for (int q = 0; q < TX * TY && !hit; ++q) {
-      const int x = x0 + q / TY, y = y0 + q % TY;
-      if (x >= a.g.rx || y >= a.g.ry) continue;
-      const int b0 = lin3(a.g, x, y, z0), b1 = lin3(a.g, x, y, z1);
-      for (int w = b0 >> 5; w <= (b1 >> 5); ++w) {
-        uint32_t m = 0xffffffffu;
-        if (w == (b0 >> 5)) m &= 0xffffffffu << (b0 & 31);
-        if (w == (b1 >> 5)) m &= 0xffffffffu >> (31 - (b1 & 31));
-        hit |= (__ldg(bm + w) & m) != 0u;
+    if (t < ntiles) {
+      int x0, y0, z0;
+      tile_origin(a, t, x0, y0, z0);
+      const int x = x0 + q / TY, y = y0 + q % TY, z1 = min(z0 + TZ, a.g.rz) - 1;
+      if (x < a.g.rx && y < a.g.ry) {
+        const int b0 = lin3(a.g, x, y, z0), b1 = lin3(a.g, x, y, z1);
+        for (int w = b0 >> 5; w <= (b1 >> 5); ++w) {  // 32 bits: at most two words
+          uint32_t m = 0xffffffffu;
+          if (w == (b0 >> 5)) m &= 0xffffffffu << (b0 & 31);
+          if (w == (b1 >> 5)) m &= 0xffffffffu >> (31 - (b1 & 31));
+          hit |= (__ldg(bm + w) & m) != 0u;
+        }
       }
     }
-    flags[t] = hit ? 1 : 0;
+    const unsigned any = __ballot_sync(0xffffffffu, hit);
+    if (q == 0 && t < ntiles) flags[t] = (any >> (lane & 16) & 0xffffu) ? 1 : 0;
   }
 }
 
-// Fused eikonal + curvature gradient in gather form over 32x4x4 tiles. Warp w of the grid owns
-// tiles w, w + W, w + 2W, ... (W warps); its lanes test 32 of them at once against the flags of the
-// 3x3x3 tiles around each (a tile's outputs need the vertices of its halo), and the warp then
-// works through the tiles that need it, one at a time, lane = z offset. Lane c < 36 loads the V_R
-// window of column (x0 - 1 + c / 6, y0 - 1 + c % 6) of the tile's halo; each output voxel reads its
-// 7 neighbour bits from those windows (warp shuffles of a uniform column) and sums, in a fixed
-// order, the terms of the active ones, each evaluated from the SDF through L1 — V_R is a thin
-// band, so few vertices are active. No atomics, no shared staging; per-block loss partials
-// (fixed assignment and order) for k_reg_finalize.
-__global__ void __launch_bounds__(256) k_reg_stencil(StencilArgs a, const uint8_t* __restrict__ flags,
-                                                     double* __restrict__ partials, int ntiles) {
-  __shared__ double red[3][8];
-  __shared__ uint16_t vlist_all[8][MX * MY * (TZ + 2)];  // per warp: active vertices of the halo box
-  __shared__ float acc_all[8][TX * TY * TZ];             // per warp: the tile's output sums
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint16_t* vlist = vlist_all[warp];
-  float* acc_s = acc_all[warp];
-  for (int o = lane; o < TX * TY * TZ; o += 32) acc_s[o] = 0.0f;
+// Fused eikonal + curvature gradient in gather form over 32x4x4 tiles. Block b of B owns tiles b, b + B,
+// b + 2B, ...; its threads test kRegThreads of them at once against the flags of the 3x3x3 tiles around each
+// (a tile's outputs need the vertices of its halo). A warp then takes every eighth tile that needs it: the
+// V_R windows of the halo's columns, a compact list of their active vertices, each vertex's terms evaluated
+// once (SDF through L1) and added to the tile's sums in ordered passes. Tiles of more than kWarpVerts vertices,
+// and all but the thinnest where a block has fewer tiles than warps, wait for the whole block, which keeps
+// the terms in slots and lets each output sum its neighbours' in a fixed order. An output gets one addition
+// a launch; per-cluster loss partials (fixed assignment and order) for k_reg_finalize. Bound by the chain of one
+// tile (loads, ~150 instructions a vertex, passes): V_R is a thin band of few, unevenly filled tiles. A warp
+// for every tile: 256^3 and 8,192 rays 55 us, 64^3 and 2,048 rays 33 us; a block for every tile 81 and 15 us;
+// so 39 and 13 us.
+constexpr int kRegThreads = 256;
+constexpr int kRegWarps = kRegThreads / 32;
+constexpr int kHaloVerts = MX * MY * (TZ + 2);
+constexpr int kWarpVerts = 152;  // 48: 59 us, 96: 46, 144: 39 (256^3, 8,192 rays)
+
+struct TileColumns {
+  uint64_t win[MX * MY];  // bits of the columns' vertices z0 - 1 .. z0 + 32
+  int off[MX * MY + 1];   // first slot of a column
+};
+
+// A tile's windows and slots, by one warp. Returns how many vertices are active.
+__device__ __forceinline__ int tile_columns(const StencilArgs& a, const uint32_t* bm, int x0, int y0, int z0,
+                                            TileColumns& tc, int lane) {
+  // the halo's corner columns touch no output
+  const bool corner = (lane / MY == 0 || lane / MY == MX - 1) && (lane % MY == 0 || lane % MY == MY - 1);
+  const uint64_t w0 = corner ? 0ull : column_window(a, bm, x0 - 1 + lane / MY, y0 - 1 + lane % MY, z0);
+  const uint64_t w1 = lane < MX * MY - 33 ? column_window(a, bm, x0 - 1 + (lane + 32) / MY, y0 - 1 + (lane + 32) % MY, z0) : 0ull;
+  const int c0 = __popcll(w0), c1 = __popcll(w1);
+  int inc = c0, inc1 = c1;  // columns 0..31, then 32..35
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o), v1 = __shfl_up_sync(0xffffffffu, inc1, o);
+    if (lane >= o) {
+      inc += v;
+      inc1 += v1;
+    }
+  }
+  const int first = __shfl_sync(0xffffffffu, inc, 31), total = first + __shfl_sync(0xffffffffu, inc1, 31);
+  tc.win[lane] = w0;
+  tc.off[lane] = inc - c0;
+  if (lane < MX * MY - 32) {
+    tc.win[lane + 32] = w1;
+    tc.off[lane + 32] = first + inc1 - c1;
+  }
   __syncwarp();
+  return total;
+}
+
+// A tile of few vertices by one warp: 32 vertices at a time, their 7 terms added into the outputs' sums in 7
+// ordered passes (two vertices never share a target within a pass), then the sums to the gradient. acc:
+// zeros, and zeros again afterwards.
+__device__ __forceinline__ void tile_by_warp(const StencilArgs& a, const StencilConsts& k, int x0, int y0, int z0,
+                                             const TileColumns& tc, int total, float* acc, uint16_t* list, int lane,
+                                             double* loss) {
+  for (int c = lane; c < MX * MY; c += 32) {
+    int pos = tc.off[c];
+    for (uint64_t m = tc.win[c]; m; m &= m - 1) list[pos++] = (uint16_t)(c * (TZ + 2) + __ffsll((long long)m) - 1);
+  }
+  __syncwarp();
+  for (int s = lane; s - lane < total; s += 32) {  // whole warps
+    const bool mine = s < total;
+    float e[3] = {0.0f, 0.0f, 0.0f}, c[3] = {0.0f, 0.0f, 0.0f};
+    int ox = -9, oy = 0, oz = 0;
+    if (mine) {
+      const int code = list[s], col = code / (TZ + 2), kb = code - (TZ + 2) * col;
+      ox = col / MY - 1;
+      oy = col % MY - 1;
+      oz = kb - 1;
+      const bool owned = (unsigned)ox < TX && (unsigned)oy < TY && (unsigned)oz < TZ;
+      vertex_terms(a, k, x0 + ox, y0 + oy, z0 + oz, e, c, owned ? loss : nullptr);
+    }
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+      const int ax = p == 1 ? 1 : (p == 2 ? -1 : 0), ay = p == 3 ? 1 : (p == 4 ? -1 : 0);
+      const int az = p == 5 ? 1 : (p == 6 ? -1 : 0), q = p ? (p - 1) >> 1 : 0;
+      const float term = p == 0 ? -2.0f * (c[0] + c[1] + c[2]) : (p & 1) ? e[q] + c[q] : c[q] - e[q];
+      if ((unsigned)(ox + ax) < TX && (unsigned)(oy + ay) < TY && (unsigned)(oz + az) < TZ)
+        acc[((ox + ax) * TY + oy + ay) * TZ + oz + az] += term;
+      __syncwarp();
+    }
+  }
+#pragma unroll 4
+  for (int o = lane; o < TX * TY * TZ; o += 32) {
+    const float v = acc[o];
+    if (v != 0.0f) {
+      atomicAdd(a.gg + lin3(a.g, x0 + o / (TY * TZ), y0 + o / TZ % TY, z0 + lane), v);  // its only one: no load to wait for
+      acc[o] = 0.0f;
+    }
+  }
+  __syncwarp();
+}
+
+// A tile by the whole block: terms into slots, then every output sums its neighbours'. term: [6][kHaloVerts].
+__device__ __forceinline__ void tile_by_block(const StencilArgs& a, const StencilConsts& k, int x0, int y0, int z0,
+                                              const TileColumns& tc, int total, float* term, uint16_t* list, int warp,
+                                              int lane, double* loss) {
+  constexpr int kWarps = kRegWarps, cap = kHaloVerts;
+  for (int c = warp; c < MX * MY; c += kWarps) {
+    const uint64_t w = tc.win[c];
+    if (w == 0ull) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int kb = lane + 32 * h;
+      if (kb < TZ + 2 && (w >> kb & 1ull)) list[tc.off[c] + __popcll(w & ((1ull << kb) - 1ull))] = (uint16_t)(c * (TZ + 2) + kb);
+    }
+  }
+  __syncthreads();
+  for (int s = 32 * warp + lane; s < total; s += 32 * kWarps) {
+    const int code = list[s], col = code / (TZ + 2), kb = code - (TZ + 2) * col, cx = col / MY, cy = col % MY;
+    const bool owned = cx >= 1 && cx <= TX && cy >= 1 && cy <= TY && kb >= 1 && kb <= TZ;
+    float e[3], c[3];
+    vertex_terms(a, k, x0 - 1 + cx, y0 - 1 + cy, z0 - 1 + kb, e, c, owned ? loss : nullptr);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      term[q * cap + s] = e[q];
+      term[(3 + q) * cap + s] = c[q];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int o = warp; o < TX * TY; o += kWarps) {  // lane = z
+    const int col = (o / TY + 1) * MY + o % TY + 1;
+    const uint64_t near[5] = {tc.win[col], tc.win[col - MY], tc.win[col + MY], tc.win[col - 1], tc.win[col + 1]};
+    if ((near[0] | near[1] | near[2] | near[3] | near[4]) == 0ull) continue;
+    const int first[5] = {tc.off[col], tc.off[col - MY], tc.off[col + MY], tc.off[col - 1], tc.off[col + 1]};
+    auto slot = [&](int c, int b) {  // of vertex b of column near[c], or -1
+      return (near[c] >> b & 1ull) ? first[c] + __popcll(near[c] & ((1ull << b) - 1ull)) : -1;
+    };
+    const int kb = lane + 1;
+    float v = 0.0f;
+    bool any = false;
+    int q = slot(0, kb);
+    if (q >= 0) {
+      v = -2.0f * (term[3 * cap + q] + term[4 * cap + q] + term[5 * cap + q]);
+      any = true;
+    }
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {  // the neighbour below adds e + c, the one above c - e
+      const int ax = d >> 1;
+      q = ax < 2 ? slot(1 + d, kb) : slot(0, (d & 1) ? kb + 1 : kb - 1);
+      if (q >= 0) {
+        v += (d & 1) ? term[(3 + ax) * cap + q] - term[ax * cap + q] : term[ax * cap + q] + term[(3 + ax) * cap + q];
+        any = true;
+      }
+    }
+    if (any) atomicAdd(a.gg + lin3(a.g, x0 + o / TY, y0 + o % TY, z0 + lane), v);  // its only one: no load to wait for
+  }
+  __syncthreads();  // the columns, the list and the terms are read
+}
+
+__global__ void __launch_bounds__(kRegThreads, 4) k_reg_stencil(StencilArgs a, const uint8_t* __restrict__ flags,
+                                                             double* __restrict__ partials, int ntiles) {
+  __shared__ float term[6 * kHaloVerts];  // the block's slots, or the warps' sums
+  __shared__ uint16_t list[kHaloVerts];
+  __shared__ TileColumns cols[kRegWarps];
+  __shared__ int queue[kRegThreads], dense[kRegThreads];  // tiles to do; vertices of those left to the block, else 0
+  __shared__ int qcount[kRegWarps];
+  __shared__ double red[3][kRegWarps];
+  static_assert(kRegWarps * kWarpVerts <= kHaloVerts && kRegWarps * TX * TY * TZ <= 6 * kHaloVerts, "a warp's part");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool relax_on = a.relax_r > 0.0f && a.counts[1] > 0;
   const uint32_t* bm = a.fb + (relax_on ? a.nwords : 0);
   // |V_R| after the filters: counts[3] (relax) / counts[2] (no relax); the filtered bitmaps
@@ -328,12 +446,12 @@ __global__ void __launch_bounds__(256) k_reg_stencil(StencilArgs a, const uint8_
   k.sc = k.inv_nv * a.w_curv;
   k.w_eik = a.w_eik;
   double loss[3] = {0.0, 0.0, 0.0};
-  const int gw = blockIdx.x * 8 + warp, nw = gridDim.x * 8;
-  for (int base = 0; gw + base * nw < ntiles; base += 32) {
-    const int tl = gw + (base + lane) * nw;
+  const int nblk = gridDim.x;
+  for (int64_t base = blockIdx.x; base < ntiles; base += (int64_t)nblk * kRegThreads) {
+    const int64_t tl = base + (int64_t)tid * nblk;
     bool need = false;
     if (tl < ntiles) {
-      const int tz = tl % a.tiles_z, ty = (tl / a.tiles_z) % a.tiles_y, tx = tl / (a.tiles_z * a.tiles_y);
+      const int t = (int)tl, tz = t % a.tiles_z, ty = (t / a.tiles_z) % a.tiles_y, tx = t / (a.tiles_z * a.tiles_y);
       for (int dx = -1; dx <= 1; ++dx)
         for (int dy = -1; dy <= 1; ++dy)
           for (int dz = -1; dz <= 1; ++dz) {
@@ -342,68 +460,41 @@ __global__ void __launch_bounds__(256) k_reg_stencil(StencilArgs a, const uint8_
             need |= __ldg(flags + ((int64_t)nx * a.tiles_y + ny) * a.tiles_z + nz) != 0;
           }
     }
-    unsigned todo = __ballot_sync(0xffffffffu, need);
-    while (todo) {
-      const int b = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int t = gw + (base + b) * nw;
+    const unsigned votes = __ballot_sync(0xffffffffu, need);
+    if (lane == 0) qcount[warp] = __popc(votes);
+    __syncthreads();
+    int at = __popc(votes & ((1u << lane) - 1u)), todo = 0;
+#pragma unroll
+    for (int w = 0; w < kRegWarps; ++w) {
+      if (w < warp) at += qcount[w];
+      todo += qcount[w];
+    }
+    if (need) queue[at] = (int)tl;
+    __syncthreads();
+    for (int o = lane; o < TX * TY * TZ; o += 32) term[TX * TY * TZ * warp + o] = 0.0f;
+    __syncwarp();
+    for (int n = warp; n < todo; n += kRegWarps) {
       int x0, y0, z0;
-      tile_origin(a, t, x0, y0, z0);
-      const uint64_t w0 = column_window(a, bm, x0 - 1 + lane / 6, y0 - 1 + lane % 6, z0);
-      const uint64_t w1 =
-          lane < 4 ? column_window(a, bm, x0 - 1 + (lane + 32) / 6, y0 - 1 + (lane + 32) % 6, z0) : 0ull;
-      const int cnt0 = __popcll(w0), cnt1 = __popcll(w1);
-      int incl = cnt0 + cnt1;  // inclusive warp prefix of the vertex counts (column order)
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      if (total == 0) continue;
-      // compact the active vertices of the halo box: code = column * 34 + window bit
-      int pos = incl - cnt0 - cnt1;
-      for (uint64_t m = w0; m; m &= m - 1) vlist[pos++] = (uint16_t)(lane * 34 + __ffsll((long long)m) - 1);
-      for (uint64_t m = w1; m; m &= m - 1) vlist[pos++] = (uint16_t)((lane + 32) * 34 + __ffsll((long long)m) - 1);
-      __syncwarp();
-      // evaluate each vertex once and add its 7 terms into the tile's accumulators in 7 ordered
-      // passes (two vertices never share a target within a pass)
-      for (int base = 0; base < total; base += 32) {
-        const int idx = base + lane;
-        float t0 = 0.0f, tp[3] = {0.0f, 0.0f, 0.0f}, tm[3] = {0.0f, 0.0f, 0.0f};
-        int vx = 0, vy = 0, vz = 0;
-        const bool mine = idx < total;
-        if (mine) {
-          const int code = vlist[idx], col = code / 34, kb = code - 34 * col;
-          vx = x0 - 1 + col / MY;
-          vy = y0 - 1 + col % MY;
-          vz = z0 - 1 + kb;
-          const bool owned = vx >= x0 && vx < x0 + TX && vy >= y0 && vy < y0 + TY && vz >= z0 && vz < z0 + TZ;
-          vertex_terms(a, k, vx, vy, vz, t0, tp, tm, owned ? loss : nullptr);
-        }
-#pragma unroll
-        for (int p = 0; p < 7; ++p) {
-          const int ax = p == 1 ? 1 : (p == 2 ? -1 : 0), ay = p == 3 ? 1 : (p == 4 ? -1 : 0);
-          const int az = p == 5 ? 1 : (p == 6 ? -1 : 0);
-          const float term = p == 0 ? t0 : (p & 1) ? tp[(p - 1) >> 1] : tm[(p - 1) >> 1];
-          const int ox = vx + ax - x0, oy = vy + ay - y0, oz = vz + az - z0;
-          if (mine && ox >= 0 && ox < TX && oy >= 0 && oy < TY && oz >= 0 && oz < TZ)
-            acc_s[(ox * TY + oy) * TZ + oz] += term;
-          __syncwarp();
-        }
-      }
-      // add the tile's sums to the gradient (z-contiguous lanes) and clear the accumulators
-#pragma unroll 1
-      for (int o = lane; o < TX * TY * TZ; o += 32) {
-        const float v = acc_s[o];
-        if (v != 0.0f) {
-          const int ox = o / (TY * TZ), oy = (o / TZ) % TY, oz = o % TZ;
-          a.gg[lin3(a.g, x0 + ox, y0 + oy, z0 + oz)] += v;
-          acc_s[o] = 0.0f;
-        }
-      }
+      tile_origin(a, queue[n], x0, y0, z0);
+      const int total = tile_columns(a, bm, x0, y0, z0, cols[warp], lane);
+      const bool mine = total <= (todo < kRegWarps ? 32 : kWarpVerts);  // few tiles: all warps on each
+      if (lane == 0) dense[n] = mine ? 0 : total;
+      if (mine && total > 0)
+        tile_by_warp(a, k, x0, y0, z0, cols[warp], total, term + TX * TY * TZ * warp, list + kWarpVerts * warp, lane,
+                     loss);
       __syncwarp();
     }
+    __syncthreads();
+    for (int n = 0; n < todo; ++n) {
+      const int total = dense[n];
+      if (total == 0) continue;
+      int x0, y0, z0;
+      tile_origin(a, queue[n], x0, y0, z0);
+      if (warp == 0) tile_columns(a, bm, x0, y0, z0, cols[0], lane);
+      __syncthreads();
+      tile_by_block(a, k, x0, y0, z0, cols[0], total, term, list, warp, lane, loss);
+    }
+    __syncthreads();  // the queue is read
   }
   double le = warp_sum_d(loss[0]), lc = warp_sum_d(loss[1]), ln = warp_sum_d(loss[2]);
   if (lane == 0) {
@@ -411,18 +502,18 @@ __global__ void __launch_bounds__(256) k_reg_stencil(StencilArgs a, const uint8_
     red[1][warp] = lc;
     red[2][warp] = ln;
   }
-  __syncthreads();
-  if (tid == 0) {
-    double s0 = 0, s1 = 0, s2 = 0;
-    for (int w = 0; w < 8; ++w) {
-      s0 += red[0][w];
-      s1 += red[1][w];
-      s2 += red[2][w];
+  // the cluster's blocks in order, by its first one: one partial a cluster
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();
+  if (cl.block_rank() == 0 && tid < 3) {
+    double sum = 0;
+    for (unsigned b = 0; b < cl.num_blocks(); ++b) {
+      const double* theirs = cl.map_shared_rank(&red[tid][0], b);
+      for (int w = 0; w < kRegWarps; ++w) sum += theirs[w];
     }
-    partials[3 * blockIdx.x] = s0;
-    partials[3 * blockIdx.x + 1] = s1;
-    partials[3 * blockIdx.x + 2] = s2;
+    partials[3 * (blockIdx.x / cl.num_blocks()) + tid] = sum;
   }
+  cl.sync();  // until it has read them
 }
 
 // Mean losses over interior vertices from the per-block partials, fixed reduction order; and
@@ -523,8 +614,16 @@ static int64_t stencil_tiles(const int32_t res[3]) {
   return (int64_t)((res[2] + TZ - 1) / TZ) * ((res[1] + TY - 1) / TY) * ((res[0] + TX - 1) / TX);
 }
 
+// Blocks that share one of the nb loss partials: as many as are resident at once (6 a SM), a tile each on small
+// grids.
+static unsigned stencil_cluster(int64_t nb) {
+  unsigned c = 8;
+  while (c > 1 && nb * c > (int64_t)kSMs * 4) c /= 2;
+  return c;
+}
+
 int64_t vx_reg_stencil_blocks(const int32_t res[3]) {
-  const int64_t t = (stencil_tiles(res) + 7) / 8;  // at least one tile per warp
+  const int64_t t = (stencil_tiles(res) + 7) / 8;  // up to 8 blocks share a partial (stencil_cluster)
   const int64_t cap = (int64_t)kSMs * 4;
   return t < cap ? t : cap;
 }
@@ -561,8 +660,19 @@ int vx_reg_stencil(const float* grid, const uint32_t* bitmap, const int32_t res[
   const int64_t ntiles = stencil_tiles(res);
   uint8_t* flags = reinterpret_cast<uint8_t*>(partials + 3 * nb);
   cudaStream_t st = (cudaStream_t)stream;
-  k_tile_flags<<<grid_for(ntiles, 256), 256, 0, st>>>(a, (int)ntiles, flags);
-  k_reg_stencil<<<(unsigned)nb, 256, 0, st>>>(a, flags, partials, (int)ntiles);
+  k_tile_flags<<<grid_for(ntiles, 16), 256, 0, st>>>(a, (int)ntiles, flags);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = stencil_cluster(nb);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nb * attr.val.clusterDim.x);
+  cfg.blockDim = dim3(kRegThreads);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_reg_stencil, a, static_cast<const uint8_t*>(flags), partials, (int)ntiles);
+  if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "reg_stencil: %s", cudaGetErrorString(e));
   if (losses || n_active)
     k_reg_finalize<<<1, 256, 0, st>>>(partials, (int)nb, losses, counts, relax_radius > 0.0f ? 1 : 0,
                                       band > 0.0f ? 1 : 0, reinterpret_cast<long long*>(n_active));
