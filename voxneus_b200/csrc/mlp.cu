@@ -726,7 +726,9 @@ __global__ void __launch_bounds__(256) k_mlp_wgrad_reduce(const float* __restric
 // 32(w%2)..32(w%2)+31, so each gather instruction reads one level for 32 consecutive samples of
 // a ray, and neighbouring samples that share a coarse-level cell share its request. Warps of
 // level group 0 also evaluate the SH of the view direction, group 1 copies the normal; the rows
-// meet in shared memory and leave as one contiguous block (or row by row for a wider stride).
+// meet in shared memory and leave as one contiguous block (or row by row for a wider stride), evicted first
+// from L2, where the 64 MB table is to stay: 1 M samples 229 -> 224 us, a view's 61 M 11.79 -> 11.65 ms. Bound by
+// the table's sector requests from L1 to L2, 78% of the rate that random reads reach.
 constexpr int kRowsPerBlock = 64;
 
 template <bool kCompact>
@@ -779,7 +781,7 @@ __global__ void __launch_bounds__(256) k_hash_rows(HashArgs a) {
     const int nrows = (int)(a.P - base < kRowsPerBlock ? a.P - base : kRowsPerBlock);
     if (a.ld == 4 * kChunks) {
       float4* out = reinterpret_cast<float4*>(a.out + base * (4 * kChunks));
-      for (int k = tid; k < nrows * kChunks; k += 256) out[k] = srow[k];
+      for (int k = tid; k < nrows * kChunks; k += 256) __stcs(out + k, srow[k]);
     } else {
       for (int k = tid; k < nrows * kChunks; k += 256)
         reinterpret_cast<float4*>(a.out + (base + k / kChunks) * a.ld)[k % kChunks] = srow[k];
