@@ -208,7 +208,7 @@ def algorithmic_bytes(name, n_rays, n_samples, res, n_levels=16, ld=52, nnz=None
     }
     if nnz is not None:
         table["vx_masked_adam_upd"] = voxels * 4 + nnz * 24
-    return table.get(name)
+    return table.get(name.removesuffix("_masked"))  # the training forward is the same work and writes its ReLU bits
 
 
 # FP32 FLOPs per sample of the MLP kernels (51 -> 64 ReLU -> 3 Sigmoid; the 52nd input column is padding)
@@ -221,12 +221,17 @@ MLP_FLOPS = {
     # the same adjoint on the compact rows (SH(d) recomputed from the ray direction: ~40 FLOPs, not counted)
     "vx_appearance_mlp_backward": 2 * 52 * 64 + 2 * 3 * 64 * 2 + 2 * 52 * 64 + 2 * 64 * 35,
 }
+MLP_FLOPS["vx_appearance_mlp_forward_masked"] = MLP_FLOPS["vx_appearance_mlp_forward"]
+# from the forward's ReLU bits: no hidden recompute; dW0 and dX are contractions of the 0/1 mask, exact in bf16,
+# with three bf16 parts of the other operand
+MLP_FLOPS["vx_appearance_mlp_backward_masked"] = 2 * 3 * 64 * 2 + 2 * 52 * 64 + 2 * 64 * 35
+BF16_PRODUCTS = {"vx_appearance_mlp_backward_masked"}  # the others issue tf32 products
 
 
 def mlp_tensor(per_kernel, n_points):
-    """FLOP rate of the MLP kernels: FP32-equivalent, and the tf32 tensor-core rate they issue (three
-    tf32 products per FP32 product, hi*hi + hi*lo + lo*hi) against the dense tf32 peak, taken as half
-    the measured bf16 GEMM peak (MEASURED_PEAKS.json)."""
+    """FLOP rate of the MLP kernels: FP32-equivalent, and the tensor-core rate they issue, three products
+    per FP32 product: tf32 (hi*hi + hi*lo + lo*hi) against the dense tf32 peak, taken as half the measured
+    bf16 GEMM peak (MEASURED_PEAKS.json), or bf16 parts against that peak itself."""
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             bf16, kind = float(json.load(f)["bf16_tflops"]), "measured bf16 / 2"
@@ -236,8 +241,10 @@ def mlp_tensor(per_kernel, n_points):
     for k, fl in MLP_FLOPS.items():
         if k in per_kernel and per_kernel[k] > 0:
             tf = n_points * fl / (per_kernel[k] / 1e3) / 1e12
-            out[k] = {"fp32_flops_per_sample": fl, "fp32_equiv_tflops": tf, "tf32_issued_tflops": 3 * tf,
-                      "frac": 3 * tf / (bf16 / 2)}
+            kind_peak = bf16 if k in BF16_PRODUCTS else bf16 / 2
+            out[k] = {"fp32_flops_per_sample": fl, "fp32_equiv_tflops": tf, "issued_tflops": 3 * tf,
+                      "issued_type": "bf16" if k in BF16_PRODUCTS else "tf32", "peak_tflops": kind_peak,
+                      "frac": 3 * tf / kind_peak}
     return out
 
 
@@ -518,7 +525,7 @@ def render_roofline(per_kernel, n_rays, peak, peak_kind):
     if ms > 0:
         out["achieved"] = n_rays * RENDER_BYTES_PER_RAY / (ms / 1e3) / 1e9
         out["frac"] = out["achieved"] / peak
-    app = per_kernel.get("vx_appearance_mlp_forward")
+    app = per_kernel.get("vx_appearance_mlp_forward_masked", per_kernel.get("vx_appearance_mlp_forward"))
     if app and ms > 0:
         b = RENDER_BYTES_PER_RAY + HASH_FWD_BYTES_PER_RAY
         ach = n_rays * b / ((ms + app) / 1e3) / 1e9
@@ -649,7 +656,7 @@ def run_fused(args):
         ab = algorithmic_bytes(name, **sizes)
         ach = ab / (k_ms / 1e3) / 1e9
         return {"bound": "hbm", "kernel": name, "achieved": ach, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-                "frac": ach / peak, "traffic": load_traffic().get(name), "algorithmic_bytes_per_launch": ab,
+                "frac": ach / peak, "traffic": load_traffic().get(name.removesuffix("_masked")), "algorithmic_bytes_per_launch": ab,
                 "ms_per_launch": k_ms}
 
     def tensor_roofline(name):
@@ -657,11 +664,11 @@ def run_fused(args):
         k_ms = sum(d) / len(d)
         mt = mlp_tensor({name: k_ms}, args.rays * (N_SAMPLES + N_IMPORTANCE))
         r = mt[name]
-        return {"bound": "tensor", "kernel": name, "achieved": r["tf32_issued_tflops"], "peak": mt["peak_tf32_tflops"],
+        return {"bound": "tensor", "kernel": name, "achieved": r["issued_tflops"], "peak": r["peak_tflops"],
                 "peak_kind": mt["peak_kind"], "unit": "TFLOP/s", "frac": r["frac"],
-                "traffic": load_traffic().get(name), "fp32_equiv_tflops": r["fp32_equiv_tflops"],
+                "traffic": load_traffic().get(name.removesuffix("_masked")), "fp32_equiv_tflops": r["fp32_equiv_tflops"],
                 "ms_per_launch": k_ms,
-                "note": "tf32 products issued (3 per FP32 product: hi*hi + hi*lo + lo*hi); the kernel is "
+                "note": f"{r['issued_type']} products issued (3 per FP32 product); the kernel is "
                         "latency/issue bound at one CTA per SM, not at the tensor pipe"}
 
     # the dominant call's binding limit: where it has both an algorithmic byte count and tensor-core

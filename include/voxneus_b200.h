@@ -318,9 +318,9 @@ int vx_mlp_blocks(int64_t n_points);
 int vx_mlp_partial_floats(void);
 
 /* The MLP kernels run on the tcgen05 tensor cores (forward: kind::tf32, hi/lo split; adjoint:
- * kind::f16 on three exact bf16 parts; both of FP32-level accuracy) and wait on the tensor core with bounded mbarrier polls. Returns how many blocks gave
- * up on such a wait since the last call (their outputs are invalid) and resets the count; -1 on
- * a CUDA error. Synchronises the device (diagnostic only). No counterpart in the reference. */
+ * kind::f16 on three exact bf16 parts; both of FP32-level accuracy) and wait on the tensor core with
+ * bounded mbarrier polls. Returns how many blocks gave up on such a wait since the last call (their
+ * outputs are invalid) and resets the count; -1 on a CUDA error. Synchronises the device (diagnostic only). No counterpart in the reference. */
 int vx_tensor_core_timeouts(void);
 
 /* The wait policy of this thread's later MLP launches (vx_radiance_mlp_forward/backward,
@@ -477,13 +477,13 @@ int vx_vr_compact_noalloc(const uint32_t* bitmap, const float* grid, const int32
                           const float xyz_max[3], float relax_radius, float band, const unsigned long long* counts,
                           int64_t* verts_out, int64_t* linear_out, int64_t capacity, void* stream);
 
-/* Blocks of the fused regularizer, and the doubles of its workspace (3 loss partials per block,
- * then one flag byte per 32x4x4 tile). */
+/* Loss partials of the fused regularizer (each of a cluster of up to 8 blocks), and the doubles of its
+ * workspace (3 a partial, then one flag byte per 32x4x4 tile). */
 int64_t vx_reg_stencil_blocks(const int32_t res[3]);
 int64_t vx_reg_stencil_workspace(const int32_t res[3]);
 
 /* Fused eikonal + curvature closed forms (regularization/eikonal.py:13-171 and curvature.py:13-165 as
- * called by training/trainer.py:268-319), gather form (deterministic, no atomics), accumulated into
+ * called by training/trainer.py:268-319), gather form (deterministic: one addition an output), accumulated into
  * grad_grid with weights w_eik and w_curv and scale 2/|V_R|. bitmap is the filtered pair written by
  * vx_vr_count; counts selects its relax half (the reference applies the relax filter only when a
  * vertex passes it) and gives |V_R|. band is applied by vx_vr_count (here it only selects which

@@ -6,13 +6,12 @@
 //  * list form (the reference's kernel interface, eikonal_grad.cu / curvature_grad.cu):
 //    one thread per listed vertex, atomics into the gradient, scale 2/|list|;
 //  * fused gather form for the training step: one pass over 32x4x4 voxel tiles of the
-//    grid, skipping tiles with no active vertex. Each output voxel sums, in registers, the
+//    grid, skipping tiles with no active vertex. Each output voxel sums, in a fixed order, the
 //    contributions of the <= 7 active interior vertices whose stencil touches it (itself
-//    and its 6 face neighbours), reading a halo-2 tile of the SDF from shared memory. No
-//    atomics: the result is deterministic. The active set is the V_R bitmap with the relax
-//    and narrow-band predicates, and |V_R| comes from the device-side counts.
-// Both forms also reduce the monitoring losses (mean over interior vertices) through
-// per-block partials and a last-block epilogue.
+//    and its 6 face neighbours) and is added to the gradient once: the result is
+//    deterministic. The active set is the V_R bitmap with the relax and narrow-band
+//    predicates, and |V_R| comes from the device-side counts.
+// Both forms also reduce the monitoring losses (mean over interior vertices) through partials.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(256) k_tile_flags(StencilArgs a, int ntiles, u
 // a launch; per-cluster loss partials (fixed assignment and order) for k_reg_finalize. Bound by the chain of one
 // tile (loads, ~150 instructions a vertex, passes): V_R is a thin band of few, unevenly filled tiles. A warp
 // for every tile: 256^3 and 8,192 rays 55 us, 64^3 and 2,048 rays 33 us; a block for every tile 81 and 15 us;
-// so 39 and 13 us.
+// so 39 and 12 us; 512^3 with every vertex active 5.03 and now 5.09 ms.
 constexpr int kRegThreads = 256;
 constexpr int kRegWarps = kRegThreads / 32;
 constexpr int kHaloVerts = MX * MY * (TZ + 2);
@@ -319,8 +318,8 @@ __device__ __forceinline__ int tile_columns(const StencilArgs& a, const uint32_t
 }
 
 // A tile of few vertices by one warp: 32 vertices at a time, their 7 terms added into the outputs' sums in 7
-// ordered passes (two vertices never share a target within a pass), then the sums to the gradient. acc:
-// zeros, and zeros again afterwards.
+// ordered passes (two vertices never share a target within a pass), then the sums to the gradient. acc
+// holds zeros.
 __device__ __forceinline__ void tile_by_warp(const StencilArgs& a, const StencilConsts& k, int x0, int y0, int z0,
                                              const TileColumns& tc, int total, float* acc, uint16_t* list, int lane,
                                              double* loss) {
@@ -356,7 +355,6 @@ __device__ __forceinline__ void tile_by_warp(const StencilArgs& a, const Stencil
     const float v = acc[o];
     if (v != 0.0f) {
       atomicAdd(a.gg + lin3(a.g, x0 + o / (TY * TZ), y0 + o / TZ % TY, z0 + lane), v);  // its only one: no load to wait for
-      acc[o] = 0.0f;
     }
   }
   __syncwarp();
@@ -425,7 +423,7 @@ __global__ void __launch_bounds__(kRegThreads, 4) k_reg_stencil(StencilArgs a, c
   __shared__ float term[6 * kHaloVerts];  // the block's slots, or the warps' sums
   __shared__ uint16_t list[kHaloVerts];
   __shared__ TileColumns cols[kRegWarps];
-  __shared__ int queue[kRegThreads], dense[kRegThreads];  // tiles to do; vertices of those left to the block, else 0
+  __shared__ int queue[kRegThreads], dense[kRegWarps];  // tiles to do; vertices of a warp's left to the block, else 0
   __shared__ int qcount[kRegWarps];
   __shared__ double red[3][kRegWarps];
   static_assert(kRegWarps * kWarpVerts <= kHaloVerts && kRegWarps * TX * TY * TZ <= 6 * kHaloVerts, "a warp's part");
@@ -471,28 +469,33 @@ __global__ void __launch_bounds__(kRegThreads, 4) k_reg_stencil(StencilArgs a, c
     }
     if (need) queue[at] = (int)tl;
     __syncthreads();
-    for (int o = lane; o < TX * TY * TZ; o += 32) term[TX * TY * TZ * warp + o] = 0.0f;
-    __syncwarp();
-    for (int n = warp; n < todo; n += kRegWarps) {
-      int x0, y0, z0;
-      tile_origin(a, queue[n], x0, y0, z0);
-      const int total = tile_columns(a, bm, x0, y0, z0, cols[warp], lane);
-      const bool mine = total <= (todo < kRegWarps ? 32 : kWarpVerts);  // few tiles: all warps on each
-      if (lane == 0) dense[n] = mine ? 0 : total;
-      if (mine && total > 0)
-        tile_by_warp(a, k, x0, y0, z0, cols[warp], total, term + TX * TY * TZ * warp, list + kWarpVerts * warp, lane,
-                     loss);
-      __syncwarp();
-    }
-    __syncthreads();
-    for (int n = 0; n < todo; ++n) {
-      const int total = dense[n];
-      if (total == 0) continue;
-      int x0, y0, z0;
-      tile_origin(a, queue[n], x0, y0, z0);
-      if (warp == 0) tile_columns(a, bm, x0, y0, z0, cols[0], lane);
+    for (int n0 = 0; n0 < todo; n0 += kRegWarps) {  // a tile a warp, then the crowded ones of them
+      const int n = n0 + warp;
+      int total = 0;
+      if (n < todo) {
+        int x0, y0, z0;
+        tile_origin(a, queue[n], x0, y0, z0);
+        total = tile_columns(a, bm, x0, y0, z0, cols[warp], lane);
+        if (total <= (todo < kRegWarps ? 32 : kWarpVerts)) {  // few tiles: all warps on each
+          if (total > 0) {
+            float* acc = term + TX * TY * TZ * warp;
+            for (int o = lane; o < TX * TY * TZ; o += 32) acc[o] = 0.0f;
+            __syncwarp();
+            tile_by_warp(a, k, x0, y0, z0, cols[warp], total, acc, list + kWarpVerts * warp, lane, loss);
+          }
+          total = 0;
+        }
+      }
+      if (lane == 0) dense[warp] = total;
       __syncthreads();
-      tile_by_block(a, k, x0, y0, z0, cols[0], total, term, list, warp, lane, loss);
+#pragma unroll 1
+      for (int w = 0; w < kRegWarps; ++w) {
+        if (dense[w] == 0) continue;
+        int x0, y0, z0;
+        tile_origin(a, queue[n0 + w], x0, y0, z0);
+        tile_by_block(a, k, x0, y0, z0, cols[w], dense[w], term, list, warp, lane, loss);
+      }
+      __syncthreads();  // the columns and dense are read
     }
     __syncthreads();  // the queue is read
   }
