@@ -442,9 +442,11 @@ static_assert(FwdShape<true, true>::kOffRed % 16 == 0 && FwdShape<true, true>::k
               "shared-memory alignment");
 constexpr int kFwdThreads = 512 + 64;
 
-// A barrier of a slot's workers that also agrees on whether any of them gave up a wait.
+// A barrier of a slot's workers that also agrees on whether any of them gave up a wait. Like the tensor-memory loads
+// and stores it is an instruction of a converged warp: __syncwarp() first wherever lanes can have parted.
 __device__ __forceinline__ bool slot_sync_or(int slot, bool v) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(r)
@@ -501,6 +503,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     tc::mbar_init(bar_rows + 1, 1);
     s_fail[slot] = 0;
   }
+  __syncwarp();
   if (warp == 0) tc::tmem_alloc(s_taddr, 512);
   tc::fence_smem_to_async();
   tc::fence_before_sync();
@@ -601,6 +604,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         for (int i4 = 0; i4 < 4; ++i4) tc::split_tf32(v[i4], xh[4 * j + i4], lo[i4]);
         *reinterpret_cast<float4*>(XL + x_off(c, m)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
       }
+      __syncwarp();
       // stores aligned to their widths (the column base is a multiple of 64)
       const uint32_t ta = acol + 64 * buf + lane_base + 4 * c0;
       if (kFold && hh == 0) {
@@ -628,6 +632,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         BETA[NH * buf + stid] = b;
         if (t + tstride < ntiles) load_dir(t + tstride);
       }
+      __syncwarp();
       tc::tmem_wait_st();
     };
     auto tell = [&]() {  // to the issuing warp: what this warp wrote and read is done
@@ -679,6 +684,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   }
   tc::fence_before_sync();
   __syncthreads();
+  __syncwarp();
   if (warp == 0) tc::tmem_dealloc(tb, 512);
 }
 

@@ -136,12 +136,24 @@ __device__ __forceinline__ void stage_mask(uint8_t* M, uint32_t taddr, int m, in
 constexpr int kAdjShTid = 5;  // the worker that evaluates SH(d) of a tile's ray
 
 // Named barriers: 1 once a tile's A is staged (the workers go on, the issuing warp waits), 2 at the end
-// of a tile, which also agrees on whether any thread gave up a wait.
-__device__ __forceinline__ void adj_staged_arrive() { asm volatile("bar.arrive 1, %0;" ::"n"(kAdjThreads) : "memory"); }
-__device__ __forceinline__ void adj_staged_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kAdjThreads) : "memory"); }
-__device__ __forceinline__ void adj_workers_sync() { asm volatile("bar.sync 3, %0;" ::"n"(kAdjWork) : "memory"); }
+// of a tile, which also agrees on whether any thread gave up a wait. They, and the tensor-memory loads and stores, are
+// instructions of a converged warp: __syncwarp() first wherever lanes can have parted before (polls that
+// end at different times, a branch of some lanes), because nothing else makes them meet again.
+__device__ __forceinline__ void adj_staged_arrive() {
+  __syncwarp();
+  asm volatile("bar.arrive 1, %0;" ::"n"(kAdjThreads) : "memory");
+}
+__device__ __forceinline__ void adj_staged_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(kAdjThreads) : "memory");
+}
+__device__ __forceinline__ void adj_workers_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 3, %0;" ::"n"(kAdjWork) : "memory");
+}
 __device__ __forceinline__ bool adj_sync_or(bool v) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 2, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(r)
@@ -209,6 +221,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     tc::mbar_init(bar_rows, 1);
     tc::mbar_init(bar_rows + 1, 1);
   }
+  __syncwarp();
   if (wid == 0) tc::tmem_alloc(s_taddr, 512);
   tc::fence_before_sync();
   __syncthreads();
@@ -376,6 +389,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 #pragma unroll
       for (int c = 0; c < NO; ++c) d[c] = dy[c] * ((1.0f - yv[c]) * yv[c]);  // 0 on rows past P
       sb += hh == 0 ? d[0] : (hh == 1 ? d[1] : d[2]);
+      __syncwarp();
       stage_mask(MK + buf * kAdjMask, tb + lane_base + kAdjMk + 8 * hh, m, hh, bits >> (16 * (hh & 1)));
       if (!S::kBulk) {
 #pragma unroll
@@ -494,10 +508,12 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           o[1] = make_float4(r[4], r[5], r[6], r[7]);
         }
         if (!kFold && it > 0) {  // (not in flight together: the unfolded forms have no registers left)
+          __syncwarp();
           load_g(par ^ 1, gv);
           tc::tmem_wait_ld();
         }
         if (it > 0) add_g(par ^ 1, gv);
+        __syncwarp();
       }
       if (hh == 3) {
         float r[4], u[4], v[4];
@@ -511,6 +527,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         }
       }
       if constexpr (kFold) {  // the four warps of 32 samples: their rows leave in whole lines
+        __syncwarp();
         asm volatile("bar.sync %0, 128;" ::"r"(4 + q) : "memory");
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
@@ -532,6 +549,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
       }
     }
     if (!failed && it > 0) failed = !tc::mbar_wait(bar_g, (it - 1) & 1, wait_limit);
+    __syncwarp();
   }
   failed = __syncthreads_or(failed);
   if (failed && tid == kAdjWork) {
@@ -625,6 +643,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   }
   tc::fence_before_sync();
   __syncthreads();
+  __syncwarp();
   if (wid == 0) tc::tmem_dealloc(tb, 512);
 }
 
