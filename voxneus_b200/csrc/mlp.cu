@@ -535,7 +535,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     bool bad = false;
     for (int64_t t = t0; t < ntiles; t += tstride, ++it) {
       bool ok = tc::mbar_wait_unless(ready, it & 1, wait_limit, s_fail + slot);
-      if (__shfl_sync(0xffffffffu, (int)!ok, 0)) {
+      // a worker that gave up a wait said so before it arrived: nothing more is issued, so that no barrier has
+      // two phases outstanding
+      if (__shfl_sync(0xffffffffu, (int)(!ok || s_fail[slot] != 0), 0)) {
         bad = true;
         break;
       }
@@ -636,6 +638,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       tc::tmem_wait_st();
     };
     auto tell = [&]() {  // to the issuing warp: what this warp wrote and read is done
+      if (!ok) s_fail[slot] = 1;
       tc::fence_smem_to_async();
       tc::fence_before_sync();
       __syncwarp();
@@ -653,7 +656,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       const int64_t m0 = t * TM;
       const bool valid = m0 + m < P, more = t + tstride < ntiles;
       if (more) stage(t + tstride, it + 1);
-      ok = tc::mbar_wait(bar, par, wait_limit) && ok;
+      ok = tc::mbar_wait_unless(bar, par, wait_limit, s_fail + slot) && ok;
       __syncwarp();
       tc::fence_after_sync();
       float z[32];

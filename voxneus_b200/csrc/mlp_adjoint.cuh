@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   uint64_t* bar_dx = bar_g + 1;
   uint64_t* bar_rows = bar_g + 2;  // [2]
   uint32_t* s_taddr = reinterpret_cast<uint32_t*>(bar_g + 4);
+  volatile int* s_fail = reinterpret_cast<volatile int*>(s_taddr + 1);  // a worker gave up a wait before staging A
   const int tid = threadIdx.x, lane = tid & 31;
   const int wid = __shfl_sync(0xffffffffu, tid >> 5, 0);  // in a uniform register: warp-uniform branches
   const int q = wid & 3, hh = wid >> 2;
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     tc::mbar_init(bar_dx, 1);
     tc::mbar_init(bar_rows, 1);
     tc::mbar_init(bar_rows + 1, 1);
+    *s_fail = 0;
   }
   __syncwarp();
   if (wid == 0) tc::tmem_alloc(s_taddr, 512);
@@ -231,7 +233,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   const int64_t ntiles = (P + TM - 1) / TM, tstep = gridDim.x, t0 = blockIdx.x;
   bool failed = false;
   int it = 0;  // tiles done
-  // the issuing warp: phases issued on each barrier (for the drain after a give-up)
+  // The issuing warp: phases issued on each barrier. A worker that gave up a wait says so before it arrives at the
+  // staged barrier, and then nothing more is issued: no barrier ever has two phases outstanding, so that the
+  // drain after a give-up can wait for the last one.
   int n_g = 0, n_dx = 0, n_rows[2] = {0, 0};
   // the workers' sums over the tiles. G of every tile is added up in registers (rounded to nearest; the
   // tensor core's own accumulation truncates, a bias that grows with the number of additions): thread
@@ -328,8 +332,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     for (int64_t t = t0; t < ntiles; t += tstep, ++it) {
       const int par = it & 1;
       adj_staged_sync();  // A of this tile is staged, its rows are read
-      issue_g(par);
-      if (S::kBulk && t + S::kBufs * tstep < ntiles) fetch_rows(t + S::kBufs * tstep, S::kBufs == 2 ? par : 0);
+      if (__shfl_sync(0xffffffffu, (int)*s_fail, 0) == 0) {
+        issue_g(par);
+        if (S::kBulk && t + S::kBufs * tstep < ntiles) fetch_rows(t + S::kBufs * tstep, S::kBufs == 2 ? par : 0);
+      }
       if (__shfl_sync(0xffffffffu, (int)adj_sync_or(false), 0)) {  // uniform, so that the loop stays so
         failed = true;
         break;
@@ -415,7 +421,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
       const int64_t m0 = t * TM;
       const bool valid = m0 + m < P, more = t + tstep < ntiles;
       // 1: G of the previous tile (A is free), this tile's rows. A wait that gives up is agreed on at the
-      // end of the tile; until then the block goes on with whatever the memory holds.
+      // end of the tile; until then the block goes on with whatever the memory holds, but issues nothing.
       if (it > 0) ok = tc::mbar_wait(bar_g, par ^ 1, wait_limit) && ok;
       if (S::kBulk && !kFold) ok = tc::mbar_wait(bar_rows, par, wait_limit) && ok;
       __syncwarp();
@@ -481,6 +487,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           }
         }
       }
+      if (!ok) *s_fail = 1;
       tc::fence_smem_to_async();
       tc::fence_before_sync();
       adj_staged_arrive();
