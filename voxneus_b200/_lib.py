@@ -6,8 +6,10 @@ no CUDA device is present, every kernel-backed call raises RuntimeError.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import functools
+import gc
 import os
 import threading
 from typing import Optional, Sequence
@@ -211,6 +213,31 @@ def query(name: str, *args):
 
 def launch_count() -> int:
     return int(load(require_cuda=False).vx_launch_count())
+
+
+# ------------------------------------------------------------------ graph capture ---------
+
+_hold_lock = threading.Lock()
+_hold = [0, False]  # captures in progress, whether the collector was on before the first
+
+
+@contextlib.contextmanager
+def collector_held():
+    """Python's cyclic garbage collector held off around a CUDA graph capture. A collection inside the capture may
+    free another graph (of a dropped trainer or engine in a reference cycle), which CUDA does not permit while a
+    stream captures: the capture is invalidated and the step that was being captured raises."""
+    with _hold_lock:
+        if _hold[0] == 0:
+            _hold[1] = gc.isenabled()
+            gc.disable()
+        _hold[0] += 1
+    try:
+        yield
+    finally:
+        with _hold_lock:
+            _hold[0] -= 1
+            if _hold[0] == 0 and _hold[1]:
+                gc.enable()
 
 
 # ------------------------------------------------------------------ argument helpers ------

@@ -50,6 +50,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 from . import ops
+from ._lib import collector_held
 from .models import VoxNeuS
 from .rendering import RaySampler
 
@@ -153,7 +154,7 @@ class _GraphBucket:
             self._run()  # warm caches (tables, scratch) outside capture
             stream.synchronize()
             self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph, pool=pool, stream=stream):
+            with collector_held(), torch.cuda.graph(self.graph, pool=pool, stream=stream):
                 self.out = self._run()
 
     def _run(self):

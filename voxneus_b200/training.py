@@ -23,7 +23,7 @@ from typing import Dict, Optional
 import torch
 from torch.optim import Optimizer
 
-from . import ops
+from . import _lib, ops
 from .models import VoxNeuS
 from .rendering import RaySampler
 
@@ -303,7 +303,7 @@ class FusedTrainer:
             g = _StepGraph(self, rays_o, rays_d, target, amplify, self.bitmap.device)
             self._graphs[amplify] = g
         self._refresh_occupancy(step)
-        g.run(rays_o, rays_d, target, step)
+        g.run(self, rays_o, rays_d, target, step)
         self.replayed_launches += g.launches
         return g.outputs
 
@@ -328,8 +328,9 @@ class _StepGraph:
     """
 
     def __init__(self, tr: FusedTrainer, rays_o, rays_d, target, amplify: bool, dev: torch.device):
+        # The trainer owns its graph: no reference back, so that a dropped trainer's graph and memory go at once and
+        # not with a later garbage collection.
         m = tr.model
-        self.tr = tr
         self.amplify = amplify
         # the inputs as one (3, N, 3) buffer: a caller whose rays and targets are the three slices of
         # one host tensor is served with a single copy
@@ -353,34 +354,32 @@ class _StepGraph:
         for opt in (self.grid_opt, self.net_opt):
             opt.zero_grad(set_to_none=True)  # backward inside the capture allocates the gradients
         amp_k = tr.amplify_k if amplify else 0.0
-        from . import _lib
-
         self.graph = torch.cuda.CUDAGraph(keep_graph=True)
         self.graph2 = None
         self.amp_k = amp_k
         l0 = _lib.launch_count()
         if tr.exchange is None:
-            with torch.cuda.graph(self.graph):
+            with _lib.collector_held(), torch.cuda.graph(self.graph):
                 self.outputs = tr._render_backward_regularize(self.o, self.d, self.t, amp_k)
-                self._optimizer_launches(m)
+                self._optimizer_launches(tr)
         else:
             # data-parallel ranks: two graphs, the collectives between them run eagerly (no NCCL
             # call inside a graph): render + backward, then V_R + regularizer + optimizers
-            with torch.cuda.graph(self.graph):
+            with _lib.collector_held(), torch.cuda.graph(self.graph):
                 loss, rgb = tr._render_backward(self.o, self.d, self.t, amp_k)
             self.graph.instantiate()
             tr._exchange(amp_k)  # the gradients the capture allocated, as every replay leaves them
             self.graph2 = torch.cuda.CUDAGraph(keep_graph=True)
-            with torch.cuda.graph(self.graph2):
+            with _lib.collector_held(), torch.cuda.graph(self.graph2):
                 self.outputs = tr._regularize(loss, rgb)
-                self._optimizer_launches(m)
+                self._optimizer_launches(tr)
             self.graph2.instantiate()
         self.launches = _lib.launch_count() - l0
         if self.graph2 is None:
             self.graph.instantiate()
 
-    def _optimizer_launches(self, m) -> None:
-        grid = m.sdf_grid.grid
+    def _optimizer_launches(self, tr: FusedTrainer) -> None:
+        grid = tr.model.sdf_grid.grid
         b1, b2 = self.grid_opt.param_groups[0]["betas"]
         st = self.grid_opt.state[grid]
         if self.grid_opt.formula == "torch":
@@ -389,7 +388,7 @@ class _StepGraph:
         else:
             ops.masked_adam_update_dev(grid, grid.grad, st["exp_avg"], st["exp_avg_sq"], self.scalars[0:1], b1, b2,
                                        self.grid_opt.param_groups[0]["eps"])
-        flag = self.tr.amp_flag if self.amplify else None
+        flag = tr.amp_flag if self.amplify else None
         batches: Dict[tuple, list] = {}
         for k, (gi, p) in enumerate(self.net_params):
             grp = self.net_opt.param_groups[gi]
@@ -403,10 +402,9 @@ class _StepGraph:
         for (b1, b2, eps), segs in batches.items():
             ops.adam_torch(segs, b1, b2, eps)
 
-    def _advance_scalars(self, step: int) -> torch.Tensor:
+    def _advance_scalars(self, tr: FusedTrainer, step: int) -> torch.Tensor:
         """Advance the optimizer state's step counts as the eager optimizers do; return this
         step's scalar row (the values the eager kernels would compute on the host)."""
-        tr = self.tr
         row = [0.0] * self.scalars.numel()
         grp = self.grid_opt.param_groups[0]
         st = self.grid_opt.state[tr.model.sdf_grid.grid]
@@ -433,7 +431,7 @@ class _StepGraph:
             row[3 + 3 * k:6 + 3 * k] = [ss, inv, amp]
         return torch.tensor(row, dtype=torch.float32)
 
-    def run(self, rays_o, rays_d, target, step: int) -> None:
+    def run(self, tr: FusedTrainer, rays_o, rays_d, target, step: int) -> None:
         b = rays_o._base
         if (b is not None and rays_d._base is b and target._base is b and b.shape == self.io.shape
                 and b.dtype == self.io.dtype and b.is_contiguous() and rays_o.data_ptr() == b[0].data_ptr()
@@ -447,12 +445,12 @@ class _StepGraph:
         self.slot = (s + 1) % _SCALAR_SLOTS
         if self.slot_events[s] is not None:
             self.slot_events[s].synchronize()  # the copy that last read this pinned slot has run
-        self.host[s].copy_(self._advance_scalars(step))
+        self.host[s].copy_(self._advance_scalars(tr, step))
         self.scalars.copy_(self.host[s], non_blocking=True)
         ev = self.slot_events[s] or torch.cuda.Event()
         ev.record()
         self.slot_events[s] = ev
         self.graph.replay()
         if self.graph2 is not None:  # data-parallel: the exchange between the two graphs
-            self.tr._exchange(self.amp_k)
+            tr._exchange(self.amp_k)
             self.graph2.replay()
