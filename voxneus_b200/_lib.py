@@ -285,14 +285,15 @@ def ptr(t: Optional[torch.Tensor]):
 
 
 def stream_ptr(device=None):
-    """The current stream of `device` (the current device when None) as an address."""
-    idx = device.index if isinstance(device, torch.device) else device
-    if not isinstance(idx, int):
-        if idx is not None:
-            idx = torch.device(idx).index
-        if idx is None:
-            idx = torch.cuda.current_device()
-    return torch._C._cuda_getCurrentRawStream(idx)
+    """The current stream of `device` (the current device when None) as an address. Refuses a device that is
+    not a CUDA device, so that no kernel is launched on host tensors."""
+    if device is not None and not isinstance(device, int):
+        if not isinstance(device, torch.device):
+            device = torch.device(device)
+        if device.type != "cuda":
+            raise ValueError(f"Expected a cuda device, but got: {device}")
+        device = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device is None else device)
 
 
 def check_tensor(t: torch.Tensor, name: str, dtype=torch.float32, device=None, contiguous=True):
