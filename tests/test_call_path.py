@@ -23,3 +23,13 @@ def test_mlp_modules_refuse_host_tensors():
     ws = [p.detach() for p in (mlp.net[0].weight, mlp.net[0].bias, mlp.net[2].weight, mlp.net[2].bias)]
     with pytest.raises(ValueError, match="Expected a cuda device"):
         ops.mlp_forward(torch.rand(5, 52), *ws)
+
+
+def test_host_triples_keep_the_sign_of_zero():
+    import math
+
+    from voxneus_b200._lib import f3
+
+    for v in ((0.0, 1.0, 2.0), (-0.0, 1.0, 2.0), (0.0, 1.0, 2.0)):
+        assert math.copysign(1.0, f3(v)[0]) == math.copysign(1.0, v[0])
+    assert f3((1, 2.5, -3))[:] == [1.0, 2.5, -3.0]

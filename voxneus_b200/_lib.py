@@ -259,7 +259,8 @@ def i3(v) -> ctypes.Array:
 
 
 def f3(v) -> ctypes.Array:
-    return _f3(tuple(map(float, v)))
+    v = tuple(map(float, v))
+    return _f3.__wrapped__(v) if 0.0 in v else _f3(v)  # 0.0 and -0.0 are one key
 
 
 def iarr(v) -> ctypes.Array:
