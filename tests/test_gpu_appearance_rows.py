@@ -87,3 +87,34 @@ def test_radiance_parts_equal_rows(p, offset, grads):
         assert torch.equal(n.grad.view(p, 3), want[0][:, 48:51])
     for w, g in zip(ws, want[1:]):
         assert torch.equal(w.grad, g)
+
+
+@pytest.mark.parametrize("change", [lambda t: t.mul_(0.5), lambda t: t.clamp_(0.4, 0.6), lambda t: t.data.mul_(0.5)],
+                         ids=["mul_", "clamp_", "data"])
+@pytest.mark.parametrize("rows", [False, True])
+def test_colours_may_be_changed_in_place_before_the_backward(rows, change):
+    """Neither MLP function keeps the tensor it returns, so a caller may change it; the gradients are those of
+    the same change out of place (the change's own part is left to autograd: none for .data)."""
+    from voxneus_b200 import ops
+    from voxneus_b200.models import RadianceMLP
+
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    mlp = RadianceMLP().to(DEV)
+    ws = [mlp.net[0].weight, mlp.net[0].bias, mlp.net[2].weight, mlp.net[2].bias]
+    x = torch.randn(300, 51, device=DEV, generator=gen).requires_grad_(True)
+    cot = torch.randn(300, 3, device=DEV, generator=gen)
+
+    def colours():
+        return ops.RadianceMLPFn.apply(x, *ws) if rows else mlp(x[:, :32], x[:, 32:48].detach(), x[:, 48:])
+
+    out = colours()
+    y = out.detach().clone()
+    change(out)
+    got = torch.autograd.grad((out * cot).sum(), [x, *ws])
+    u = y.clone().requires_grad_(True)
+    v = u * 1.0
+    change(v)
+    (d,) = torch.autograd.grad((v * cot).sum(), u)
+    want = torch.autograd.grad(colours(), [x, *ws], d)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)

@@ -620,13 +620,14 @@ class RadianceMLPFn(torch.autograd.Function):
     def forward(ctx, rows, W0, b0, W1, b1):
         mask = torch.empty(rows.shape[0], 2, dtype=torch.int32, device=rows.device)
         out = mlp_forward(rows.detach(), W0, b0, W1, b1, mask)
-        ctx.save_for_backward(rows, W0, b0, W1, b1, out, mask)
+        # a copy: callers may change the colours in place before the backward
+        ctx.save_for_backward(rows, W0, b0, W1, b1, out.clone(), mask)
         return out
 
     @staticmethod
     def backward(ctx, g):
         rows, W0, b0, W1, b1, out, mask = ctx.saved_tensors
-        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows.detach(), W0, b0, W1, b1, g, out.detach(), mask=mask)
+        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows.detach(), W0, b0, W1, b1, g, out, mask=mask)
         d_rows = None
         if ctx.needs_input_grad[0]:
             d_rows = torch.zeros(rows.shape, device=rows.device)
@@ -647,14 +648,15 @@ class RadiancePartsFn(torch.autograd.Function):
         call("vx_radiance_rows", ptr(h), ptr(v), ptr(n), p, ptr(rows), stream_ptr(h.device))
         mask = torch.empty(p, 2, dtype=torch.int32, device=h.device)
         out = mlp_forward(rows[:, :51], W0, b0, W1, b1, mask)
-        ctx.save_for_backward(rows, W0, b0, W1, b1, out, mask)
+        # a copy: callers may change the colours in place before the backward
+        ctx.save_for_backward(rows, W0, b0, W1, b1, out.clone(), mask)
         ctx.shapes = hash_features.shape, normals.shape
         return out
 
     @staticmethod
     def backward(ctx, g):
         rows, W0, b0, W1, b1, out, mask = ctx.saved_tensors
-        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows[:, :51], W0, b0, W1, b1, g, out.detach(), mask=mask)
+        d_hash, d_normal, dW0, db0, dW1, db1 = mlp_backward(rows[:, :51], W0, b0, W1, b1, g, out, mask=mask)
         need = ctx.needs_input_grad
         return (d_hash.reshape(ctx.shapes[0]) if need[0] else None, None,
                 d_normal.reshape(ctx.shapes[1]) if need[2] else None, dW0, db0, dW1, db1)
