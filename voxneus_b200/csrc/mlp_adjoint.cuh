@@ -12,6 +12,11 @@
 // operand needs three bf16 parts only: a float32's 24 bits cut into 8 + 8 + 8 (cut3), which
 // is exact, where a tf32 hi + lo pair carries 22 of them.
 //
+// A product with the mask is no selection: 0 times an infinity or a NaN is a NaN, and d x overflows where d W1 x does
+// not. So a sample of which no unit is active takes part with d = 0, and a block whose sums are not finite
+// forms them again on the CUDA cores, selecting (adj_plain_sums): units that such a sample leaves inactive keep
+// their gradients, as ReLU's adjoint has it.
+//
 // Layouts (no swizzle, 16-byte units; tc.cuh). The operands of G are written once, sample by sample,
 // and read with their sample index as the contraction: kind::f16 takes MN-major operands.
 //   A (G)    row r = c * stride + k of the 3 x features matrix, element (r, s) at
@@ -160,6 +165,113 @@ __device__ __forceinline__ bool adj_sync_or(bool v) {
       : "r"(v ? 1u : 0u), "n"(kAdjThreads)
       : "memory");
   return r != 0;
+}
+
+// The weight gradients of this block's tiles in plain float32, for blocks in which the products above leave the finite
+// range: dz = active ? sum_c d_c W1[c] : 0, dW0 = dz^T x, db0 = sum dz, dW1 = d^T h, db1 = sum d, in the layout of
+// pb. y and mask are formed again where the caller's launch kept them in d_hash's rows (row strides of 32), which
+// are overwritten by now. By the whole block; sm: its shared memory. 17 warps, ~10 us a tile: only for sums that
+// are not finite.
+template <int kMode>
+__device__ __noinline__ void adj_plain_sums(float* sm, const float* X, int64_t ldx, int64_t P, MlpW w, const float* d_out,
+                                            const float* y, int64_t ldy, const uint32_t* mask, int64_t ldm, float* pb,
+                                            RowSrc src) {
+  using S = AdjShape<kMode>;
+  constexpr int kXp = 53, kZp = 65;  // pitches
+  float* WS = sm;                    // W0 [64][51]
+  float* XS = WS + NH * KIN;         // x [128][kXp], feature 51 the one of db0
+  float* DZ = XS + TM * kXp;         // [128][kZp]
+  float* HS = DZ + TM * kZp;         // relu(z) [128][kZp]
+  float* DS = HS + TM * kZp;         // d [128][3]
+  float* RES = DS + TM * NO;         // [WG]
+  static_assert((NH * KIN + TM * (kXp + 2 * kZp + NO) + WG) * 4 <= 200 * 1024, "the block's shared memory");
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int e = tid; e < NH * KIN; e += kAdjThreads) WS[e] = w.W0[e];
+  for (int e = tid; e < WG; e += kAdjThreads) RES[e] = 0.0f;
+  const int64_t ntiles = (P + TM - 1) / TM;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    __syncthreads();  // the previous tile's values are read
+    for (int e = tid; e < TM * KIN; e += kAdjThreads) {
+      const int r = e / KIN, k = e - r * KIN;
+      const int64_t i = t * TM + r;
+      if (S::kCompact && k >= 32 && k < 48) continue;
+      XS[r * kXp + k] = i >= P ? 0.0f : S::kCompact ? X[i * KC + (k < 32 ? k : k - 16)] : X[i * ldx + k];
+    }
+    if (tid < TM) {
+      const int64_t i = t * TM + tid;
+      XS[tid * kXp + KIN] = i < P ? 1.0f : 0.0f;
+      if (S::kCompact) {
+        float sh[16];
+        const float* dir = src.rays_d + 3 * ((i < P ? i : P - 1) / src.S);
+        sh16(dir[0], dir[1], dir[2], sh);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) XS[tid * kXp + 32 + k] = sh[k];
+      }
+    }
+    __syncthreads();
+    for (int r = wid; r < TM; r += kAdjThreads / 32) {  // a warp a sample, two hidden units a lane
+      const int64_t i = t * TM + r;
+      float z[2] = {w.b0[lane], w.b0[lane + 32]};
+      for (int k = 0; k < KIN; ++k) {
+        z[0] = fmaf(WS[lane * KIN + k], XS[r * kXp + k], z[0]);
+        z[1] = fmaf(WS[(lane + 32) * KIN + k], XS[r * kXp + k], z[1]);
+      }
+      float h[2], d[NO];
+      bool on[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        on[u] = i < P && (ldm == 2 ? (mask[i * 2 + u] >> lane & 1u) != 0 : z[u] > 0.0f);
+        h[u] = on[u] ? z[u] : 0.0f;
+      }
+#pragma unroll
+      for (int c = 0; c < NO; ++c) {
+        float v = 0.0f;
+        if (ldy != NO)
+          v = sigmoidf_ref(w.b1[c] + warp_sum(fmaf(w.W1[c * NH + lane], h[0], w.W1[c * NH + lane + 32] * h[1])));
+        else if (i < P)
+          v = y[i * NO + c];
+        v = __shfl_sync(0xffffffffu, v, 0);
+        d[c] = i < P ? d_out[i * NO + c] * ((1.0f - v) * v) : 0.0f;
+        if (lane == 0) DS[r * NO + c] = d[c];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int n = lane + 32 * u;
+        const float dh = d[0] * w.W1[n] + d[1] * w.W1[NH + n] + d[2] * w.W1[2 * NH + n];
+        DZ[r * kZp + n] = on[u] ? dh : 0.0f;
+        HS[r * kZp + n] = h[u];
+      }
+    }
+    __syncthreads();
+    for (int e = tid; e < WG; e += kAdjThreads) {  // each thread's own entries
+      const float *a, *b;
+      int pa = kZp, pbb = NO;
+      if (e < NH * KP) {  // dW0, and db0 in its padding column
+        a = DZ + e / KP;
+        b = XS + e % KP;
+        pbb = kXp;
+      } else if (e < NH * KP + NO * NH) {
+        a = HS + (e - NH * KP) % NH;
+        b = DS + (e - NH * KP) / NH;
+      } else if (e >= WG - NO) {  // db1: the ones of the samples are its other factor
+        a = XS + KIN;
+        pa = kXp;
+        b = DS + (e - (WG - NO));
+      } else {
+        continue;
+      }
+      float v = 0.0f;
+#pragma unroll 4
+      for (int r = 0; r < TM; ++r)
+        if (t * TM + r < P) v = fmaf(a[r * pa], b[r * pbb], v);
+      RES[e] += v;
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < WG; e += kAdjThreads) {
+    const int n = e - NH * KP - NO * NH;  // db0's unit
+    pb[e] = n >= 0 && n < NH ? RES[n * KP + KIN] : e < NH * KP && e % KP == KIN ? 0.0f : RES[e];
+  }
 }
 
 // X (P rows), d_out (P,3), the forward's colours y (row stride ldy) and mask bits (two words a row,
@@ -347,7 +459,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     // Folded: they arrive with the rows. Otherwise loaded here a tile ahead of their use (and, for
     // kAdjStrided, this thread's share of the rows).
     float dy[NO], yv[NO], d[NO];
-    uint32_t bits = 0;
+    uint32_t bits[2] = {0, 0};
     float pre[13], dir[3] = {0.0f, 0.0f, 0.0f};  // dir: kFold, one thread, the tile's ray
     auto load_tile = [&](int64_t t) {
       if (kFold) {
@@ -364,7 +476,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         dy[c] = in ? __ldg(d_out + i * NO + c) : 0.0f;
         yv[c] = in ? y[i * ldy + c] : 0.0f;
       }
-      bits = in ? mask[i * ldm + (hh >> 1)] : 0u;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) bits[k] = in ? mask[i * ldm + k] : 0u;
       if (!S::kBulk) {
 #pragma unroll
         for (int k = 0; k < 13; ++k) {
@@ -384,7 +497,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           dy[c] = aux[NO * m + c];
           yv[c] = aux[NO * (TM + m) + c];
         }
-        bits = __float_as_uint(aux[2 * NO * TM + 2 * m + (hh >> 1)]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) bits[k] = __float_as_uint(aux[2 * NO * TM + 2 * m + k]);
         if (tid == kAdjShTid) {
           float sh[16];
           sh16(dir[0], dir[1], dir[2], sh);
@@ -395,8 +509,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 #pragma unroll
       for (int c = 0; c < NO; ++c) d[c] = dy[c] * ((1.0f - yv[c]) * yv[c]);  // 0 on rows past P
       sb += hh == 0 ? d[0] : (hh == 1 ? d[1] : d[2]);
+      if ((bits[0] | bits[1]) == 0u) d[0] = d[1] = d[2] = 0.0f;  // no unit is active: nothing to pass on
       __syncwarp();
-      stage_mask(MK + buf * kAdjMask, tb + lane_base + kAdjMk + 8 * hh, m, hh, bits >> (16 * (hh & 1)));
+      stage_mask(MK + buf * kAdjMask, tb + lane_base + kAdjMk + 8 * hh, m, hh, bits[hh >> 1] >> (16 * (hh & 1)));
       if (!S::kBulk) {
 #pragma unroll
         for (int k = 0; k < 13; ++k) {
@@ -604,13 +719,20 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
 #pragma unroll
     for (int k = 0; k < 8; ++k) SHD[pair * 17 + sh0 + k] = shacc[k];
   }
+  bool finite = fabsf(sb) < INFINITY;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {  // rows past 3 * kStride hold nothing
+    finite = finite && (m >= 3 * S::kStride || fabsf(acc[i]) < INFINITY);
+    if (!kFold) finite = finite && (m + S::kRow2 >= 3 * S::kStride || fabsf(acc2[i]) < INFINITY);
+    if (kFold && i < 8) finite = finite && fabsf(shacc[i]) < INFINITY;
+  }
   sb = warp_sum(sb);
   if (hh < NO && lane == 0) SB[hh * 4 + q] = sb;
-  __syncthreads();
+  const bool plain = __syncthreads_or(have && !finite);
   constexpr int kOnes = kFold ? 35 : 51;
   // a warp per hidden unit, lanes over the 51 columns of W0 (and the padding column, 0)
 #pragma unroll 4
-  for (int n = wid; n < NH; n += kAdjThreads / 32) {
+  for (int n = plain ? NH : wid; n < NH; n += kAdjThreads / 32) {
     float w1[NO], s[NO];
 #pragma unroll
     for (int c = 0; c < NO; ++c) {
@@ -644,10 +766,11 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     }
     if (lane == 0) pb[NH * KP + NO * NH + n] = db;
   }
-  if (tid < NO) {
+  if (tid < NO && !plain) {
     const float* s = SB + tid * 4;
     pb[NH * KP + NO * NH + NH + tid] = have ? (s[0] + s[1]) + (s[2] + s[3]) : 0.0f;
   }
+  if (plain) adj_plain_sums<kMode>(reinterpret_cast<float*>(smem), X, ldx, P, w, d_out, y, ldy, mask, ldm, pb, src);
   tc::fence_before_sync();
   __syncthreads();
   __syncwarp();
