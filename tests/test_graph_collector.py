@@ -60,18 +60,32 @@ def _step(seed):
 
 
 @pytest.mark.gpu
-def test_a_dropped_graph_waiting_for_the_collector_does_not_break_a_capture():
+def test_a_dropped_graph_waiting_for_the_collector_does_not_break_a_capture(monkeypatch):
+    """A trainer that only the collector frees is garbage when the next one captures its step, and the objects made
+    inside the capture are more than the collector's threshold."""
+    from voxneus_b200 import training
+
+    inner, keep = training.FusedTrainer._render_backward, gc.get_threshold()
+
+    def busy(self, *a, **k):
+        if torch.cuda.is_current_stream_capturing():
+            gc.set_threshold(50, 1, 1)
+            kept = [[i] for i in range(5000)]
+            assert kept
+        return inner(self, *a, **k)
+
     gc.collect()
-    keep = gc.get_threshold()
-    for seed in range(3):
-        ring = [_step(seed)]
-        ring.append(ring)  # garbage that only the collector frees
+    gc.set_threshold(10 ** 9)
+    try:
+        ring = [_step(0)]
+        gone = weakref.ref(ring[0])
+        ring.append(ring)
         del ring
-        gc.set_threshold(1, 1, 1)  # a full collection every few allocations
-        try:
-            _step(10 + seed)
-        finally:
-            gc.set_threshold(*keep)
+        assert gone() is not None
+        monkeypatch.setattr(training.FusedTrainer, "_render_backward", busy)
+        _step(1)
+    finally:
+        gc.set_threshold(*keep)
     torch.cuda.synchronize()
 
 
