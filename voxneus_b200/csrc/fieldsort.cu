@@ -42,7 +42,7 @@ constexpr int kDenseNormals = 160, kDenseSdf = 256, kDenseMean = 400;
 constexpr int kSmemBins = 48 * 1024;        // bins of a block's histogram in shared memory
 constexpr int64_t kBatch = int64_t(1) << 24;  // points per pass: bounds the workspace
 constexpr int kMaxAxis = 1 << 24;             // longer axes (float32 cell numbers): the plain kernel
-constexpr int kMaxBins = 1 << 22;             // of grids below 2^31 voxels with such axes: 1 x 4 x 2^20 bricks
+constexpr int kMaxBins = 1 << 22;             // more bricks (grids a few voxels thick): the plain kernel
 
 struct Bins {
   int n[3];
@@ -55,7 +55,22 @@ Bins make_bins(const int32_t res[3]) {
   return b;
 }
 
-inline bool long_axis(const int32_t res[3]) { return res[0] > kMaxAxis || res[1] > kMaxAxis || res[2] > kMaxAxis; }
+// Bricks of a bucket: 2^bucket_shift.
+inline int bucket_shift(int64_t nbins) {
+  int shift = 0;
+  while (((nbins - 1) >> shift) >= kBuckets) ++shift;
+  return shift;
+}
+
+// Dynamic shared memory of k_brick_order: a tile's records with their bricks, and two counters a brick of the bucket.
+constexpr size_t order_bytes(int shift) { return (size_t)kTile * 18 + ((size_t)8 << shift); }
+static_assert(kMaxBins / kBuckets == 1 << 14 && order_bytes(14) <= 220 * 1024, "the largest bucket's counters fit");
+
+// Grids that the bricks do not take and the plain kernel does: axes too long for exact cell numbers, and more
+// bricks than the buckets' counters hold (2 x 65 x 16,000,000 has 5 M, a cube of 2^31 voxels 0.5 M).
+inline bool plain_grid(const int32_t res[3]) {
+  return res[0] > kMaxAxis || res[1] > kMaxAxis || res[2] > kMaxAxis || make_bins(res).total() > kMaxBins;
+}
 
 __device__ __forceinline__ int point_bin(const Grid& g, const Bins& b, float px, float py, float pz) {
   // cell indices (the clamp of gs_coord keeps them in [0, R-1]; NaN reads as 0)
@@ -510,7 +525,7 @@ extern "C" {
 int64_t vx_field_query_sorted_workspace(int64_t n, const int32_t res[3]) {
   if (n <= 0 || n > INT32_MAX || !res) return 0;
   if (res[0] < 2 || res[1] < 2 || res[2] < 2) return 0;
-  if (long_axis(res)) return kAlign;
+  if (plain_grid(res)) return kAlign;
   return make_layout(n < kBatch ? n : kBatch, make_bins(res).total()).bytes;
 }
 
@@ -526,7 +541,7 @@ int vx_field_query_sorted(const float* grid, const int32_t res[3], const float x
   VX_REQUIRE(workspace_bytes >= need, "workspace holds %lld bytes, need %lld", (long long)workspace_bytes,
              (long long)need);
   VX_REQUIRE(((uintptr_t)workspace & (kAlign - 1)) == 0, "workspace must be 256-byte aligned");
-  if (long_axis(res))
+  if (plain_grid(res))
     return vx_field_query(grid, res, xyz_min, xyz_max, xyz, n, sdf, grad, normal, nullptr, nullptr, stream);
   const Bins b = make_bins(res);
   const int64_t nbins = b.total();
@@ -543,16 +558,15 @@ int vx_field_query_sorted(const float* grid, const int32_t res[3], const float x
   int2* list = reinterpret_cast<int2*>(w + l.list);
   const bool normals = grad || normal;
   const int vec = res[2] % 4 == 0 && (reinterpret_cast<uintptr_t>(grid) & 15) == 0;
-  int shift = 0;
-  while (((nbins - 1) >> shift) >= kBuckets) ++shift;
+  const int shift = bucket_shift(nbins);
   const int nbuckets = (int)((nbins - 1) >> shift) + 1;
-  const size_t count_smem = nbins <= kSmemBins ? (size_t)nbins * 4 : 0, order_smem = (size_t)kTile * 18 + ((size_t)8 << shift);
+  const size_t count_smem = nbins <= kSmemBins ? (size_t)nbins * 4 : 0, order_smem = order_bytes(shift);
   constexpr int part_smem = kTile * 17;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaFuncSetAttribute(k_bin_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBins * 4);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_brick_order, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kTile * 18 + 8 * (kMaxBins / kBuckets));
+                             (int)order_bytes(bucket_shift(kMaxBins)));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_partition, cudaFuncAttributeMaxDynamicSharedMemorySize, part_smem);
   int launches = 0;
   for (int64_t i0 = 0; i0 < n && e == cudaSuccess; i0 += kBatch) {
@@ -571,6 +585,8 @@ int vx_field_query_sorted(const float* grid, const int32_t res[3], const float x
     k_partition<<<tiles, kTileThreads, part_smem, st>>>(p, m, g, b, shift, starts, cursor + nbins, place, res0);
     k_brick_order<<<tiles + nbuckets, kTileThreads, order_smem, st>>>(res0, g, b, shift, nbuckets, starts, cursor, rec);
     launches += 6;
+    e = cudaGetLastError();  // what follows stores at the places that these four wrote
+    if (e != cudaSuccess) break;
     // at least the work list's length
     const unsigned blocks = (unsigned)((nbins < m / dense ? nbins : m / dense) + m / kChunk);
     float* s = reinterpret_cast<float*>(res0);
