@@ -1,0 +1,51 @@
+"""The brick query beyond one pass and without its workspace, bit for bit against the plain query: more than 2^24 points
+(offset outputs, a reused workspace, a short last pass whose bricks are sparse where the full pass's are staged), and
+the plain kernel in its place when the workspace cannot be allocated."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = torch.device("cuda", 0)
+LO, HI = (-1.0, -1.1, -0.9), (1.0, 0.9, 1.1)
+
+
+def _equal(want, a, b):
+    for w, x, y in zip(want, a, b):
+        assert (y is None) == (not w)
+        if w:
+            assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+
+
+@pytest.mark.parametrize("rest", [1, 4099, (1 << 24) + 7])
+def test_more_points_than_a_pass(rest):
+    from voxneus_b200 import ops
+
+    torch.manual_seed(1)
+    grid = torch.randn(1, 1, 64, 64, 64, device=DEV)
+    pts = torch.rand((1 << 24) + rest, 3, device=DEV) * 2.2 - 1.1
+    a = ops.field_query(grid, LO, HI, pts, sdf=True, grad=True, normal=True)[:3]
+    for want in ((1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)):
+        _equal(want, a, ops.field_query_sorted(grid, LO, HI, pts, *map(bool, want))[:3])
+
+
+def test_no_room_for_the_workspace(monkeypatch):
+    from voxneus_b200 import ops
+
+    torch.manual_seed(2)
+    grid = torch.randn(1, 1, 40, 40, 40, device=DEV)
+    pts = torch.rand(30_001, 3, device=DEV) * 2.0 - 1.0
+    a = ops.field_query_sorted(grid, LO, HI, pts, True, True, True)[:3]
+    real, tried = torch.empty, []
+
+    def empty(*args, **kw):
+        if kw.get("dtype") is torch.uint8:
+            tried.append(args)
+            raise torch.cuda.OutOfMemoryError("no room")
+        return real(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    for want in ((1, 1, 1), (1, 0, 0)):
+        _equal(want, a, ops.field_query_sorted(grid, LO, HI, pts, *map(bool, want))[:3])
+    assert len(tried) == 2
