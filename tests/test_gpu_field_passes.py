@@ -49,3 +49,31 @@ def test_no_room_for_the_workspace(monkeypatch):
     for want in ((1, 1, 1), (1, 0, 0)):
         _equal(want, a, ops.field_query_sorted(grid, LO, HI, pts, *map(bool, want))[:3])
     assert len(tried) == 2
+
+
+@pytest.mark.parametrize("res", [(48, 50, 52), (600, 600, 560)], ids=["counted in shared memory", "in device memory"])
+@pytest.mark.parametrize("kind", ["outside", "nan", "cell", "five cells", "six cells", "runs"])
+def test_crowded_points(res, kind):
+    """Points of few cells among 32 neighbours, answered in the order they came: to the line between them and
+    bricks from both sides, and crowded stretches beside scattered ones."""
+    from voxneus_b200 import ops
+
+    torch.manual_seed(4)
+    grid = torch.randn(1, 1, *res, device=DEV)
+    n = 40_961
+    pts = torch.rand(n, 3, device=DEV) * 2.0 - 1.0
+    cell = 2.0 / max(res)
+    if kind == "outside":
+        pts += 4.0
+    elif kind == "nan":
+        pts[:] = float("nan")
+    elif kind == "cell":
+        pts = 0.3 + 0.5 * cell * torch.rand(n, 3, device=DEV)
+    elif kind.endswith("cells"):
+        at = torch.arange(n, device=DEV) % (5 if kind == "five cells" else 6)
+        pts = (torch.rand(6, 3, device=DEV) * 1.6 - 0.8)[at]
+    else:
+        pts[: n * 9 // 10] = 0.2
+    a = ops.field_query(grid, LO, HI, pts, sdf=True, grad=True, normal=True, corners=True)[:3]  # the plain kernel
+    for want in ((1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1)):
+        _equal(want, a, ops.field_query_sorted(grid, LO, HI, pts, *map(bool, want))[:3])

@@ -16,6 +16,8 @@
 //   query      a brick's points from shared memory, or those of sparse bricks from the grid; results at k,
 //              inside the bucket's window
 //   collect    each point's result from its k: neighbours of a partition block read the same 256 runs
+// Points that crowd into a few cells, 32 neighbours at a time, as a caller's own order or the clamp of points outside
+// the box may have them, are answered in the order they came (kCrowded).
 // What bounds it: DRAM traffic (records, grid, results: ~180 bytes a point with normals and the grid once)
 // and, with normals, issue. 2^24 uniform points of a 512^3 grid, one query of
 // the SDF and one of gradient and normal: 4.40 ms (Morton keys, a four-pass radix sort, queries through
@@ -39,6 +41,11 @@ constexpr int kBuckets = 256;               // at most
 // points 536 against ~1080 and 270 against ~460. From a mean of kDenseMean on all are staged, which saves
 // the other pass over the records.
 constexpr int kDenseNormals = 160, kDenseSdf = 256, kDenseMean = 400;
+// With at most this many cells among 32 consecutive points on average, the points are queried in the order they came,
+// with nothing moved. 2^24 points with gradients and normals, all in one cell (1 cell in 32 points), 9 in 10 there and the
+// rest anywhere (4.2), 8 in 10 (7.4): 564, 1009 and 1150 us so, 1101, 1324 and 1291 us by bricks. The line lies lower than
+// where these meet because crowded and scattered stretches may also follow one another (8 in 10 so: ~1730 us).
+constexpr int kCrowded = 5;
 constexpr int kSmemBins = 48 * 1024;        // bins of a block's histogram in shared memory
 constexpr int64_t kBatch = int64_t(1) << 24;  // points per pass: bounds the workspace
 constexpr int kMaxAxis = 1 << 24;             // longer axes (float32 cell numbers): the plain kernel
@@ -80,24 +87,63 @@ __device__ __forceinline__ int point_bin(const Grid& g, const Bins& b, float px,
   return (x * b.n[1] + y) * b.n[2] + z;
 }
 
+// What k_bin_count saw of the points' order, every fourth run of 32 of a block's: how many runs, and their cells.
+struct Sample {
+  int runs, cells;
+};
+
+__device__ __forceinline__ bool crowded(const Sample* s) {
+  const int runs = __ldg(&s->runs);
+  return runs > 0 && __ldg(&s->cells) <= kCrowded * runs;
+}
+
 // Points per brick. kSmem: a histogram per block (one block per SM), added up at its end; otherwise (more
 // bricks than fit) straight into the counts.
 template <bool kSmem>
 __global__ void __launch_bounds__(kCountThreads) k_bin_count(const float* __restrict__ xyz, int64_t n, Grid g, Bins b,
-                                                            int* __restrict__ counts) {
+                                                            int* __restrict__ counts, Sample* __restrict__ sample) {
   extern __shared__ int hist[];
-  const int nbins = (int)b.total();
-  if (kSmem) {
+  __shared__ int seen[2];
+  const int nbins = (int)b.total(), lane = threadIdx.x & 31;
+  int runs = 0, cells = 0;
+  if (threadIdx.x < 2) seen[threadIdx.x] = 0;
+  if (kSmem)
     for (int i = threadIdx.x; i < nbins; i += kCountThreads) hist[i] = 0;
-    __syncthreads();
+  __syncthreads();
+  constexpr int kPer = 4;  // points a thread, their loads in flight together
+  const int64_t step = (int64_t)gridDim.x * kCountThreads;
+  for (int64_t i0 = blockIdx.x * (int64_t)kCountThreads + threadIdx.x; i0 - lane < n; i0 += kPer * step) {  // whole warps
+    float p[kPer][3];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int64_t i = i0 + u * step;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) p[u][a] = i < n ? __ldg(xyz + 3 * i + a) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int64_t i = i0 + u * step;
+      const int x = (int)gs_coord(p[u][0], g.lo[0], g.den[0], g.inv_den[0], g.rx);
+      const int y = (int)gs_coord(p[u][1], g.lo[1], g.den[1], g.inv_den[1], g.ry);
+      const int z = (int)gs_coord(p[u][2], g.lo[2], g.den[2], g.inv_den[2], g.rz);
+      if (i < n) atomicAdd((kSmem ? hist : counts) + (x / kBrick * b.n[1] + y / kBrick) * b.n[2] + z / kBrick, 1);
+      if (u == 0 && i - lane + 32 <= n) {
+        const unsigned same = __match_any_sync(0xffffffffu, lin3(g, x, y, z));
+        cells += __popc(__ballot_sync(0xffffffffu, __ffs(same) - 1 == lane));
+        ++runs;
+      }
+    }
   }
-#pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)kCountThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kCountThreads) {
-    const int bin = point_bin(g, b, __ldg(xyz + 3 * i), __ldg(xyz + 3 * i + 1), __ldg(xyz + 3 * i + 2));
-    atomicAdd((kSmem ? hist : counts) + bin, 1);
+  if (lane == 0) {
+    atomicAdd(seen, runs);
+    atomicAdd(seen + 1, cells);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicAdd(&sample->runs, seen[0]);
+    atomicAdd(&sample->cells, seen[1]);
   }
   if (kSmem) {
-    __syncthreads();
     for (int i = threadIdx.x; i < nbins; i += kCountThreads)
       if (hist[i]) atomicAdd(counts + i, hist[i]);
   }
@@ -106,12 +152,13 @@ __global__ void __launch_bounds__(kCountThreads) k_bin_count(const float* __rest
 constexpr int kScanBins = 4096;  // bins of a scan block, 4 a thread
 
 // Counts -> their exclusive starts, and the work list of bricks with at least `dense` points: {brick, first
-// record} of every chunk, nchunks entries in any order. A block adds up the counts before its own bins
+// record} of every chunk, nchunks entries in any order (none for crowded points). A block adds up the counts before its own bins
 // itself (L2 reads, all in flight at once) instead of waiting for the blocks before it: 32,768 bins take
 // 6 us, 26 as one block's loop over carries.
 __global__ void __launch_bounds__(1024) k_bin_scan(const int* __restrict__ counts, int64_t nbins, int dense,
                                                    int* __restrict__ starts, int* __restrict__ nchunks,
-                                                   int2* __restrict__ list) {
+                                                   int2* __restrict__ list, const Sample* __restrict__ sample) {
+  if (crowded(sample)) return;
   __shared__ int2 part[32];
   __shared__ int before[32], first;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -203,7 +250,8 @@ __device__ __forceinline__ void scan_counts(const int* cnt, int* loc, int width)
 __global__ void __launch_bounds__(kTileThreads, 2) k_partition(const float* __restrict__ xyz, int64_t n, Grid g, Bins b,
                                                                int shift, const int* __restrict__ starts,
                                                                int* __restrict__ cursor, int* __restrict__ place,
-                                                               float4* __restrict__ rec) {
+                                                               float4* __restrict__ rec, const Sample* __restrict__ sample) {
+  if (crowded(sample)) return;
   extern __shared__ __align__(16) float4 stage[];  // [kTile]
   uint8_t* which = reinterpret_cast<uint8_t*>(stage + kTile);  // [kTile] bucket of a staged record
   __shared__ int cnt[kBuckets], loc[kBuckets], delta[kBuckets];
@@ -249,7 +297,9 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_partition(const float* __re
 // the buckets' sizes.
 __global__ void __launch_bounds__(kTileThreads, 2) k_brick_order(const float4* __restrict__ rec, Grid g, Bins b, int shift,
                                                               int nbuckets, const int* __restrict__ starts,
-                                                              int* __restrict__ cursor, float4* __restrict__ out) {
+                                                              int* __restrict__ cursor, float4* __restrict__ out,
+                                                              const Sample* __restrict__ sample) {
+  if (crowded(sample)) return;
   extern __shared__ __align__(16) float4 stage[];  // [kTile]
   uint16_t* which = reinterpret_cast<uint16_t*>(stage + kTile);  // [kTile] bin of a staged record
   int* hist = reinterpret_cast<int*>(which + kTile);              // [2^shift] counts, then deltas
@@ -345,8 +395,8 @@ __device__ __forceinline__ void store_normals(const float* f, const Grid& g, con
 template <bool kNormals>
 __global__ void __launch_bounds__(kQueryThreads, kNormals ? 4 : 6)
     k_brick_query(const float* __restrict__ f, Grid g, Bins b, int vec, const int* __restrict__ starts,
-                  const int* __restrict__ nchunks, const int2* __restrict__ list, const float4* __restrict__ rec, float4* __restrict__ res, int want_sdf, int want_normal,
-                  float* __restrict__ sdf) {
+                  const int* __restrict__ nchunks, const int2* __restrict__ list, const float4* __restrict__ rec,
+                  float4* __restrict__ res, int want_sdf, int want_normal, float* __restrict__ sdf) {
   __shared__ __align__(16) float vox[kReg * kReg * kPitch];
   if ((int)blockIdx.x >= __ldg(nchunks)) return;
   const int tid = threadIdx.x;
@@ -425,13 +475,43 @@ __global__ void __launch_bounds__(kQueryThreads, kNormals ? 4 : 6)
   }
 }
 
+// A pass's outputs, null where not asked for.
+struct PointOut {
+  float *sdf, *grad, *normal;
+};
+
 // The records of bricks with fewer than `dense` points, a thread each, from the grid itself: staging a brick
-// costs 34 KB of reads.
+// costs 34 KB of reads. Crowded points: all of them, from xyz to the caller's outputs.
 template <bool kNormals>
 __global__ void __launch_bounds__(256) k_sparse_query(const float* __restrict__ f, Grid g, Bins b, int dense,
                                                       const int* __restrict__ starts, const float4* __restrict__ rec,
                                                       int64_t n, float4* __restrict__ res, int want_sdf, int want_normal,
-                                                      float* __restrict__ sdf) {
+                                                      float* __restrict__ sdf, const Sample* __restrict__ sample,
+                                                      const float* __restrict__ xyz, PointOut out) {
+  if (crowded(sample)) {
+    for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+      const float px = __ldg(xyz + 3 * i), py = __ldg(xyz + 3 * i + 1), pz = __ldg(xyz + 3 * i + 2);
+      if (!kNormals) {
+        out.sdf[i] = query_sdf(f, g, px, py, pz);
+        continue;
+      }
+      Eq7 e;
+      eq7_setup(g, px, py, pz, e);
+      float w[8], c[8], gr[3], nn[3], len;
+      eq7_load_block(f, g, e, c);
+      if (out.sdf) out.sdf[i] = query_sdf_block(f, g, px, py, pz, e, c);
+      eq7_weights(e, w);
+      eq7_gradient_block(f, g, e, w, c, gr);
+      normalize_eps(gr, nn, len);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (out.grad) out.grad[3 * i + a] = gr[a];
+        if (out.normal) out.normal[3 * i + a] = nn[a];
+      }
+    }
+    return;
+  }
+  if (dense <= 1) return;
   for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
     const float4 q = __ldg(rec + i);
     const int bin = point_bin(g, b, q.x, q.y, q.z);
@@ -456,8 +536,10 @@ __global__ void __launch_bounds__(256) k_sparse_query(const float* __restrict__ 
 // Each point's results from its place.
 template <bool kNormals>
 __global__ void __launch_bounds__(256) k_collect(const int* __restrict__ place, int64_t n, const float4* __restrict__ res,
-                                                 const float* __restrict__ s, float* __restrict__ sdf,
-                                                 float* __restrict__ grad, float* __restrict__ normal) {
+                                                 const float* __restrict__ s, PointOut out,
+                                                 const Sample* __restrict__ sample) {
+  if (crowded(sample)) return;
+  float *sdf = out.sdf, *grad = out.grad, *normal = out.normal;
   constexpr int kPer = 4;  // points a thread, their loads in flight together
   for (int64_t i0 = blockIdx.x * (int64_t)(256 * kPer) + threadIdx.x; i0 < n; i0 += (int64_t)gridDim.x * 256 * kPer) {
     int64_t k[kPer];
@@ -509,7 +591,7 @@ Layout make_layout(int64_t batch, int64_t nbins) {
   l.starts = l.place + align_up(batch * 4);
   l.counts = l.starts + align_up((nbins + 1) * 4);
   l.cursor = l.counts + align_up(nbins * 4);
-  l.zeroed = align_up(nbins * 4) + (nbins + kBuckets + 1) * 4;  // counts and cursors
+  l.zeroed = align_up(nbins * 4) + (nbins + kBuckets + 3) * 4;  // counts, cursors and sample
   l.list = l.counts + align_up(l.zeroed);
   l.bytes = l.list + align_up(((nbins < batch ? nbins : batch) + batch / kChunk) * 8);
   return l;
@@ -555,6 +637,7 @@ int vx_field_query_sorted(const float* grid, const int32_t res[3], const float x
   int* counts = reinterpret_cast<int*>(w + l.counts);
   int* cursor = reinterpret_cast<int*>(w + l.cursor);  // [nbins] bricks, [kBuckets], the work list's length
   int* nchunks = cursor + nbins + kBuckets;
+  Sample* sample = reinterpret_cast<Sample*>(nchunks + 1);
   int2* list = reinterpret_cast<int2*>(w + l.list);
   const bool normals = grad || normal;
   const int vec = res[2] % 4 == 0 && (reinterpret_cast<uintptr_t>(grid) & 15) == 0;
@@ -577,37 +660,37 @@ int vx_field_query_sorted(const float* grid, const int32_t res[3], const float x
     const unsigned tiles = (unsigned)((m + kTile - 1) / kTile);
     const int dense = m < (int64_t)kDenseMean * nbins ? (normals ? kDenseNormals : kDenseSdf) : 1;
     if (count_smem)
-      k_bin_count<true><<<tiles < kSMs ? tiles : kSMs, kCountThreads, count_smem, st>>>(p, m, g, b, counts);
+      k_bin_count<true><<<tiles < kSMs ? tiles : kSMs, kCountThreads, count_smem, st>>>(p, m, g, b, counts, sample);
     else
-      k_bin_count<false><<<grid_for(m, kCountThreads, 2), kCountThreads, 0, st>>>(p, m, g, b, counts);
+      k_bin_count<false><<<grid_for(m, kCountThreads, 2), kCountThreads, 0, st>>>(p, m, g, b, counts, sample);
     k_bin_scan<<<(unsigned)((nbins + kScanBins - 1) / kScanBins), 1024, 0, st>>>(counts, nbins, dense, starts, nchunks,
-                                                                               list);
-    k_partition<<<tiles, kTileThreads, part_smem, st>>>(p, m, g, b, shift, starts, cursor + nbins, place, res0);
-    k_brick_order<<<tiles + nbuckets, kTileThreads, order_smem, st>>>(res0, g, b, shift, nbuckets, starts, cursor, rec);
+                                                                               list, sample);
+    k_partition<<<tiles, kTileThreads, part_smem, st>>>(p, m, g, b, shift, starts, cursor + nbins, place, res0, sample);
+    k_brick_order<<<tiles + nbuckets, kTileThreads, order_smem, st>>>(res0, g, b, shift, nbuckets, starts, cursor, rec,
+                                                                             sample);
     launches += 6;
     e = cudaGetLastError();  // what follows stores at the places that these four wrote
     if (e != cudaSuccess) break;
     // at least the work list's length
     const unsigned blocks = (unsigned)((nbins < m / dense ? nbins : m / dense) + m / kChunk);
+    const PointOut out{sdf ? sdf + i0 : nullptr, grad ? grad + 3 * i0 : nullptr, normal ? normal + 3 * i0 : nullptr};
     float* s = reinterpret_cast<float*>(res0);
     if (normals) {
       if (blocks)
         k_brick_query<true><<<blocks, kQueryThreads, 0, st>>>(grid, g, b, vec, starts, nchunks, list, rec, res0,
                                                               sdf != nullptr, normal != nullptr, nullptr);
-      if (dense > 1)
-        k_sparse_query<true><<<grid_for(m, 256), 256, 0, st>>>(grid, g, b, dense, starts, rec, m, res0, sdf != nullptr,
-                                                               normal != nullptr, nullptr);
-      k_collect<true><<<grid_for(m, 256), 256, 0, st>>>(place, m, res0, nullptr, sdf ? sdf + i0 : nullptr,
-                                                        grad ? grad + 3 * i0 : nullptr, normal ? normal + 3 * i0 : nullptr);
+      k_sparse_query<true><<<grid_for(m, 256), 256, 0, st>>>(grid, g, b, dense, starts, rec, m, res0, sdf != nullptr,
+                                                             normal != nullptr, nullptr, sample, p, out);
+      k_collect<true><<<grid_for(m, 256), 256, 0, st>>>(place, m, res0, nullptr, out, sample);
     } else {
       if (blocks)
         k_brick_query<false><<<blocks, kQueryThreads, 0, st>>>(grid, g, b, vec, starts, nchunks, list, rec, nullptr, 1, 0,
                                                                s);
-      if (dense > 1)
-        k_sparse_query<false><<<grid_for(m, 256), 256, 0, st>>>(grid, g, b, dense, starts, rec, m, nullptr, 1, 0, s);
-      k_collect<false><<<grid_for(m, 256), 256, 0, st>>>(place, m, nullptr, s, sdf + i0, nullptr, nullptr);
+      k_sparse_query<false><<<grid_for(m, 256), 256, 0, st>>>(grid, g, b, dense, starts, rec, m, nullptr, 1, 0, s, sample,
+                                                              p, out);
+      k_collect<false><<<grid_for(m, 256), 256, 0, st>>>(place, m, nullptr, s, out, sample);
     }
-    launches += dense > 1;
+    launches += 1;
   }
   if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "field_query_sorted: %s", cudaGetErrorString(e));
   count_launches(launches);
