@@ -272,17 +272,21 @@ __global__ void __launch_bounds__(256) k_tile_flags(StencilArgs a, int ntiles, u
 // b + 2B, ...; its threads test kRegThreads of them at once against the flags of the 3x3x3 tiles around each
 // (a tile's outputs need the vertices of its halo). A warp then takes every eighth tile that needs it: the
 // V_R windows of the halo's columns, a compact list of their active vertices, each vertex's terms evaluated
-// once (SDF through L1) and added to the tile's sums in ordered passes. Tiles of more than kWarpVerts vertices,
-// and all but the thinnest where a block has fewer tiles than warps, wait for the whole block, which keeps
-// the terms in slots and lets each output sum its neighbours' in a fixed order. An output gets one addition
-// a launch; per-cluster loss partials (fixed assignment and order) for k_reg_finalize. Bound by the chain of one
-// tile (loads, ~150 instructions a vertex, passes): V_R is a thin band of few, unevenly filled tiles. A warp
-// for every tile: 256^3 and 8,192 rays 55 us, 64^3 and 2,048 rays 33 us; a block for every tile 81 and 15 us;
-// so 39 and 12 us; 512^3 with every vertex active 5.03 and now 5.09 ms.
+// once (SDF through L1) and added to the tile's sums in ordered passes. A round of eight tiles lasts as long as its
+// most crowded one, so the most crowded may wait for the whole block, which keeps the terms in slots and lets each
+// output sum its neighbours' in a fixed order (round_limit). An output gets one addition a launch; per-cluster loss
+// partials (fixed assignment and order) for k_reg_finalize. Bound by the chain of one tile (loads, ~150 instructions
+// a vertex, passes): V_R is a thin band of few, unevenly filled tiles in a training step, and what a batch's samples
+// touch without a band.
 constexpr int kRegThreads = 256;
 constexpr int kRegWarps = kRegThreads / 32;
 constexpr int kHaloVerts = MX * MY * (TZ + 2);
-constexpr int kWarpVerts = 152;  // 48: 59 us, 96: 46, 144: 39 (256^3, 8,192 rays)
+// Costs of a tile of v vertices, in the same unit (~5 ns with every block busy): kWarpCost * v by a warp, kBlockCost + v
+// by the block. With 8 full tiles a round both ways are equal at kBlockCost = 1224; 1060, 1240, 1400, 1600:
+// 256^3 and 8,192 rays 38.2, 37.9, 37.4, 36.9 us; 64^3 and 2,048 rays 12.1, 12.2, 12.2, 13.1; 512^3 with every vertex
+// active 5.11, 4.27, 4.26, 4.26 ms. All tiles by warps, 55, 33 us and 5.00 ms; by the block from 152 vertices on 39, 12 us
+// and 5.06 ms, but 3.16 ms instead of 1.69 where 30% of 512^3 vertices are active anywhere.
+constexpr int kWarpCost = 16, kBlockCost = 1400;
 
 struct TileColumns {
   uint64_t win[MX * MY];  // bits of the columns' vertices z0 - 1 .. z0 + 32
@@ -317,7 +321,18 @@ __device__ __forceinline__ int tile_columns(const StencilArgs& a, const uint32_t
   return total;
 }
 
-// A tile of few vertices by one warp: 32 vertices at a time, their 7 terms added into the outputs' sums in 7
+// The most vertices that a tile of this round may have for a warp, v[w] being those of warp w's tile: the limit with the
+// smallest sum of the longest warp and of what is left to the block, one tile after the other. By one warp.
+__device__ __forceinline__ int round_limit(const int* v, int lane) {
+  const int limit = lane < kRegWarps ? v[lane] : 0;
+  int cost = kWarpCost * limit;
+#pragma unroll
+  for (int w = 0; w < kRegWarps; ++w) cost += v[w] > limit ? kBlockCost + v[w] : 0;
+  const int best = __reduce_min_sync(0xffffffffu, cost);
+  return __reduce_max_sync(0xffffffffu, cost == best ? limit : 0);
+}
+
+// A tile by one warp: 32 vertices at a time, their 7 terms added into the outputs' sums in 7
 // ordered passes (two vertices never share a target within a pass), then the sums to the gradient. acc
 // holds zeros.
 __device__ __forceinline__ void tile_by_warp(const StencilArgs& a, const StencilConsts& k, int x0, int y0, int z0,
@@ -420,13 +435,15 @@ __device__ __forceinline__ void tile_by_block(const StencilArgs& a, const Stenci
 
 __global__ void __launch_bounds__(kRegThreads, 4) k_reg_stencil(StencilArgs a, const uint8_t* __restrict__ flags,
                                                              double* __restrict__ partials, int ntiles) {
-  __shared__ float term[6 * kHaloVerts];  // the block's slots, or the warps' sums
-  __shared__ uint16_t list[kHaloVerts];
+  // the block's slots and their list, or the warps' sums and lists
+  constexpr int kSums = kRegWarps * TX * TY * TZ, kSlots = 6 * kHaloVerts;
+  __shared__ float term[kSums + kRegWarps * kHaloVerts / 2];
+  static_assert(kSlots + kHaloVerts / 2 <= kSums + kRegWarps * kHaloVerts / 2 && kHaloVerts % 2 == 0, "slots and list");
+  uint16_t* list = reinterpret_cast<uint16_t*>(term + kSlots);
   __shared__ TileColumns cols[kRegWarps];
-  __shared__ int queue[kRegThreads], dense[kRegWarps];  // tiles to do; vertices of a warp's left to the block, else 0
+  __shared__ int queue[kRegThreads], verts[kRegWarps];  // tiles to do; vertices of the warps' tiles
   __shared__ int qcount[kRegWarps];
   __shared__ double red[3][kRegWarps];
-  static_assert(kRegWarps * kWarpVerts <= kHaloVerts && kRegWarps * TX * TY * TZ <= 6 * kHaloVerts, "a warp's part");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool relax_on = a.relax_r > 0.0f && a.counts[1] > 0;
   const uint32_t* bm = a.fb + (relax_on ? a.nwords : 0);
@@ -469,33 +486,31 @@ __global__ void __launch_bounds__(kRegThreads, 4) k_reg_stencil(StencilArgs a, c
     }
     if (need) queue[at] = (int)tl;
     __syncthreads();
-    for (int n0 = 0; n0 < todo; n0 += kRegWarps) {  // a tile a warp, then the crowded ones of them
+    for (int n0 = 0; n0 < todo; n0 += kRegWarps) {  // a tile a warp, then the most crowded ones of them
       const int n = n0 + warp;
-      int total = 0;
+      int x0, y0, z0, total = 0;
       if (n < todo) {
-        int x0, y0, z0;
         tile_origin(a, queue[n], x0, y0, z0);
         total = tile_columns(a, bm, x0, y0, z0, cols[warp], lane);
-        if (total <= (todo < kRegWarps ? 32 : kWarpVerts)) {  // few tiles: all warps on each
-          if (total > 0) {
-            float* acc = term + TX * TY * TZ * warp;
-            for (int o = lane; o < TX * TY * TZ; o += 32) acc[o] = 0.0f;
-            __syncwarp();
-            tile_by_warp(a, k, x0, y0, z0, cols[warp], total, acc, list + kWarpVerts * warp, lane, loss);
-          }
-          total = 0;
-        }
       }
-      if (lane == 0) dense[warp] = total;
+      if (lane == 0) verts[warp] = total;
+      __syncthreads();
+      const int limit = round_limit(verts, lane);
+      if (total > 0 && total <= limit) {
+        float* acc = term + TX * TY * TZ * warp;
+        for (int o = lane; o < TX * TY * TZ; o += 32) acc[o] = 0.0f;
+        __syncwarp();
+        tile_by_warp(a, k, x0, y0, z0, cols[warp], total, acc,
+                     reinterpret_cast<uint16_t*>(term + kSums) + kHaloVerts * warp, lane, loss);
+      }
       __syncthreads();
 #pragma unroll 1
       for (int w = 0; w < kRegWarps; ++w) {
-        if (dense[w] == 0) continue;
-        int x0, y0, z0;
+        if (verts[w] <= limit) continue;
         tile_origin(a, queue[n0 + w], x0, y0, z0);
-        tile_by_block(a, k, x0, y0, z0, cols[w], dense[w], term, list, warp, lane, loss);
+        tile_by_block(a, k, x0, y0, z0, cols[w], verts[w], term, list, warp, lane, loss);
       }
-      __syncthreads();  // the columns and dense are read
+      __syncthreads();  // the columns and verts are read
     }
     __syncthreads();  // the queue is read
   }
