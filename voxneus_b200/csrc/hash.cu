@@ -260,8 +260,10 @@ int vx_hash_encode_backward(float* table_grad, int n_levels, int log2_size, int 
   a.P = n_points;
   a.d_out = d_out;
   a.ld_d = ld_d;
-  // Samples of rays share cells and take runs of 8 from 2^18 on; fewer need the threads (102,400: 13.8 us in runs
-  // of 4, 14.9 of 8), and a caller's own points share nothing (200,003: 74 and 77 us).
+  // Samples of rays share cells. With a training step's gradients, most of them 0, runs of 8 and of 4 cross near 2^18
+  // samples (80 and 128 a ray: 102,400 27.6 us in runs of 4, 29.7 of 8; 163,840 35.9, 36.9; 262,144 43.1, 43.0; 384,000
+  // 54.3, 52.3; 1,048,576 106.5, 99.3): longer runs send fewer atomics, shorter ones have the threads. A caller's own points
+  // share nothing (200,003: 74 and 77 us).
   const bool longer = !pts_norm && n_points >= (int64_t(1) << 18);
   const int run = longer ? 8 : 4;
   const dim3 threads(n_levels, 256 / n_levels);
