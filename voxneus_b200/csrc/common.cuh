@@ -163,7 +163,9 @@ __device__ __forceinline__ void gs_setup(const Grid& g, float px, float py, floa
 
 __device__ __forceinline__ float gs_sample(const float* __restrict__ f, const Grid& g, const Tri& t) {
   float acc = 0.0f;
-  if (t.inb == 0xffu) {  // all corners inside: fixed offsets from the lower one, no predicates
+  // all corners of all lanes inside: fixed offsets from the lower one, no predicates (lanes apart would take both ways:
+  // 1 M points around the box 13.7 -> 15.6 us)
+  if (__all_sync(__activemask(), t.inb == 0xffu)) {
     const float* p = f + lin3(g, t.x0, t.y0, t.z0);
     const int sx = g.ry * g.rz, sy = g.rz;
 #pragma unroll
