@@ -199,9 +199,10 @@ __device__ __forceinline__ bool relax_mode(const unsigned long long* counts, flo
   return relax_r > 0.0f && counts[1] > 0;
 }
 
-// Per-thread word chunk for compaction: one word a thread (four took 33 us where one takes 26, k_vr_write below).
-constexpr int kWordsPerThread = 1;
-constexpr int kCompactThreads = 1024;
+// Words of a thread in the compaction and threads of a block. 1 x 1024, 2 x 512, 4 x 256 words: 400^3 with 0.05% of the
+// vertices active 23.5, 16.4, 14.6 us, with 12% 81.8, 63.3, 60.3; 64^3 with all of them 66.9, 88.2, 172 us.
+constexpr int kWordsPerThread = 2;
+constexpr int kCompactThreads = 512;
 constexpr int64_t kWordsPerBlock = (int64_t)kWordsPerThread * kCompactThreads;
 
 // The chunk's words with only the final set's bits; returns how many.
@@ -250,9 +251,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* tmp, int& total) {
   }
   __syncthreads();
   total = tmp[32];
-  const int r = tmp[warp] + inc - v;
-  __syncthreads();
-  return r;
+  return tmp[warp] + inc - v;
 }
 
 __global__ void __launch_bounds__(kCompactThreads) k_vr_block_counts(VrArgs a, const unsigned long long* counts,
@@ -261,9 +260,12 @@ __global__ void __launch_bounds__(kCompactThreads) k_vr_block_counts(VrArgs a, c
   const bool relax_on = relax_mode(counts, a.relax_r);
   const int64_t w0 = blockIdx.x * kWordsPerBlock + (int64_t)threadIdx.x * kWordsPerThread;
   uint32_t fw[kWordsPerThread];
-  int total;
-  block_excl_scan(filter_chunk(a, w0, relax_on, fw), tmp, total);
-  if (threadIdx.x == 0) block_counts[blockIdx.x] = total;
+  const int lane = threadIdx.x & 31, mine = __reduce_add_sync(0xffffffffu, filter_chunk(a, w0, relax_on, fw));
+  if (lane == 0) tmp[threadIdx.x >> 5] = mine;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int total = __reduce_add_sync(0xffffffffu, lane < kCompactThreads / 32 ? tmp[lane] : 0);
+  if (lane == 0) block_counts[blockIdx.x] = total;
 }
 
 // Single-block exclusive scan of the block counts (in place).
@@ -282,9 +284,10 @@ __global__ void __launch_bounds__(1024) k_vr_scan(int* __restrict__ block_counts
 }
 
 // The block's vertices meet in shared memory, kListRound at a time, and leave as contiguous stores: written by
-// the threads that found them (24 bytes each, runs of a thread apart) 2 M vertices of a 256^3 grid took 65 us,
-// now 26 us; the output's bytes take 10 us.
+// the threads that found them (24 bytes each, runs of a thread apart) 2 M vertices of a 256^3 grid took 60 us,
+// now 22 us; the output's bytes take 10 us. A block of few has nothing to gain by that.
 constexpr int kListRound = 2048;
+constexpr int kFewVerts = 64;
 
 __global__ void __launch_bounds__(kCompactThreads) k_vr_write(VrArgs a, const unsigned long long* counts,
                                                                const int* __restrict__ block_offsets,
@@ -295,10 +298,29 @@ __global__ void __launch_bounds__(kCompactThreads) k_vr_write(VrArgs a, const un
   const bool relax_on = relax_mode(counts, a.relax_r);
   const int64_t w0 = blockIdx.x * kWordsPerBlock + (int64_t)threadIdx.x * kWordsPerThread;
   uint32_t fw[kWordsPerThread];
-  int total;
-  const int first = block_excl_scan(filter_chunk(a, w0, relax_on, fw), tmp, total);
+  const int mine = filter_chunk(a, w0, relax_on, fw);
   const int64_t pos = block_offsets[blockIdx.x];
+  if (blockIdx.x + 1 < gridDim.x && block_offsets[blockIdx.x + 1] == pos) return;
+  int total;
+  const int first = block_excl_scan(mine, tmp, total);
   if (pos + total > capacity) total = capacity > pos ? (int)(capacity - pos) : 0;
+  if (total <= kFewVerts) {  // straight from their threads
+    int p = first;
+#pragma unroll
+    for (int k = 0; k < kWordsPerThread; ++k) {
+      for (uint32_t bits = fw[k]; bits && p < total; bits &= bits - 1, ++p) {
+        const int idx = (int)((w0 + k) * 32 + (__ffs(bits) - 1));
+        if (linear) linear[pos + p] = idx;
+        if (!verts) continue;
+        int x, y, z;
+        vox_xyz(a.g, idx, x, y, z);
+        verts[3 * (pos + p)] = x;
+        verts[3 * (pos + p) + 1] = y;
+        verts[3 * (pos + p) + 2] = z;
+      }
+    }
+    return;
+  }
   for (int r0 = 0; r0 < total; r0 += kListRound) {
     const int cnt = min(total - r0, kListRound);
     int p = first - r0;
