@@ -12,28 +12,35 @@
 
 namespace vx {
 
-// A block takes 64 rows, four threads each: thread group g encodes levels [g * lpt, (g + 1) * lpt), builds
-// the SH values 4g .. 4g+3 and group 1 copies the normal; the rows meet in shared memory and leave with
+// A block takes 256 / kGroups rows, kGroups threads each: thread group g encodes levels [g * lpt, (g + 1) * lpt), builds
+// its share of the four SH quarters and one group copies the normal; the rows meet in shared memory and leave with
 // consecutive lanes on consecutive columns. Bound by the table's sector requests (L1 to L2). 200,003 points,
 // 11 of 16 levels open, with the SH of as many directions: 111 us with a thread a row (4-byte stores a row
-// apart, levels one after the other), 70 us so.
-constexpr int kAppRows = 64;
-
+// apart, levels one after the other), 70 us with four. Four threads need levels to share: app_groups.
 __host__ __device__ inline int app_columns(const HashArgs& a) {
   return (a.table ? 2 * a.L : 0) + (a.sh_col >= 0 ? 16 : 0) + (a.nrm_col >= 0 ? 3 : 0) + (a.pad_col >= 0 ? 1 : 0);
 }
 
+// Threads a row. One thread writes its row itself, which pays up to two levels: 300,000 points of one level 13.9 us by four
+// threads, 6.5 by one, of two levels 17.1 and 11.1, of three 26.0 and 25.0; 15,000 points of three 4.5 and 5.4.
+inline int app_groups(const HashArgs& a) { return a.table && a.L <= 2 ? 1 : 4; }
+
+template <int kGroups>
 __global__ void __launch_bounds__(256) k_appearance_fwd(HashArgs a) {
+  constexpr int kAppRows = 256 / kGroups, kWarps = 8 / kGroups;  // rows of a block, warps of a group
   extern __shared__ float srow[];  // [kAppRows][pitch]
   const uint32_t mask = (1u << a.log2T) - 1u;
   const size_t T = (size_t)1 << a.log2T;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = w >> 1;
-  const int ls = 32 * (w & 1) + lane;  // this thread's row in the block
-  const int ncol = app_columns(a), pitch = ncol | 1, lpt = (a.L + 3) >> 2;
-  const int sh0 = a.table ? 2 * a.L : 0, nrm0 = sh0 + (a.sh_col >= 0 ? 16 : 0), pad0 = nrm0 + (a.nrm_col >= 0 ? 3 : 0);
-  float* mine = srow + ls * pitch;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = w / kWarps;
+  const int ls = 32 * (w % kWarps) + lane;  // this thread's row in the block
+  const int ncol = app_columns(a), pitch = ncol | 1, lpt = (a.L + kGroups - 1) / kGroups;
+  constexpr bool kDirect = kGroups == 1;  // a thread's row goes straight to its columns
+  const int sh0 = kDirect ? a.sh_col : a.table ? 2 * a.L : 0, nrm0 = kDirect ? a.nrm_col : sh0 + (a.sh_col >= 0 ? 16 : 0);
+  const int pad0 = kDirect ? a.pad_col : nrm0 + (a.nrm_col >= 0 ? 3 : 0);
+  const int width = ncol >= 32 ? 32 : 1 << (32 - __clz(max(ncol - 1, 1)));  // lanes of a row on the way out
   for (int64_t base = (int64_t)blockIdx.x * kAppRows; base < a.P; base += (int64_t)gridDim.x * kAppRows) {
     const int64_t i = base + ls;
+    float* mine = kDirect ? a.out + i * a.ld : srow + ls * pitch;
     if (i < a.P) {
       if (a.table) {
         float x[3];
@@ -70,7 +77,7 @@ __global__ void __launch_bounds__(256) k_appearance_fwd(HashArgs a) {
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          if (g != k) continue;
+          if (k % kGroups != g) continue;
           const float4 v = sh_chunk(dx, dy, dz, k);
           mine[sh0 + 4 * k] = v.x;
           mine[sh0 + 4 * k + 1] = v.y;
@@ -78,16 +85,17 @@ __global__ void __launch_bounds__(256) k_appearance_fwd(HashArgs a) {
           mine[sh0 + 4 * k + 3] = v.w;
         }
       }
-      if (a.nrm_col >= 0 && g == 1) {
+      if (a.nrm_col >= 0 && g == 1 % kGroups) {
         mine[nrm0] = a.normals[3 * i];
         mine[nrm0 + 1] = a.normals[3 * i + 1];
         mine[nrm0 + 2] = a.normals[3 * i + 2];
       }
-      if (a.pad_col >= 0 && g == 2) mine[pad0] = 0.0f;
+      if (a.pad_col >= 0 && g == 2 % kGroups) mine[pad0] = 0.0f;
     }
+    if (kDirect) continue;
     __syncthreads();
     const int nrows = (int)(a.P - base < kAppRows ? a.P - base : kAppRows);
-    for (int c = lane; c < ncol; c += 32) {
+    for (int c = lane & (width - 1); c < ncol; c += width) {
       int to = c;  // the value's column; of parts laid over one another the last stays
       bool gone = false;
       const bool pad = a.pad_col >= 0, nrm = a.nrm_col >= 0, sh = a.sh_col >= 0;
@@ -102,7 +110,7 @@ __global__ void __launch_bounds__(256) k_appearance_fwd(HashArgs a) {
                (c < sh0 && sh && to >= a.sh_col && to < a.sh_col + 16);
       }
       if (!gone)
-        for (int r = w; r < nrows; r += 8) a.out[(base + r) * a.ld + to] = srow[r * pitch + c];
+        for (int r = (32 * w + lane) / width; r < nrows; r += 256 / width) a.out[(base + r) * a.ld + to] = srow[r * pitch + c];
     }
     __syncthreads();
   }
@@ -236,8 +244,13 @@ int vx_appearance_forward(const float* table, int n_levels, int log2_size, int n
   a.nrm_col = normal_col;
   a.normals = normals;
   a.pad_col = pad_col;
-  const size_t smem = (size_t)kAppRows * (app_columns(a) | 1) * sizeof(float);  // at most 21 KB
-  k_appearance_fwd<<<grid_for((n_points + kAppRows - 1) / kAppRows * 256, 256, 32), 256, smem, (cudaStream_t)stream>>>(a);
+  const int rows = 256 / app_groups(a);  // of a block
+  const size_t smem = rows == 256 ? 0 : (size_t)rows * (app_columns(a) | 1) * sizeof(float);  // at most 22 KB
+  const unsigned blocks = grid_for((n_points + rows - 1) / rows * 256, 256, 32);
+  if (app_groups(a) == 1)
+    k_appearance_fwd<1><<<blocks, 256, smem, (cudaStream_t)stream>>>(a);
+  else
+    k_appearance_fwd<4><<<blocks, 256, smem, (cudaStream_t)stream>>>(a);
   count_launches(1);
   return check_launch("appearance_forward");
 }
