@@ -164,6 +164,25 @@ __global__ void __launch_bounds__(256) k_hash_bwd(HashArgs a) {
     }
     int cx = -1, cy = 0, cz = 0;
     float2 acc[8];
+    if constexpr (kRun == 1) {  // the position's loads beside the gradient's, no loop
+      float x[3];
+      sample_pos(a, i0, x);
+      if (g[0].x == 0.0f && g[0].y == 0.0f) continue;
+      const float g0 = lw < 1.0f ? g[0].x * lw : g[0].x, g1 = lw < 1.0f ? g[0].y * lw : g[0].y;
+      const float sx = x[0] * fr, sy = x[1] * fr, sz = x[2] * fr;
+      cx = (int)floorf(sx);
+      cy = (int)floorf(sy);
+      cz = (int)floorf(sz);
+      const float dx = sx - (float)cx, dy = sy - (float)cy, dz = sz - (float)cz;
+      const float ox = 1.0f - dx, oy = 1.0f - dy, oz = 1.0f - dz;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float w = ((k & 4) ? dx : ox) * ((k & 2) ? dy : oy) * ((k & 1) ? dz : oz);
+        acc[k] = make_float2(w * g0, w * g1);
+      }
+      flush_cell(tab, cx, cy, cz, mask, acc);
+      continue;
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
@@ -273,18 +292,17 @@ int vx_hash_encode_backward(float* table_grad, int n_levels, int log2_size, int 
   a.P = n_points;
   a.d_out = d_out;
   a.ld_d = ld_d;
-  // Samples of rays share cells. With a training step's gradients, most of them 0, runs of 8 and of 4 cross near 2^18
-  // samples (80 and 128 a ray: 102,400 27.6 us in runs of 4, 29.7 of 8; 163,840 35.9, 36.9; 262,144 43.1, 43.0; 384,000
-  // 54.3, 52.3; 1,048,576 106.5, 99.3): longer runs send fewer atomics, shorter ones have the threads. A caller's own points
-  // share nothing (200,003: 74 and 77 us).
-  const bool longer = !pts_norm && n_points >= (int64_t(1) << 18);
-  const int run = longer ? 8 : 4;
+  // Consecutive samples of a ray share cells; a caller's own points and rays of few samples hardly do and take one sample
+  // a thread (100,000 points of 4 levels 18.6 us in runs of 1, 20.2 of 2, 21.1 of 4; 300,000 of 16 levels 153 us all
+  // three). Few samples of rays need the threads too: below 2^17 samples x levels (6,400 samples, 8 levels 4.8, 4.8, 6.6 us;
+  // 16 levels 7.3, 7.1, 6.9). With a training step's gradients, most of them 0, runs of 8 and of 4 cross near 2^18 samples
+  // (80 and 128 a ray: 102,400 27.6 us in runs of 4, 29.7 of 8; 163,840 35.9, 36.9; 262,144 43.1, 43.0; 384,000 54.3, 52.3;
+  // 1,048,576 106.5, 99.3).
+  const bool shared = !pts_norm && n_samples >= 8 && n_points * n_levels >= (int64_t(1) << 17);
+  const int run = !shared ? 1 : n_points < (int64_t(1) << 18) ? 4 : 8;
+  auto kern = run == 1 ? k_hash_bwd<1> : run == 4 ? k_hash_bwd<4> : k_hash_bwd<8>;
   const dim3 threads(n_levels, 256 / n_levels);
-  const unsigned blocks = grid_for((n_points + run - 1) / run, (int)threads.y, 32);
-  if (longer)
-    k_hash_bwd<8><<<blocks, threads, 0, (cudaStream_t)stream>>>(a);
-  else
-    k_hash_bwd<4><<<blocks, threads, 0, (cudaStream_t)stream>>>(a);
+  kern<<<grid_for((n_points + run - 1) / run, (int)threads.y, 32), threads, 0, (cudaStream_t)stream>>>(a);
   count_launches(1);
   return check_launch("hash_encode_backward");
 }
