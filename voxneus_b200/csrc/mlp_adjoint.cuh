@@ -145,11 +145,9 @@ constexpr int kAdjShTid = 5;  // the worker that evaluates SH(d) of a tile's ray
 // instructions of a converged warp: __syncwarp() first wherever lanes can have parted before (polls that
 // end at different times, a branch of some lanes), because nothing else makes them meet again.
 __device__ __forceinline__ void adj_staged_arrive() {
-  __syncwarp();
   asm volatile("bar.arrive 1, %0;" ::"n"(kAdjThreads) : "memory");
 }
 __device__ __forceinline__ void adj_staged_sync() {
-  __syncwarp();
   asm volatile("bar.sync 1, %0;" ::"n"(kAdjThreads) : "memory");
 }
 __device__ __forceinline__ void adj_workers_sync() {
@@ -444,7 +442,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
     for (int64_t t = t0; t < ntiles; t += tstep, ++it) {
       const int par = it & 1;
       adj_staged_sync();  // A of this tile is staged, its rows are read
-      if (__shfl_sync(0xffffffffu, (int)*s_fail, 0) == 0) {
+      if (!__any_sync(0xffffffffu, *s_fail)) {
         issue_g(par);
         if (S::kBulk && t + S::kBufs * tstep < ntiles) fetch_rows(t + S::kBufs * tstep, S::kBufs == 2 ? par : 0);
       }
@@ -539,6 +537,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
       // end of the tile; until then the block goes on with whatever the memory holds, but issues nothing.
       if (it > 0) ok = tc::mbar_wait(bar_g, par ^ 1, wait_limit) && ok;
       if (S::kBulk && !kFold) ok = tc::mbar_wait(bar_rows, par, wait_limit) && ok;
+      if (!ok) *s_fail = 1;
       __syncwarp();
       tc::fence_after_sync();
       // 2: the rows of A
@@ -602,9 +601,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           }
         }
       }
-      if (!ok) *s_fail = 1;
       tc::fence_smem_to_async();
       tc::fence_before_sync();
+      if (!kFold) __syncwarp();
       adj_staged_arrive();
       // 3: G of this tile runs; G of the previous tile and dX of this one are read out (their loads in
       // flight together), the next tile's mask is staged
@@ -649,7 +648,6 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         }
       }
       if constexpr (kFold) {  // the four warps of 32 samples: their rows leave in whole lines
-        __syncwarp();
         asm volatile("bar.sync %0, 128;" ::"r"(4 + q) : "memory");
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
