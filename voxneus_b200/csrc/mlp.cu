@@ -151,46 +151,6 @@ __device__ void stage_weights(const MlpW& w, uint8_t* W2, uint8_t* XH, uint8_t* 
   if (tid < NO) B1[tid] = w.b1[tid];
 }
 
-// Row chunks of sample m of the tile at m0 into registers: thread (m, hh) takes the 16-byte
-// chunks 0..6 (hh = 0) or 7..12 (hh = 1, v[6] unused). Rows past P read as 0.
-__device__ __forceinline__ void load_row_chunks(const float* __restrict__ X, int64_t ldx, bool vec, int64_t P,
-                                                int64_t m0, int m, int hh, float4 v[7]) {
-  const bool ok = m0 + m < P;
-  const float* row = X + (m0 + m) * ldx;
-  const int c0 = hh ? 7 : 0;
-#pragma unroll
-  for (int j = 0; j < 7; ++j) {
-    const int c = c0 + j;
-    v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (ok && c < 13) {
-      if (vec) {
-        v[j] = __ldg(reinterpret_cast<const float4*>(row) + c);
-      } else {
-        v[j].x = __ldg(row + 4 * c);
-        v[j].y = __ldg(row + 4 * c + 1);
-        v[j].z = __ldg(row + 4 * c + 2);
-        v[j].w = 4 * c + 3 < KIN ? __ldg(row + 4 * c + 3) : 0.0f;
-      }
-    }
-  }
-}
-
-// The chunks of load_row_chunks into the X buffers (hi/lo tf32); column 51 becomes `one` on
-// real rows.
-__device__ __forceinline__ void store_row_chunks(const float4 v[7], bool valid, uint8_t* XH, uint8_t* XL, int m,
-                                                 int hh, float one) {
-  const int c0 = hh ? 7 : 0;
-#pragma unroll
-  for (int j = 0; j < 7; ++j) {
-    const int c = c0 + j;
-    if (c < 13) {
-      float4 u = v[j];
-      if (c == 12 && valid) u.w = one;
-      st_split4(XH, XL, x_off(c, m), u.x, u.y, u.z, u.w);
-    }
-  }
-}
-
 constexpr uint32_t kId128 = tc::idesc_tf32(TM, 2 * NH, false, false);
 constexpr uint32_t kId64 = tc::idesc_tf32(TM, NH, false, false);
 
@@ -222,7 +182,7 @@ __device__ __forceinline__ void tmem_ld_sum32(uint32_t taddr, float v[32]) {
   for (int j = 0; j < 32; ++j) v[j] += u[j];
 }
 
-// Where a forward's outputs go: colours (row stride ldc) and, when mask is given, each sample's ReLU
+// Where a forward's outputs go: colours (row stride ldc; may be null when mask is given) and, when mask is given, each sample's ReLU
 // mask (bit j of word k: hidden unit 32 k + j is active; two words a sample, row stride ldm).
 struct MlpOut {
   float* colors;
@@ -259,13 +219,24 @@ __device__ __forceinline__ uint32_t colour_partial(const float z[32], int hh, co
   return bits;
 }
 
-// Forward. kHashIn: the 51 features of a tile are built in place (two threads per sample, 8 hash
-// levels each; SH of the view direction; the normal); else they are read from rows X. kRowsOut
-// also writes the rows for the adjoint. 256 threads: warp w reads TMEM lanes 32*(w%4).. and
-// hidden columns 32*(w/4)..; the two column halves meet in shared memory.
-template <bool kHashIn, bool kRowsOut, bool kMask, bool kCustomWait>
-__global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* __restrict__ X, int64_t ldx, int xvec,
-                                                       int64_t P, MlpW w, MlpOut out, TcGuard g) {
+// The ReLU bits alone, of the same pre-activations.
+__device__ __forceinline__ uint32_t relu_bits(const float z[32], int hh, const float* B0) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j4 = 0; j4 < 8; ++j4) {
+    const float4 b = *reinterpret_cast<const float4*>(B0 + 32 * hh + 4 * j4);
+    const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bits |= (z[4 * j4 + i] + bb[i] > 0.0f ? 1u : 0u) << (4 * j4 + i);
+  }
+  return bits;
+}
+
+// Forward with the 51 features of a tile built in place: two threads per sample, 8 hash levels each; SH of the view
+// direction; the normal. 256 threads: warp w reads TMEM lanes 32*(w%4).. and hidden columns 32*(w/4)..; the two
+// column halves meet in shared memory.
+template <bool kCustomWait>
+__global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, int64_t P, MlpW w, MlpOut out, TcGuard g) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t wait_limit = kCustomWait ? g.limit : kWaitLimit;  // a constant bound unless a caller set one
   uint8_t* XH = smem;
@@ -290,74 +261,54 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
   const size_t T = (size_t)1 << a.log2T;
   uint32_t phase = 0;
   const int64_t ntiles = (P + TM - 1) / TM;
-  float4 pre[7];
-  if (!kHashIn && (int64_t)blockIdx.x < ntiles)
-    load_row_chunks(X, ldx, xvec != 0, P, (int64_t)blockIdx.x * TM, tid & (TM - 1), tid >> 7, pre);
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int64_t m0 = t * TM;
-    if (kHashIn) {
-      const int m = tid & (TM - 1), half = tid >> 7;
-      const int64_t i = m0 + m;
-      float feat[16], extra[16];
-      if (i < P) {
-        float x[3];
-        sample_pos(a, i, x);
+    const int m = tid & (TM - 1), half = tid >> 7;
+    const int64_t i = m0 + m;
+    float feat[16], extra[16];
+    if (i < P) {
+      float x[3];
+      sample_pos(a, i, x);
 #pragma unroll
-        for (int qq = 0; qq < 8; ++qq) {
-          const int l = 8 * half + qq;
-          const float lw = a.lw[l];
-          float f0 = 0.0f, f1 = 0.0f;
-          if (lw != 0.0f) {
-            LevelCell c;
-            level_cell(x, a.res[l], mask, c);
-            const float2* tab = reinterpret_cast<const float2*>(a.table) + (size_t)l * T;
-            gather_level(tab, c, f0, f1);
-            if (lw < 1.0f) {
-              f0 *= lw;
-              f1 *= lw;
-            }
+      for (int qq = 0; qq < 8; ++qq) {
+        const int l = 8 * half + qq;
+        const float lw = a.lw[l];
+        float f0 = 0.0f, f1 = 0.0f;
+        if (lw != 0.0f) {
+          LevelCell c;
+          level_cell(x, a.res[l], mask, c);
+          const float2* tab = reinterpret_cast<const float2*>(a.table) + (size_t)l * T;
+          gather_level(tab, c, f0, f1);
+          if (lw < 1.0f) {
+            f0 *= lw;
+            f1 *= lw;
           }
-          feat[2 * qq] = f0;
-          feat[2 * qq + 1] = f1;
         }
-        if (half == 0) {
-          const int64_t r = i / a.S;
-          sh16(__ldg(a.rays_d + 3 * r), __ldg(a.rays_d + 3 * r + 1), __ldg(a.rays_d + 3 * r + 2), extra);
-        } else {
-          extra[0] = a.normals[3 * i];
-          extra[1] = a.normals[3 * i + 1];
-          extra[2] = a.normals[3 * i + 2];
-          extra[3] = 0.0f;
-        }
-      } else {
-#pragma unroll
-        for (int qq = 0; qq < 16; ++qq) feat[qq] = extra[qq] = 0.0f;
+        feat[2 * qq] = f0;
+        feat[2 * qq + 1] = f1;
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        st_split4(XH, XL, x_off(4 * half + c, m), feat[4 * c], feat[4 * c + 1], feat[4 * c + 2], feat[4 * c + 3]);
       if (half == 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          st_split4(XH, XL, x_off(8 + c, m), extra[4 * c], extra[4 * c + 1], extra[4 * c + 2], extra[4 * c + 3]);
+        const int64_t r = i / a.S;
+        sh16(__ldg(a.rays_d + 3 * r), __ldg(a.rays_d + 3 * r + 1), __ldg(a.rays_d + 3 * r + 2), extra);
       } else {
-        st_split4(XH, XL, x_off(12, m), extra[0], extra[1], extra[2], extra[3]);
-      }
-      if (kRowsOut && i < P) {
-        float4* row = reinterpret_cast<float4*>(a.out + i * a.ld);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          row[4 * half + c] = make_float4(feat[4 * c], feat[4 * c + 1], feat[4 * c + 2], feat[4 * c + 3]);
-        if (half == 0) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            row[8 + c] = make_float4(extra[4 * c], extra[4 * c + 1], extra[4 * c + 2], extra[4 * c + 3]);
-        } else {
-          row[12] = make_float4(extra[0], extra[1], extra[2], extra[3]);
-        }
+        extra[0] = a.normals[3 * i];
+        extra[1] = a.normals[3 * i + 1];
+        extra[2] = a.normals[3 * i + 2];
+        extra[3] = 0.0f;
       }
     } else {
-      store_row_chunks(pre, m0 + (tid & (TM - 1)) < P, XH, XL, tid & (TM - 1), tid >> 7, 0.0f);
+#pragma unroll
+      for (int qq = 0; qq < 16; ++qq) feat[qq] = extra[qq] = 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      st_split4(XH, XL, x_off(4 * half + c, m), feat[4 * c], feat[4 * c + 1], feat[4 * c + 2], feat[4 * c + 3]);
+    if (half == 0) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        st_split4(XH, XL, x_off(8 + c, m), extra[4 * c], extra[4 * c + 1], extra[4 * c + 2], extra[4 * c + 3]);
+    } else {
+      st_split4(XH, XL, x_off(12, m), extra[0], extra[1], extra[2], extra[3]);
     }
     tc::fence_smem_to_async();
     __syncthreads();
@@ -366,8 +317,6 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
       issue_z(tbase, xh, xl, w2);
       tc::commit(bar);
     }
-    if (!kHashIn && t + gridDim.x < ntiles)  // next tile's rows fly during the MMA and the epilogue
-      load_row_chunks(X, ldx, xvec != 0, P, (t + gridDim.x) * TM, tid & (TM - 1), tid >> 7, pre);
     const bool ok = tc::mbar_wait(bar, phase, wait_limit);
     phase ^= 1u;
     if (__syncthreads_or(!ok)) {
@@ -381,8 +330,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
     float z[32];
     tmem_ld_sum32(tbase + ((uint32_t)(32 * q) << 16) + 32 * hh, z);
     float p0, p1, p2;
-    const uint32_t bits = colour_partial<kMask>(z, hh, B0, W1s, p0, p1, p2);
-    if (kMask && m0 + 32 * q + lane < P) out.mask[(m0 + 32 * q + lane) * out.ldm + hh] = bits;
+    colour_partial<false>(z, hh, B0, W1s, p0, p1, p2);
     float* r = RED + (hh * TM + 32 * q + lane) * 4;
     r[0] = p0;
     r[1] = p1;
@@ -404,7 +352,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_fwd_tc(HashArgs a, const float* 
 
 constexpr size_t kFwdSmem = 2 * kXBytes + kWBytes + sizeof(float) * (NH + NO * NH + 4 + 2 * TM * 4) + 16;
 
-// Forward on contiguous rows (52 floats, or compact): one CTA per SM holding two independent tile slots
+// Forward on rows (52 floats, compact, or any stride from 51 on): one CTA per SM holding two independent tile slots
 // of 256 worker threads, which share the stacked weights and the tensor core, and one issuing warp a slot
 // (16 + slot), which issues the slot's MMAs and row copies (issuing blocks while the tensor core's queue
 // is full; warp-issued, tc.cuh). A slot has two X operands (the lo part in shared memory, the hi part in
@@ -442,6 +390,10 @@ static_assert(FwdShape<true, true>::kOffRed % 16 == 0 && FwdShape<true, true>::k
               "shared-memory alignment");
 constexpr int kFwdThreads = 512 + 64;
 
+// The rows of a forward: compact and folded, compact, contiguous 52 floats, any other stride. The last are brought in
+// element by element by the lanes of the issuing warp (16 bytes at a time where the rows are aligned).
+enum FwdRows { kFwdFold = 0, kFwdCompact = 1, kFwdFull = 2, kFwdStrided = 3 };
+
 // A barrier of a slot's workers that also agrees on whether any of them gave up a wait. Like the tensor-memory loads
 // and stores it is an instruction of a converged warp: __syncwarp() first wherever lanes can have parted.
 __device__ __forceinline__ bool slot_sync_or(int slot, bool v) {
@@ -455,10 +407,12 @@ __device__ __forceinline__ bool slot_sync_or(int slot, bool v) {
   return r != 0;
 }
 
-template <bool kCustomWait, bool kCompact, bool kFold, bool kMask>
+template <bool kCustomWait, FwdRows kRows, bool kMask>
 __global__ void __launch_bounds__(kFwdThreads, 1)
-    k_mlp_fwd_rows2(const float* __restrict__ X, int64_t P, MlpW w, MlpOut out, TcGuard g, RowSrc src) {
-  static_assert(!kFold || kCompact, "the folded MLP reads compact rows");
+    k_mlp_fwd_rows2(const float* __restrict__ X, int64_t ldx, int xvec, int64_t P, MlpW w, MlpOut out, TcGuard g,
+                    RowSrc src) {
+  constexpr bool kFold = kRows == kFwdFold, kCompact = kRows == kFwdFold || kRows == kFwdCompact;
+  constexpr bool kStrided = kRows == kFwdStrided;
   using S = FwdShape<kCompact, kFold>;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t wait_limit = kCustomWait ? g.limit : kWaitLimit;
@@ -499,7 +453,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   if (issuer && lane == 0) {
     tc::mbar_init(bar, 1);
     tc::mbar_init(ready, 8);
-    tc::mbar_init(bar_rows, 1);
+    tc::mbar_init(bar_rows, kStrided ? 256 : 1);
     tc::mbar_init(bar_rows + 1, 1);
     s_fail[slot] = 0;
   }
@@ -530,7 +484,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     };
 #pragma unroll
     for (int b = 0; b < S::kBufs; ++b)
-      if (t0 + b * tstride < ntiles) fetch_rows(t0 + b * tstride, b);
+      if (!kStrided && t0 + b * tstride < ntiles) fetch_rows(t0 + b * tstride, b);
     int it = 0;
     bool bad = false;
     for (int64_t t = t0; t < ntiles; t += tstride, ++it) {
@@ -553,7 +507,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       tc::commit_warp(lead, bar);
       ++n_mma;
       const int64_t tn = t + S::kBufs * tstride;  // the tile's rows have been read
-      if (tn < ntiles) fetch_rows(tn, S::kBufs == 2 ? it & 1 : 0);
+      if (!kStrided && tn < ntiles) fetch_rows(tn, S::kBufs == 2 ? it & 1 : 0);
     }
     if (bad && lane == 0) s_fail[slot] = 1;
     // the workers leave on their own or see the flag; then nothing of this slot may still be in flight
@@ -577,6 +531,37 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       }
     };
     bool ok = true;  // no wait of this thread has given up
+    auto load_rows = [&](int64_t t) {  // kStrided: this thread's part of tile t's rows
+      const float* from = X + t * TM * ldx;
+      const int nrows = (int)(P - t * TM < TM ? P - t * TM : TM);
+      if (xvec) {  // 12 chunks of 16 bytes and three columns (the row may end there)
+        constexpr int kCh = KP / 4;
+        for (int e = stid; e < nrows * kCh; e += 256) {
+          const int r = e / kCh, c = 4 * (e - r * kCh);
+          const uint32_t to = tc::smem_u32(ROWS) + (r * KP + c) * 4;
+          const float* p = from + r * ldx + c;
+          if (c < 48) {
+            tc::async16(to, p);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) tc::async4(to + 4 * k, p + k);
+          }
+        }
+      } else {
+        int r = stid / KIN, k = stid - r * KIN;
+#pragma unroll 4
+        for (; r < nrows;) {
+          tc::async4(tc::smem_u32(ROWS) + (r * KP + k) * 4, from + r * ldx + k);
+          k += 256 % KIN;
+          r += 256 / KIN;
+          if (k >= KIN) {
+            k -= KIN;
+            ++r;
+          }
+        }
+      }
+      tc::async_arrive(bar_rows);
+    };
     auto stage = [&](int64_t t, int i) {  // tile t, number i of this slot: rows -> X_hi / X_lo
       const int buf = i & 1;
       const bool valid = t * TM + m < P;
@@ -646,9 +631,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     };
     if (t0 < ntiles) {
       load_dir(t0);
+      if (kStrided) load_rows(t0);
       stage(t0, 0);
       tell();
-      slot_sync_or(slot, false);  // the first tile's bias
+      slot_sync_or(slot, false);  // the first tile's bias is written, its rows are read
+      if (kStrided && t0 + tstride < ntiles) load_rows(t0 + tstride);
     }
     int it = 0;
     for (int64_t t = t0; t < ntiles; t += tstride, ++it) {
@@ -662,16 +649,24 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
       float z[32];
       tmem_ld_sum32(tcol + lane_base + 32 * hh, z);
       if (more) tell();
-      float p0, p1, p2;
-      const uint32_t bits = colour_partial<kMask>(z, hh, kFold ? BETA + NH * par : B0, W1s, p0, p1, p2);
-      if (kMask && valid) out.mask[(m0 + m) * out.ldm + hh] = bits;
+      const float* b0 = kFold ? BETA + NH * par : B0;
+      const bool colours = !kMask || out.colors;
       float* red = RED + par * (2 * TM * 4);
-      *reinterpret_cast<float4*>(red + (hh * TM + m) * 4) = make_float4(p0, p1, p2, 0.0f);
+      uint32_t bits;
+      if (colours) {
+        float p0, p1, p2;
+        bits = colour_partial<kMask>(z, hh, b0, W1s, p0, p1, p2);
+        *reinterpret_cast<float4*>(red + (hh * TM + m) * 4) = make_float4(p0, p1, p2, 0.0f);
+      } else {
+        bits = relu_bits(z, hh, b0);
+      }
+      if (kMask && valid) out.mask[(m0 + m) * out.ldm + hh] = bits;
       if (slot_sync_or(slot, !ok)) {
         if (stid == 0) s_fail[slot] = 1;
         break;
       }
-      if (valid) {  // hh = 0: colours 0 and 1, hh = 1: colour 2
+      if (kStrided && t + 2 * tstride < ntiles) load_rows(t + 2 * tstride);  // the next tile's have been read
+      if (valid && colours) {  // hh = 0: colours 0 and 1, hh = 1: colour 2
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int cc = 2 * hh + c;
@@ -682,6 +677,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         }
       }
     }
+    if (kStrided) tc::async_wait_all();
     tc::fence_before_sync();
     __syncthreads();
   }
@@ -833,42 +829,43 @@ __global__ void __launch_bounds__(256) k_radiance_rows(const float* __restrict__
   }
 }
 
-template <bool kMask>
-auto rows2_kernel(bool fold, bool compact, bool cw) {
-  return fold      ? (cw ? k_mlp_fwd_rows2<true, true, true, kMask> : k_mlp_fwd_rows2<false, true, true, kMask>)
-         : compact ? (cw ? k_mlp_fwd_rows2<true, true, false, kMask> : k_mlp_fwd_rows2<false, true, false, kMask>)
-                   : (cw ? k_mlp_fwd_rows2<true, false, false, kMask> : k_mlp_fwd_rows2<false, false, false, kMask>);
+template <bool kCustomWait, bool kMask>
+auto rows2_kernel(FwdRows rows) {
+  return rows == kFwdFold      ? k_mlp_fwd_rows2<kCustomWait, kFwdFold, kMask>
+         : rows == kFwdCompact ? k_mlp_fwd_rows2<kCustomWait, kFwdCompact, kMask>
+         : rows == kFwdFull    ? k_mlp_fwd_rows2<kCustomWait, kFwdFull, kMask>
+                               : k_mlp_fwd_rows2<kCustomWait, kFwdStrided, kMask>;
 }
 
-template <bool kHashIn, bool kRowsOut>
-int launch_fwd(const HashArgs& a, const float* X, int64_t ldx, int64_t P, const MlpW& w, const MlpOut& out,
-               cudaStream_t st, RowSrc src = RowSrc{nullptr, 0}) {
-  const int64_t tiles = (P + TM - 1) / TM;
-  const bool compact = src.rays_d != nullptr;
+// The forward on rows X (row stride ldx, or compact rows when src.rays_d is given).
+int launch_fwd(const float* X, int64_t ldx, int64_t P, const MlpW& w, const MlpOut& out, cudaStream_t st,
+               RowSrc src = RowSrc{nullptr, 0}) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  // folded: compact rows whose tiles each lie inside one ray (samples per ray a multiple of the tile)
+  const FwdRows rows = src.rays_d ? (src.S % TM == 0 ? kFwdFold : kFwdCompact)
+                                  : (ldx == KP && aligned ? kFwdFull : kFwdStrided);
   const bool cw = custom_wait();
-  if (!kHashIn && (compact || ldx == KP) && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {  // contiguous rows: two slots
-    // compact rows whose tiles each lie inside one ray (samples per ray a multiple of the tile):
-    // the folded MLP
-    const bool fold = compact && src.S % TM == 0;
-    auto kern2 = out.mask ? rows2_kernel<true>(fold, compact, cw) : rows2_kernel<false>(fold, compact, cw);
-    const int smem = fold      ? (int)FwdShape<true, true>::kSmem
-                     : compact ? (int)FwdShape<true, false>::kSmem
-                               : (int)FwdShape<false, false>::kSmem;
-    cudaError_t e = cudaFuncSetAttribute(kern2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
-    const int64_t pairs = (tiles + 1) / 2;
-    const unsigned blocks = (unsigned)(pairs < (int64_t)kSMs ? pairs : (int64_t)kSMs);
-    kern2<<<blocks, kFwdThreads, smem, st>>>(X, P, w, out, t_guard, src);
-    return VX_OK;
-  }
-  auto kern = cw ? k_mlp_fwd_tc<kHashIn, kRowsOut, false, true> : k_mlp_fwd_tc<kHashIn, kRowsOut, false, false>;
-  if constexpr (!kHashIn)
-    if (out.mask) kern = cw ? k_mlp_fwd_tc<false, false, true, true> : k_mlp_fwd_tc<false, false, true, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
+  auto kern = out.mask ? (cw ? rows2_kernel<true, true>(rows) : rows2_kernel<false, true>(rows))
+                       : (cw ? rows2_kernel<true, false>(rows) : rows2_kernel<false, false>(rows));
+  const int smem = rows == kFwdFold      ? (int)FwdShape<true, true>::kSmem
+                   : rows == kFwdCompact ? (int)FwdShape<true, false>::kSmem
+                                         : (int)FwdShape<false, false>::kSmem;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
+  const int64_t pairs = ((P + TM - 1) / TM + 1) / 2;
+  const unsigned blocks = (unsigned)(pairs < (int64_t)kSMs ? pairs : (int64_t)kSMs);
+  kern<<<blocks, kFwdThreads, smem, st>>>(X, ldx, ldx % 4 == 0 && aligned, P, w, out, t_guard, src);
+  return VX_OK;
+}
+
+// The forward from the hash table and the ray, nothing but the colours written (inference of a C caller without rows).
+int launch_fwd_hash(const HashArgs& a, int64_t P, const MlpW& w, const MlpOut& out, cudaStream_t st) {
+  const int64_t tiles = (P + TM - 1) / TM;
+  auto kern = custom_wait() ? k_mlp_fwd_tc<true> : k_mlp_fwd_tc<false>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
   if (e != cudaSuccess) return set_error(VX_ERR_CUDA, "mlp forward: %s", cudaGetErrorString(e));
   const unsigned blocks = (unsigned)(tiles < (int64_t)kSMs * 2 ? tiles : (int64_t)kSMs * 2);
-  const int xvec = X && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
-  kern<<<blocks, 256, kFwdSmem, st>>>(a, X, ldx, xvec, P, w, out, t_guard);
+  kern<<<blocks, 256, kFwdSmem, st>>>(a, P, w, out, t_guard);
   return VX_OK;
 }
 
@@ -909,8 +906,7 @@ int mlp_backward_launch(const float* x, int64_t ldx, int64_t n_points, const flo
     int64_t ldy = NO, ldm = 2;
     if (!mask || !colors) {
       uint32_t* dm = reinterpret_cast<uint32_t*>(d_hash);
-      HashArgs none{};
-      if (int s = launch_fwd<false, false>(none, x, ldx, n_points, w, MlpOut{d_hash + 2, 32, dm, 32}, st, src)) return s;
+      if (int s = launch_fwd(x, ldx, n_points, w, MlpOut{colors ? nullptr : d_hash + 2, 32, dm, 32}, st, src)) return s;
       mask = dm;
       ldm = 32;
       if (!colors) {
@@ -969,10 +965,10 @@ static int appearance_forward(const float* table, int n_levels, int log2_size, i
   if (rows) {  // training: rows gathered at high occupancy, then the MLP on the rows
     launch_hash_rows(a, st);
     const RowSrc src{ld_rows == KC ? rays_d : nullptr, n_samples};
-    if (int s = launch_fwd<false, false>(a, rows, ld_rows, n_points, w, out, st, src)) return s;
+    if (int s = launch_fwd(rows, ld_rows, n_points, w, out, st, src)) return s;
     count_launches(2);
   } else {  // inference: features built in shared memory, nothing else written
-    if (int s = launch_fwd<true, false>(a, nullptr, 0, n_points, w, out, st)) return s;
+    if (int s = launch_fwd_hash(a, n_points, w, out, st)) return s;
     count_launches(1);
   }
   return check_launch("appearance_mlp_forward");
@@ -981,9 +977,7 @@ static int appearance_forward(const float* table, int n_levels, int log2_size, i
 static int radiance_forward(const float* x, int64_t ldx, int64_t n_points, const float* W0, const float* b0,
                             const float* W1, const float* b1, float* colors, uint32_t* mask, void* stream) {
   MlpW w{W0, b0, W1, b1};
-  HashArgs a{};
-  if (int s = launch_fwd<false, false>(a, x, ldx, n_points, w, MlpOut{colors, NO, mask, 2}, (cudaStream_t)stream))
-    return s;
+  if (int s = launch_fwd(x, ldx, n_points, w, MlpOut{colors, NO, mask, 2}, (cudaStream_t)stream)) return s;
   count_launches(1);
   return check_launch("radiance_mlp_forward");
 }
@@ -1049,8 +1043,8 @@ int vx_appearance_mlp_forward_chunked(const float* table, int n_levels, int log2
     ac.normals = normals + 3 * c0;
     ac.P = len;
     launch_hash_rows(ac, st);
-    if (int s = launch_fwd<false, false>(ac, scratch_rows, KC, len, w, MlpOut{colors + 3 * c0, NO, nullptr, 0}, st,
-                                         RowSrc{ac.rays_d, n_samples}))
+    if (int s = launch_fwd(scratch_rows, KC, len, w, MlpOut{colors + 3 * c0, NO, nullptr, 0}, st,
+                           RowSrc{ac.rays_d, n_samples}))
       return s;
     launches += 2;
   }
