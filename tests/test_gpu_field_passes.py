@@ -77,3 +77,18 @@ def test_crowded_points(res, kind):
     a = ops.field_query(grid, LO, HI, pts, sdf=True, grad=True, normal=True, corners=True)[:3]  # the plain kernel
     for want in ((1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1)):
         _equal(want, a, ops.field_query_sorted(grid, LO, HI, pts, *map(bool, want))[:3])
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("tiny", [1e-30, 1e-33, 1e-36, 1e-40])
+def test_vanishing_gradient_along_one_axis(axis, tiny):
+    """Differences too small for the division from the reciprocal beside ordinary ones: layers of ~1e-30 and less between
+    layers of 1, so that the gradient along the layers is tiny and the one across them is not."""
+    from voxneus_b200 import ops
+
+    torch.manual_seed(5)
+    grid = torch.randn(1, 1, 45, 47, 52, device=DEV) * tiny
+    grid.transpose(2, 2 + axis)[:, :, ::2] = 1.0
+    pts = torch.rand(60_000, 3, device=DEV) * 2.0 - 1.0
+    a = ops.field_query(grid, LO, HI, pts, sdf=True, grad=True, normal=True)[:3]
+    _equal((1, 1, 1), a, ops.field_query_sorted(grid, LO, HI, pts, True, True, True)[:3])
