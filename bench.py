@@ -225,26 +225,35 @@ MLP_FLOPS["vx_appearance_mlp_forward_masked"] = MLP_FLOPS["vx_appearance_mlp_for
 # from the forward's ReLU bits: no hidden recompute; dW0 and dX are contractions of the 0/1 mask, exact in bf16,
 # with three bf16 parts of the other operand
 MLP_FLOPS["vx_appearance_mlp_backward_masked"] = 2 * 3 * 64 * 2 + 2 * 52 * 64 + 2 * 64 * 35
-BF16_PRODUCTS = {"vx_appearance_mlp_backward_masked"}  # the others issue tf32 products
+
+# FLOPs per sample that the MLP kernels issue to the tensor cores in the folded form (128 samples a ray), and their operand
+# type; a tile is 128 samples.
+MLP_ISSUED = {
+    # Z: K = 40 features, X_hi times [W_hi; W_lo] (N = 128) and X_lo times W_hi (N = 64); the colour layer is on the CUDA cores
+    "vx_appearance_mlp_forward": (2 * 40 * (128 + 64), "tf32"),
+    # G: M = 128 rows (3 colours x 36 features and padding) x N = 64 units over the tile's samples; dX: N = 112 columns
+    # (3 colours x 35 features and padding) x K = 64 units; three bf16 parts each
+    "vx_appearance_mlp_backward_masked": (3 * 2 * (128 * 64 + 112 * 64), "bf16"),
+}
+MLP_ISSUED["vx_appearance_mlp_forward_masked"] = MLP_ISSUED["vx_appearance_mlp_forward"]
 
 
 def mlp_tensor(per_kernel, n_points):
-    """FLOP rate of the MLP kernels: FP32-equivalent, and the tensor-core rate they issue, three products
-    per FP32 product: tf32 (hi*hi + hi*lo + lo*hi) against the dense tf32 peak, taken as half the measured
-    bf16 GEMM peak (MEASURED_PEAKS.json), or bf16 parts against that peak itself."""
+    """FLOP rate of the MLP kernels: FP32-equivalent, and the rate that they issue to the tensor cores, against the dense
+    tf32 peak, taken as half the measured bf16 GEMM peak (MEASURED_PEAKS.json), or for bf16 products that peak itself."""
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             bf16, kind = float(json.load(f)["bf16_tflops"]), "measured bf16 / 2"
     except (OSError, KeyError, ValueError):
         bf16, kind = 1590.0, "fallback bf16 / 2"
     out = {"peak_tf32_tflops": bf16 / 2, "peak_kind": kind}
-    for k, fl in MLP_FLOPS.items():
+    for k, (issued, product) in MLP_ISSUED.items():
         if k in per_kernel and per_kernel[k] > 0:
-            tf = n_points * fl / (per_kernel[k] / 1e3) / 1e12
-            kind_peak = bf16 if k in BF16_PRODUCTS else bf16 / 2
-            out[k] = {"fp32_flops_per_sample": fl, "fp32_equiv_tflops": tf, "issued_tflops": 3 * tf,
-                      "issued_type": "bf16" if k in BF16_PRODUCTS else "tf32", "peak_tflops": kind_peak,
-                      "frac": 3 * tf / kind_peak}
+            per_s = n_points / (per_kernel[k] / 1e3) / 1e12
+            peak = bf16 if product == "bf16" else bf16 / 2
+            out[k] = {"fp32_flops_per_sample": MLP_FLOPS[k], "fp32_equiv_tflops": MLP_FLOPS[k] * per_s,
+                      "issued_flops_per_sample": issued, "issued_tflops": issued * per_s, "issued_type": product,
+                      "peak_tflops": peak, "frac": issued * per_s / peak}
     return out
 
 
@@ -610,7 +619,7 @@ def run_fused(args):
             hbm_cands = {k: v for k, v in per_kernel.items() if algorithmic_bytes(k, **sizes) is not None}
             hbm_dom = max(hbm_cands, key=hbm_cands.get)  # the longest HBM/L2-bound call
             cands = dict(hbm_cands)
-            cands.update({k: v for k, v in per_kernel.items() if k in MLP_FLOPS})
+            cands.update({k: v for k, v in per_kernel.items() if k in MLP_ISSUED})
             dominant = max(cands, key=cands.get)  # the longest call overall (tensor-core MLP or HBM-bound)
             dom_timer = _lib.KernelTimer(sorted({dominant, hbm_dom}))
     torch.cuda.synchronize()
@@ -668,16 +677,16 @@ def run_fused(args):
                 "peak_kind": mt["peak_kind"], "unit": "TFLOP/s", "frac": r["frac"],
                 "traffic": load_traffic().get(name.removesuffix("_masked")), "fp32_equiv_tflops": r["fp32_equiv_tflops"],
                 "ms_per_launch": k_ms,
-                "note": f"{r['issued_type']} products issued (3 per FP32 product); the kernel is "
-                        "latency/issue bound at one CTA per SM, not at the tensor pipe"}
+                "note": f"{r['issued_type']} products issued, {r['issued_flops_per_sample']} FLOPs a sample; what bounds the "
+                        "kernel is a tile's staging and readout beside them, not the tensor pipe"}
 
     # the dominant call's binding limit: where it has both an algorithmic byte count and tensor-core
     # FLOPs (the appearance forward: hash gathers + MLP), the bound it comes closer to
-    if dominant in MLP_FLOPS and algorithmic_bytes(dominant, **sizes) is not None:
+    if dominant in MLP_ISSUED and algorithmic_bytes(dominant, **sizes) is not None:
         r_t, r_h = tensor_roofline(dominant), hbm_roofline(dominant)
         roofline = r_t if r_t["frac"] >= r_h["frac"] else r_h
     else:
-        roofline = tensor_roofline(dominant) if dominant in MLP_FLOPS else hbm_roofline(dominant)
+        roofline = tensor_roofline(dominant) if dominant in MLP_ISSUED else hbm_roofline(dominant)
     roofline_hbm = hbm_roofline(hbm_dom)
 
     # end to end through the public API: pinned host rays/targets handed to FusedTrainer.step
