@@ -127,9 +127,11 @@ int vx_field_query(const float* grid, const int32_t res[3], const float xyz_min[
  * scattered points, computed in spatial order: the points are brought into bricks of 16^3 grid
  * cells, queried brick by brick and each result is written at the point's own index, so the
  * outputs are bit-identical to vx_field_query's. For grids larger than the L2 cache, where
- * scattered points read every stencil from a different DRAM row. n < 2^31, taken 2^24 points at a
- * time; workspace: at least vx_field_query_sorted_workspace(n, res) bytes, 256-byte aligned (52
- * bytes a point of a pass and 20 a brick; 0 for sizes that the query refuses). */
+ * scattered points read every stencil from a different DRAM row. Points that crowd into few cells,
+ * and grids with axes above 2^24 or more than 2^22 bricks, are answered as vx_field_query answers
+ * them. n < 2^31, taken 2^24 points at a time; workspace: at least vx_field_query_sorted_workspace(n, res) bytes, 256-byte aligned (52
+ * bytes a point of a pass and 20 a brick; 256 for the grids above; 0 for sizes that the query
+ * refuses). */
 int64_t vx_field_query_sorted_workspace(int64_t n, const int32_t res[3]);
 int vx_field_query_sorted(const float* grid, const int32_t res[3], const float xyz_min[3], const float xyz_max[3],
                           const float* xyz, int64_t n, float* sdf, float* grad, float* normal, void* workspace,
@@ -337,7 +339,8 @@ int vx_tc_guard(int* status, int64_t wait_polls);
  * dW0, db0, dW1, db1 (written, not accumulated; summed over blocks in a fixed order).
  * colors: the forward's outputs (n,3) for the sigmoid's derivative, or NULL to recompute them
  * (the same bits either way). The hidden layer's ReLU mask comes from one more forward launch; the
- * _masked form below takes the one its forward wrote. partials: >= vx_mlp_blocks(n) * vx_mlp_partial_floats() floats. */
+ * _masked form below takes the one its forward wrote. Samples whose gradients are not finite reach
+ * only the hidden units that they activate, as in ReLU's adjoint. partials: >= vx_mlp_blocks(n) * vx_mlp_partial_floats() floats. */
 int vx_radiance_mlp_backward(const float* x, int64_t ldx, int64_t n_points, int in_dim, int hidden, int out_dim,
                              const float* W0, const float* b0, const float* W1, const float* b1, const float* d_colors,
                              const float* colors, float* d_hash, float* d_normal, float* dW0, float* db0, float* dW1,

@@ -38,8 +38,8 @@
 //
 // What bounds it: the shared-memory port. A tile writes and reads A once (92 KB each way), reads V (43 KB)
 // and M (48 KB), about 2,100 cycles at 128 bytes a cycle, and staging A and running G alternate on the
-// one A buffer that fits: ~4,000 cycles a tile. 1,048,576 samples: 317 us (the adjoint that recomputed the
-// hidden layer and split dL/dz) -> 132 us; 262,144 samples: 90 -> 39 us; 200,003 strided rows: 92 -> 55 us.
+// one A buffer that fits: ~4,200 cycles a tile. 1,048,576 samples: 317 us (the adjoint that recomputed the
+// hidden layer and split dL/dz) -> 137 us; 262,144 samples: 90 -> 40 us; 200,003 contiguous rows: 92 -> 53 us.
 // Tried: 24 bf16 products held in registers over the tile boundary (spills in a 96-register budget,
 // 218 us); the G sums left in tensor memory (its truncated additions put 3e-6 of error in dW1, against
 // 2.5e-7); the MMAs issued by a branch of one thread (163 us).

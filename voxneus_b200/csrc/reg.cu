@@ -632,7 +632,7 @@ static int64_t stencil_tiles(const int32_t res[3]) {
   return (int64_t)((res[2] + TZ - 1) / TZ) * ((res[1] + TY - 1) / TY) * ((res[0] + TX - 1) / TX);
 }
 
-// Blocks that share one of the nb loss partials: as many as are resident at once (6 a SM), a tile each on small
+// Blocks that share one of the nb loss partials: up to 4 blocks a SM, as many as are resident, a tile each on small
 // grids.
 static unsigned stencil_cluster(int64_t nb) {
   unsigned c = 8;
