@@ -168,107 +168,164 @@ __device__ __forceinline__ bool adj_sync_or(bool v) {
 // The weight gradients of this block's tiles in plain float32, for blocks in which the products above leave the finite
 // range: dz = active ? sum_c d_c W1[c] : 0, dW0 = dz^T x, db0 = sum dz, dW1 = d^T h, db1 = sum d, in the layout of
 // pb. y and mask are formed again where the caller's launch kept them in d_hash's rows (row strides of 32), which
-// are overwritten by now. By the whole block; sm: its shared memory. 17 warps, ~10 us a tile: only for sums that
-// are not finite.
+// are overwritten by now. By the whole block; sm: its shared memory. 16 warps: z with four samples a warp at a time, two
+// hidden units a lane; the sums with thread (n, kg) holding hidden unit n, features 8 kg .. (1,048,576 samples: 1,180 us
+// in all where a block or all blocks do this, 138 us where none does).
 template <int kMode>
 __device__ __noinline__ void adj_plain_sums(float* sm, const float* X, int64_t ldx, int64_t P, MlpW w, const float* d_out,
                                             const float* y, int64_t ldy, const uint32_t* mask, int64_t ldm, float* pb,
                                             RowSrc src) {
   using S = AdjShape<kMode>;
-  constexpr int kXp = 53, kZp = 65;  // pitches
-  float* WS = sm;                    // W0 [64][51]
-  float* XS = WS + NH * KIN;         // x [128][kXp], feature 51 the one of db0
-  float* DZ = XS + TM * kXp;         // [128][kZp]
-  float* HS = DZ + TM * kZp;         // relu(z) [128][kZp]
-  float* DS = HS + TM * kZp;         // d [128][3]
-  float* RES = DS + TM * NO;         // [WG]
-  static_assert((NH * KIN + TM * (kXp + 2 * kZp + NO) + WG) * 4 <= 200 * 1024, "the block's shared memory");
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int e = tid; e < NH * KIN; e += kAdjThreads) WS[e] = w.W0[e];
-  for (int e = tid; e < WG; e += kAdjThreads) RES[e] = 0.0f;
+  constexpr int kXp = 60, kZp = 65, kWp = 53;  // pitches
+  constexpr int kPer = 8, kGroups = 7;         // features a thread, thread groups with features (the last forms dW1, db1)
+  float* XS = sm;                              // x [128][kXp], feature 51 the one of db0, 0 from there on
+  float* WS = XS + TM * kXp;                   // W0 [64][kWp], 0 from feature 51 on
+  float* DZ = WS + NH * kWp;                   // [128][kZp]
+  float* HS = DZ + TM * kZp;                   // relu(z) [128][kZp]
+  float* DS = HS + TM * kZp;                   // d [128][3]
+  uint32_t* MS = reinterpret_cast<uint32_t*>(DS + TM * NO);  // mask [128][2]
+  static_assert((TM * (kXp + 2 * kZp + NO + 2) + NH * kWp) * 4 <= 200 * 1024, "the block's shared memory");
+  static_assert(kGroups * kPer >= KP && kGroups * kPer <= kXp && (kGroups + 1) * NH == kAdjWork, "the threads' features");
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = tid & (NH - 1), kg = tid / NH;
+  for (int e = tid; e < NH * kWp; e += kAdjThreads) WS[e] = e % kWp < KIN ? w.W0[e / kWp * KIN + e % kWp] : 0.0f;
+  float acc[kPer], acc1[NO];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) acc[j] = 0.0f;
+#pragma unroll
+  for (int c = 0; c < NO; ++c) acc1[c] = 0.0f;
   const int64_t ntiles = (P + TM - 1) / TM;
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     __syncthreads();  // the previous tile's values are read
+    const int64_t r0 = t * TM;
+    const int nrows = (int)(P - r0 < TM ? P - r0 : TM);
     for (int e = tid; e < TM * KIN; e += kAdjThreads) {
       const int r = e / KIN, k = e - r * KIN;
-      const int64_t i = t * TM + r;
       if (S::kCompact && k >= 32 && k < 48) continue;
-      XS[r * kXp + k] = i >= P ? 0.0f : S::kCompact ? X[i * KC + (k < 32 ? k : k - 16)] : X[i * ldx + k];
+      XS[r * kXp + k] = r >= nrows ? 0.0f : S::kCompact ? X[(r0 + r) * KC + (k < 32 ? k : k - 16)] : X[(r0 + r) * ldx + k];
+    }
+    for (int e = tid; e < TM * NO; e += kAdjThreads) {
+      const bool in = e < nrows * NO;
+      const float v = in && ldy == NO ? y[r0 * NO + e] : 0.0f;
+      DS[e] = in ? d_out[r0 * NO + e] * (ldy == NO ? (1.0f - v) * v : 1.0f) : 0.0f;
+      if (e < TM * 2) MS[e] = ldm == 2 && e < nrows * 2 ? mask[r0 * 2 + e] : 0u;
     }
     if (tid < TM) {
-      const int64_t i = t * TM + tid;
-      XS[tid * kXp + KIN] = i < P ? 1.0f : 0.0f;
+      for (int k = KIN; k < kXp; ++k) XS[tid * kXp + k] = k == KIN && tid < nrows ? 1.0f : 0.0f;
       if (S::kCompact) {
         float sh[16];
-        const float* dir = src.rays_d + 3 * ((i < P ? i : P - 1) / src.S);
+        const float* dir = src.rays_d + 3 * ((r0 + (tid < nrows ? tid : nrows - 1)) / src.S);
         sh16(dir[0], dir[1], dir[2], sh);
 #pragma unroll
         for (int k = 0; k < 16; ++k) XS[tid * kXp + 32 + k] = sh[k];
       }
     }
     __syncthreads();
-    for (int r = wid; r < TM; r += kAdjThreads / 32) {  // a warp a sample, two hidden units a lane
-      const int64_t i = t * TM + r;
-      float z[2] = {w.b0[lane], w.b0[lane + 32]};
-      for (int k = 0; k < KIN; ++k) {
-        z[0] = fmaf(WS[lane * KIN + k], XS[r * kXp + k], z[0]);
-        z[1] = fmaf(WS[(lane + 32) * KIN + k], XS[r * kXp + k], z[1]);
-      }
-      float h[2], d[NO];
-      bool on[2];
+    if (wid < kAdjWork / 32) {
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        const int rq = 8 * wid + 4 * q;
+        float z[4][2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        on[u] = i < P && (ldm == 2 ? (mask[i * 2 + u] >> lane & 1u) != 0 : z[u] > 0.0f);
-        h[u] = on[u] ? z[u] : 0.0f;
-      }
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < NO; ++c) {
-        float v = 0.0f;
-        if (ldy != NO)
-          v = sigmoidf_ref(w.b1[c] + warp_sum(fmaf(w.W1[c * NH + lane], h[0], w.W1[c * NH + lane + 32] * h[1])));
-        else if (i < P)
-          v = y[i * NO + c];
-        v = __shfl_sync(0xffffffffu, v, 0);
-        d[c] = i < P ? d_out[i * NO + c] * ((1.0f - v) * v) : 0.0f;
-        if (lane == 0) DS[r * NO + c] = d[c];
-      }
+          for (int u = 0; u < 2; ++u) z[i][u] = w.b0[lane + 32 * u];
+#pragma unroll 1
+        for (int k = 0; k < KP; k += 4) {  // feature 51: W0's padding is 0
+          float w0[4], w1[4];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int n = lane + 32 * u;
-        const float dh = d[0] * w.W1[n] + d[1] * w.W1[NH + n] + d[2] * w.W1[2 * NH + n];
-        DZ[r * kZp + n] = on[u] ? dh : 0.0f;
-        HS[r * kZp + n] = h[u];
+          for (int j = 0; j < 4; ++j) {
+            w0[j] = WS[lane * kWp + k + j];
+            w1[j] = WS[(lane + 32) * kWp + k + j];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(XS + (rq + i) * kXp + k);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              z[i][0] = fmaf(w0[j], x[j], z[i][0]);
+              z[i][1] = fmaf(w1[j], x[j], z[i][1]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = rq + i;
+          const bool in = r < nrows;
+          float h[2], d[NO];
+          bool on[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            on[u] = in && (ldm == 2 ? (MS[r * 2 + u] >> lane & 1u) != 0 : z[i][u] > 0.0f);
+            h[u] = on[u] ? z[i][u] : 0.0f;
+          }
+#pragma unroll
+          for (int c = 0; c < NO; ++c) {
+            d[c] = DS[r * NO + c];
+            if (ldy != NO) {
+              const float o = w.b1[c] + warp_sum(fmaf(w.W1[c * NH + lane], h[0], w.W1[c * NH + lane + 32] * h[1]));
+              const float v = __shfl_sync(0xffffffffu, sigmoidf_ref(o), 0);
+              d[c] *= (1.0f - v) * v;
+              __syncwarp();
+              if (lane == 0) DS[r * NO + c] = d[c];
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int m = lane + 32 * u;
+            const float dh = d[0] * w.W1[m] + d[1] * w.W1[NH + m] + d[2] * w.W1[2 * NH + m];
+            DZ[r * kZp + m] = on[u] ? dh : 0.0f;
+            HS[r * kZp + m] = h[u];
+          }
+        }
       }
     }
     __syncthreads();
-    for (int e = tid; e < WG; e += kAdjThreads) {  // each thread's own entries
-      const float *a, *b;
-      int pa = kZp, pbb = NO;
-      if (e < NH * KP) {  // dW0, and db0 in its padding column
-        a = DZ + e / KP;
-        b = XS + e % KP;
-        pbb = kXp;
-      } else if (e < NH * KP + NO * NH) {
-        a = HS + (e - NH * KP) % NH;
-        b = DS + (e - NH * KP) / NH;
-      } else if (e >= WG - NO) {  // db1: the ones of the samples are its other factor
-        a = XS + KIN;
-        pa = kXp;
-        b = DS + (e - (WG - NO));
-      } else {
-        continue;
-      }
-      float v = 0.0f;
+    if (tid < kAdjWork) {  // rows past P: x, h and d are 0
+      float part[kPer], part1[NO];
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) part[j] = 0.0f;
+#pragma unroll
+      for (int c = 0; c < NO; ++c) part1[c] = 0.0f;
+      if (kg < kGroups) {
 #pragma unroll 4
-      for (int r = 0; r < TM; ++r)
-        if (t * TM + r < P) v = fmaf(a[r * pa], b[r * pbb], v);
-      RES[e] += v;
+        for (int r = 0; r < TM; ++r) {
+          const float dz = DZ[r * kZp + n];
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            const float4 v = *reinterpret_cast<const float4*>(XS + r * kXp + kPer * kg + 4 * f);
+            part[4 * f] = fmaf(dz, v.x, part[4 * f]);
+            part[4 * f + 1] = fmaf(dz, v.y, part[4 * f + 1]);
+            part[4 * f + 2] = fmaf(dz, v.z, part[4 * f + 2]);
+            part[4 * f + 3] = fmaf(dz, v.w, part[4 * f + 3]);
+          }
+        }
+      } else {  // dW1 of hidden unit n, and db1[n]
+#pragma unroll 4
+        for (int r = 0; r < TM; ++r) {
+          const float h = HS[r * kZp + n];
+#pragma unroll
+          for (int c = 0; c < NO; ++c) part1[c] = fmaf(DS[r * NO + c], h, part1[c]);
+          part[0] += n < NO ? DS[r * NO + n] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) acc[j] += part[j];
+#pragma unroll
+      for (int c = 0; c < NO; ++c) acc1[c] += part1[c];
     }
   }
-  __syncthreads();
-  for (int e = tid; e < WG; e += kAdjThreads) {
-    const int n = e - NH * KP - NO * NH;  // db0's unit
-    pb[e] = n >= 0 && n < NH ? RES[n * KP + KIN] : e < NH * KP && e % KP == KIN ? 0.0f : RES[e];
+  if (tid < kGroups * NH) {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int k = kPer * kg + j;
+      if (k < KP) pb[n * KP + k] = k == KIN ? 0.0f : acc[j];
+      if (k == KIN) pb[NH * KP + NO * NH + n] = acc[j];
+    }
+  } else if (tid < kAdjWork) {
+#pragma unroll
+    for (int c = 0; c < NO; ++c) pb[NH * KP + c * NH + n] = acc1[c];
+    if (n < NO) pb[NH * KP + NO * NH + NH + n] = acc[0];
   }
 }
 
